@@ -15,8 +15,8 @@ namespace dsplat {
 __global__ void k_gauss_project_ref(uint32_t, const float*, const float*, const float*, const float*, int, int, float*,
                                     float*, float*);
 __global__ void k_circle_project_ref(uint32_t, const float*, const float*, int, int, float, float*, float*);
-__global__ void k_prep_tiles(uint32_t, const float*, const float*, const float*, int, int, int, uint2*, uint32_t*,
-                             uint32_t*);
+__global__ void k_prep_tiles(uint32_t, const float*, const float*, const float*, int, int, int, uint2*, uint32_t*);
+__global__ void k_count_pairs(uint32_t, const float*, const float*, const float*, int, int, int, unsigned long long*);
 __global__ void k_fused_project(uint32_t, uint32_t, int, const float*, const float*, const float*, const float*,
                                 const float*, const ViewBatch, float4*, uint2*, uint32_t*, uint32_t*);
 __global__ void k_project_bwd_geom(uint32_t, const float*, const float*, const float*, const ViewBatch,
@@ -34,9 +34,11 @@ __global__ void k_sb_scatter(const uint32_t*, const uint2*, uint32_t, uint32_t, 
 __global__ void k_sb_scatter_staged(const uint32_t*, const uint2*, uint32_t, uint32_t, const ViewBatch, const uint32_t*,
                                     uint64_t, uint2*, uint32_t*, uint32_t);
 size_t sb_scatter_staged_smem(uint32_t max_sb, uint32_t max_side, uint32_t qcap);
-__global__ void k_tile_count(const uint2*, const uint32_t*, uint32_t, uint64_t, const ViewBatch, uint32_t*);
-__global__ void k_tile_scatter(const uint2*, const uint32_t*, uint32_t, uint64_t, const ViewBatch, const uint32_t*,
-                               uint32_t*, uint32_t*, uint32_t*);
+size_t tile_seg_slots(uint64_t capacity, uint32_t num_sb);
+cudaError_t split_tile_lists(cudaStream_t, const uint2*, const uint32_t*, uint32_t, uint64_t, const ViewBatch&,
+                             uint32_t*, uint32_t*);
+cudaError_t scatter_tile_lists(cudaStream_t, const uint2*, const uint32_t*, uint32_t, uint64_t, const ViewBatch&,
+                               const uint32_t*, const uint32_t*, uint32_t*, uint32_t*, uint32_t*);
 __global__ void k_clamp_ranges(uint32_t*, uint32_t, uint64_t, uint32_t*);
 __global__ void k_check_capacity(const unsigned long long*, uint64_t, uint32_t*);
 __global__ void k_make_keys64(const uint32_t*, const uint32_t*, const float*, const unsigned long long*, uint64_t,
@@ -195,17 +197,15 @@ int build_sb_lists(cudaStream_t st, const ViewBatch& b, uint32_t n, uint32_t npa
 }
 
 // Stage 2 (reference-format output only): per-tile lists tile2idx/idx2pnt.
-int build_tile_lists(cudaStream_t st, const ViewBatch& b, uint32_t npad, const ListsWs& L, uint32_t* scan_tmp,
-                     uint32_t* item_start, uint32_t* idx2pnt, uint32_t* out_tile, uint64_t capacity,
+int build_tile_lists(cudaStream_t st, const ViewBatch& b, uint32_t npad, const ListsWs& L, uint32_t* segcnt,
+                     uint32_t* scan_tmp, uint32_t* item_start, uint32_t* idx2pnt, uint32_t* out_tile, uint64_t capacity,
                      uint32_t* flags) {
   const uint32_t nchunk = npad / kChunk;
   TRY_CUDA(cudaMemsetAsync(L.tcnt + b.num_items, 0, sizeof(uint32_t), st), "memset");
-  k_tile_count<<<b.num_sb, 256, 0, st>>>(L.list1, L.off1, nchunk, capacity, b, L.tcnt);
-  count_launch();
+  TRY_CUDA(split_tile_lists(st, L.list1, L.off1, nchunk, capacity, b, segcnt, L.tcnt), "tile counts");
   TRY_CUDA(exclusive_scan(st, L.tcnt, item_start, size_t(b.num_items) + 1, scan_tmp), "scan");
-  k_tile_scatter<<<b.num_sb, 256, 0, st>>>(L.list1, L.off1, nchunk, capacity, b, item_start, idx2pnt, out_tile,
-                                           flags);
-  count_launch();
+  TRY_CUDA(scatter_tile_lists(st, L.list1, L.off1, nchunk, capacity, b, segcnt, item_start, idx2pnt, out_tile, flags),
+           "tile scatter");
   k_clamp_ranges<<<64, 256, 0, st>>>(item_start, b.num_items, capacity, flags);
   count_launch();
   TRY_CUDA(cudaGetLastError(), "tile lists");
@@ -269,7 +269,7 @@ struct TileWs {
   uint32_t* flags;  // [0] flags, [1] total pairs
   uint2* rect;
   uint2* srect;  // tile spans in depth order (written by the sort's last pass)
-  uint32_t *cnt, *dka, *dva, *dkb, *dvb, *hist, *scan_tmp, *out_tile;
+  uint32_t *dka, *dva, *dkb, *dvb, *hist, *scan_tmp, *out_tile, *segcnt;
   ListsWs lists;
   size_t bytes;
 };
@@ -299,7 +299,6 @@ TileWs carve_tiles(void* ws, uint32_t n, uint32_t tile_w, uint32_t tile_h, uint6
   t.flags = c.take<uint32_t>(16);
   t.rect = c.take<uint2>(n + 1);
   t.srect = c.take<uint2>(npad);
-  t.cnt = c.take<uint32_t>(size_t(n) + 1);
   t.dka = c.take<uint32_t>(npad);
   t.dva = c.take<uint32_t>(npad);
   t.dkb = c.take<uint32_t>(npad);
@@ -308,16 +307,17 @@ TileWs carve_tiles(void* ws, uint32_t n, uint32_t tile_w, uint32_t tile_h, uint6
   t.hist = c.take<uint32_t>(hw);
   size_t sw = lists_scan_words(b, npad);
   if (hw > sw) sw = hw;
-  if (size_t(n) + 1 > sw) sw = size_t(n) + 1;
   t.scan_tmp = c.take<uint32_t>(scan_tmp_words(sw));
   size_t d0, d1;
   carve_lists(c, b, npad, cap, &t.lists, &d0, &d1);
   t.out_tile = c.take<uint32_t>(cap);
+  t.segcnt = c.take<uint32_t>(tile_seg_slots(cap, b.num_sb) * 64);
   t.bytes = c.off;
   return t;
 }
 
-// counts only: prep + sum
+// counts only: the boxes are read and summed, nothing else is written (the
+// fill forms the spans again)
 int tiles_count(cudaStream_t st, uint32_t n, const float* xyd, const float* aabb, const float* rad, uint32_t tile_w,
                 uint32_t tile_h, uint32_t ts, void* ws, size_t ws_bytes, uint64_t* num_pairs) {
   if (!num_pairs) return fail(DSPLAT_ERR_INVALID_ARG, "num_pairs is null");
@@ -327,13 +327,14 @@ int tiles_count(cudaStream_t st, uint32_t n, const float* xyd, const float* aabb
   t = carve_tiles(ws, n, tile_w, tile_h, 0);
   *num_pairs = 0;
   if (n == 0 || tile_w == 0 || tile_h == 0) return DSPLAT_OK;
-  k_prep_tiles<<<blocks_for(n, 256), 256, 0, st>>>(n, xyd, aabb, rad, int(ts), int(tile_w), int(tile_h), t.rect,
-                                                  t.dka, t.cnt);
+  unsigned long long* const dtotal = reinterpret_cast<unsigned long long*>(t.flags);
+  TRY_CUDA(cudaMemsetAsync(dtotal, 0, sizeof(*dtotal), st), "memset");
+  k_count_pairs<<<std::min(blocks_for(n, 256), 148u * 8u), 256, 0, st>>>(n, xyd, aabb, rad, int(ts), int(tile_w),
+                                                                       int(tile_h), dtotal);
   count_launch();
-  TRY_CUDA(cudaMemsetAsync(t.cnt + n, 0, sizeof(uint32_t), st), "memset");
-  TRY_CUDA(exclusive_scan(st, t.cnt, t.dkb, size_t(n) + 1, t.scan_tmp), "scan");
-  uint32_t total = 0;
-  TRY_CUDA(cudaMemcpyAsync(&total, t.dkb + n, sizeof(uint32_t), cudaMemcpyDeviceToHost, st), "memcpy");
+  TRY_CUDA(cudaGetLastError(), "count");
+  unsigned long long total = 0;
+  TRY_CUDA(cudaMemcpyAsync(&total, dtotal, sizeof(total), cudaMemcpyDeviceToHost, st), "memcpy");
   TRY_CUDA(cudaStreamSynchronize(st), "sync");
   *num_pairs = total;
   return DSPLAT_OK;
@@ -363,7 +364,7 @@ int tiles_fill(cudaStream_t st, uint32_t n, const float* xyd, const float* aabb,
     count_launch();
   }
   k_prep_tiles<<<blocks_for(n, 256), 256, 0, st>>>(n, xyd, aabb, rad, int(ts), int(tile_w), int(tile_h), t.rect,
-                                                  t.dka, t.cnt);
+                                                  t.dka);
   count_launch();
   bool in_b = false;
   TRY_CUDA(radix_sort(st, t.dka, t.dva, t.dkb, t.dvb, npad, nullptr, 32, 1, t.hist, t.scan_tmp, &in_b, t.rect, n,
@@ -372,7 +373,7 @@ int tiles_fill(cudaStream_t st, uint32_t n, const float* xyd, const float* aabb,
   const uint32_t* order = in_b ? t.dvb : t.dva;
   int rc = build_sb_lists(st, b, n, npad, order, t.srect, t.lists, t.scan_tmp, capacity, t.flags);
   if (rc) return rc;
-  rc = build_tile_lists(st, b, npad, t.lists, t.scan_tmp, tile2idx, idx2pnt, keys64 ? t.out_tile : nullptr, capacity,
+  rc = build_tile_lists(st, b, npad, t.lists, t.segcnt, t.scan_tmp, tile2idx, idx2pnt, keys64 ? t.out_tile : nullptr, capacity,
                         t.flags);
   if (rc) return rc;
   if (keys64) {

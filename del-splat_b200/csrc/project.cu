@@ -10,8 +10,8 @@
 //   k_gauss_project_ref   del-splat-cuda-kernels/cuda/splat_gauss.cu:10-53
 //                         (CPU twin del-splat-cpu/src/pnt2xyz.rs:51-96)
 //   k_circle_project_ref  del-splat-cuda-kernels/cuda/splat_circle.cu:7-41
-//   k_prep_tiles          tile_acceleration.h:15-86 (span + key), with the
-//                         per-point counts of count_splat_in_tile
+//   k_prep_tiles          tile_acceleration.h:15-86 (span + key)
+//   k_count_pairs         the total of count_splat_in_tile's per-point counts
 //   k_fused_project       no counterpart: quaternion + log-scale + SH, all
 //                         views of a batch per parameter read.
 #include "common.cuh"
@@ -244,38 +244,69 @@ __global__ void k_circle_project_ref(uint32_t n, const float* __restrict__ xyz,
 }
 
 // ---------------------------------------------------------------------------
-// Tile span, depth key and pair count per point from an AABB source:
+// Tile span of a point from an AABB source:
 //   aabb != nullptr : Gaussian boxes [N,4] (pnt2pixaabb)
 //   aabb == nullptr : circles, box = centre +- rad (aabb2::from_point)
 // ---------------------------------------------------------------------------
-__global__ void k_prep_tiles(uint32_t n, const float* __restrict__ xyd, const float* __restrict__ aabb,
-                             const float* __restrict__ rad, int ts, int tile_w, int tile_h,
-                             uint2* __restrict__ rect, uint32_t* __restrict__ dkey,
-                             uint32_t* __restrict__ cnt) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+struct TileSpan {
+  int x0, y0, x1, y1;
+  __device__ __forceinline__ uint32_t count() const { return uint32_t(x1 - x0) * uint32_t(y1 - y0); }
+};
+
+__device__ __forceinline__ TileSpan tile_span(uint32_t i, const float* __restrict__ xyd, const float* __restrict__ aabb,
+                                              const float* __restrict__ rad, int ts, int tile_w, int tile_h) {
   float a0, a1, a2, a3;
   if (aabb) {
-    a0 = aabb[4 * i];
-    a1 = aabb[4 * i + 1];
-    a2 = aabb[4 * i + 2];
-    a3 = aabb[4 * i + 3];
+    a0 = aabb[4 * size_t(i)];
+    a1 = aabb[4 * size_t(i) + 1];
+    a2 = aabb[4 * size_t(i) + 2];
+    a3 = aabb[4 * size_t(i) + 3];
   } else {
-    const float x = xyd[3 * i], y = xyd[3 * i + 1], r = rad[i];
+    const float x = xyd[3 * size_t(i)], y = xyd[3 * size_t(i) + 1], r = rad[i];
     a0 = x - r;
     a1 = y - r;
     a2 = x + r;
     a3 = y + r;
   }
   const float tsf = tile_inv(ts);
-  int x0 = tile_lo(a0, tsf, tile_w), y0 = tile_lo(a1, tsf, tile_h);
-  int x1 = tile_hi(a2, tsf, tile_w), y1 = tile_hi(a3, tsf, tile_h);
-  if (x1 < x0) x1 = x0;
-  if (y1 < y0) y1 = y0;
-  const uint32_t c = uint32_t(x1 - x0) * uint32_t(y1 - y0);
-  rect[i] = pack_rect(x0, y0, x1, y1);
-  cnt[i] = c;
-  dkey[i] = c ? depth_bits(xyd[3 * i + 2]) : 0xffffffffu;
+  TileSpan s;
+  s.x0 = tile_lo(a0, tsf, tile_w);
+  s.y0 = tile_lo(a1, tsf, tile_h);
+  s.x1 = max(s.x0, tile_hi(a2, tsf, tile_w));
+  s.y1 = max(s.y0, tile_hi(a3, tsf, tile_h));
+  return s;
+}
+
+// Span and depth key of every point.
+__global__ void k_prep_tiles(uint32_t n, const float* __restrict__ xyd, const float* __restrict__ aabb,
+                             const float* __restrict__ rad, int ts, int tile_w, int tile_h,
+                             uint2* __restrict__ rect, uint32_t* __restrict__ dkey) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const TileSpan s = tile_span(i, xyd, aabb, rad, ts, tile_w, tile_h);
+  rect[i] = pack_rect(s.x0, s.y0, s.x1, s.y1);
+  dkey[i] = s.count() ? depth_bits(xyd[3 * size_t(i) + 2]) : 0xffffffffu;
+}
+
+// Sum of the points' tile counts (total zero at the start): only the boxes
+// are read, one atomic per block.
+__global__ void __launch_bounds__(256) k_count_pairs(uint32_t n, const float* __restrict__ xyd,
+                                                     const float* __restrict__ aabb, const float* __restrict__ rad,
+                                                     int ts, int tile_w, int tile_h,
+                                                     unsigned long long* __restrict__ total) {
+  __shared__ unsigned long long sums[8];
+  unsigned long long c = 0;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    c += tile_span(i, xyd, aabb, rad, ts, tile_w, tile_h).count();
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+  if ((threadIdx.x & 31) == 0) sums[threadIdx.x >> 5] = c;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int w = 1; w < 8; ++w) c += sums[w];
+    if (c) atomicAdd(total, c);
+  }
 }
 
 // ---------------------------------------------------------------------------

@@ -16,8 +16,8 @@
 //      whose in-warp slots come from ballots; an entry is (point, its tile
 //      span clipped to the superblock).  The batched rasteriser walks these
 //      lists directly, filtering by tile;
-//   3. stage 2 (reference-format output only): one CTA per superblock splits
-//      its list into per-tile lists with ballot ranking -> tile2idx/idx2pnt.
+//   3. stage 2 (reference-format output only, tile_lists.cu): the superblock
+//      lists split into per-tile lists with ballot ranking -> tile2idx/idx2pnt.
 // Filtering a rank-ordered superblock list by tile keeps rank order, so every
 // tile list is the reference's order, (tile, depth bits, point index)
 // ascending, bit for bit; no 64-bit pair key is sorted.
@@ -609,125 +609,6 @@ __global__ void __launch_bounds__(kMsThreads) k_sb_scatter_staged(const uint32_t
     }
     __syncthreads();
     for (int sb = threadIdx.x; sb < nsb; sb += kMsThreads) cur[sb] += sbase[sb + 1] - sbase[sb];
-    __syncthreads();
-  }
-}
-
-// ---------------------------------------------------------------------------
-// Stage 2a: per-tile pair counts, one CTA per superblock walking its list.
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ int view_of_sb(const ViewBatch& b, uint32_t sb) {
-  int v = 0;
-  for (int k = 1; k < b.num_views; ++k)
-    if (sb >= b.v[k].sb_base) v = k;
-  return v;
-}
-
-__global__ void __launch_bounds__(kMsThreads) k_tile_count(const uint2* __restrict__ list1,
-                                                           const uint32_t* __restrict__ off1, uint32_t nchunk,
-                                                           uint64_t capacity, const ViewBatch b,
-                                                           uint32_t* __restrict__ tcnt) {
-  __shared__ uint32_t h[64];
-  const uint32_t sb = blockIdx.x;
-  const int v = view_of_sb(b, sb);
-  const ViewDev& vd = b.v[v];
-  const int sl = vd.sb_log2, side = 1 << sl, sbw = sb_cols(vd);
-  const uint32_t ls = sb - vd.sb_base;
-  const int tx0 = int(ls % uint32_t(sbw)) << sl, ty0 = int(ls / uint32_t(sbw)) << sl;
-  if (threadIdx.x < 64) h[threadIdx.x] = 0;
-  __syncthreads();
-  const uint64_t s = min(uint64_t(off1[size_t(sb) * nchunk]), capacity);
-  const uint64_t e = min(uint64_t(off1[size_t(sb + 1) * nchunk]), capacity);
-  for (uint64_t i = s + threadIdx.x; i < e; i += kMsThreads) {
-    const uint32_t lr = list1[i].y;
-    const int x0 = lr & 15, y0 = (lr >> 4) & 15, x1 = (lr >> 8) & 15, y1 = (lr >> 12) & 15;
-    for (int y = y0; y < y1; ++y)
-      for (int x = x0; x < x1; ++x) atomicAdd(&h[y * 8 + x], 1u);
-  }
-  __syncthreads();
-  if (threadIdx.x < 64 && int(threadIdx.x & 7) < side && int(threadIdx.x >> 3) < side) {
-    const int x = tx0 + (threadIdx.x & 7), y = ty0 + (threadIdx.x >> 3);
-    if (x < vd.tile_w && y < vd.tile_h) tcnt[vd.item_base + uint32_t(y) * vd.tile_w + x] = h[threadIdx.x];
-  }
-}
-
-// ---------------------------------------------------------------------------
-// Stage 2b: stable scatter into tile lists.  Chunks of 256 list entries, one
-// per thread in order; for each of the 64 tiles a warp ballot says which lanes
-// cover it, and popcounts of the ballots give every pair its slot:
-//   slot = tile start + earlier chunks + earlier warps + lower lanes.
-// out_tile (nullable) receives each pair's item id.
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kMsThreads) k_tile_scatter(const uint2* __restrict__ list1,
-                                                             const uint32_t* __restrict__ off1, uint32_t nchunk,
-                                                             uint64_t capacity, const ViewBatch b,
-                                                               const uint32_t* __restrict__ item_start,
-                                                             uint32_t* __restrict__ idx2pnt,
-                                                             uint32_t* __restrict__ out_tile,
-                                                             uint32_t* __restrict__ flags) {
-  __shared__ uint32_t run[64];
-  __shared__ uint32_t tot[64];
-  __shared__ uint32_t masks[kMsWarps][64];
-  __shared__ uint32_t pre[kMsWarps][64];
-  const uint32_t sb = blockIdx.x;
-  const int v = view_of_sb(b, sb);
-  const ViewDev& vd = b.v[v];
-  const int sl = vd.sb_log2, side = 1 << sl, sbw = sb_cols(vd);
-  const uint32_t ls = sb - vd.sb_base;
-  const int tx0 = int(ls % uint32_t(sbw)) << sl, ty0 = int(ls / uint32_t(sbw)) << sl;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint32_t lt = (1u << lane) - 1u;
-  if (threadIdx.x < 64) {
-    const int x = tx0 + (threadIdx.x & 7), y = ty0 + (threadIdx.x >> 3);
-    const bool in = int(threadIdx.x & 7) < side && int(threadIdx.x >> 3) < side && x < vd.tile_w && y < vd.tile_h;
-    run[threadIdx.x] = in ? item_start[vd.item_base + uint32_t(y) * vd.tile_w + x] : 0u;
-  }
-  __syncthreads();
-  const uint64_t s = min(uint64_t(off1[size_t(sb) * nchunk]), capacity);
-  const uint64_t e = min(uint64_t(off1[size_t(sb + 1) * nchunk]), capacity);
-  for (uint64_t c0 = s; c0 < e; c0 += kMsThreads) {
-    const uint64_t i = c0 + threadIdx.x;
-    uint32_t g = 0;
-    int x0 = 0, x1 = 0, y0 = 0, y1 = 0;
-    if (i < e) {
-      const uint2 en = list1[i];
-      g = en.x;
-      x0 = en.y & 15;
-      y0 = (en.y >> 4) & 15;
-      x1 = (en.y >> 8) & 15;
-      y1 = (en.y >> 12) & 15;
-    }
-#pragma unroll
-    for (int k = 0; k < 64; ++k) {
-      const int kx = k & 7, ky = k >> 3;
-      if (kx >= side || ky >= side) continue;  // outside a smaller superblock
-      const uint32_t m = __ballot_sync(0xffffffffu, kx >= x0 && kx < x1 && ky >= y0 && ky < y1);
-      if ((k & 31) == lane) masks[warp][k] = m;
-    }
-    __syncthreads();
-    if (threadIdx.x < 64) {
-      uint32_t acc = 0;
-#pragma unroll
-      for (int w = 0; w < kMsWarps; ++w) {
-        pre[w][threadIdx.x] = acc;
-        acc += __popc(masks[w][threadIdx.x]);
-      }
-      tot[threadIdx.x] = acc;
-    }
-    __syncthreads();
-    for (int y = y0; y < y1; ++y)
-      for (int x = x0; x < x1; ++x) {
-        const int k = y * 8 + x;
-        const uint32_t slot = run[k] + pre[warp][k] + __popc(masks[warp][k] & lt);
-        if (slot < capacity) {
-          idx2pnt[slot] = g;
-          if (out_tile) out_tile[slot] = vd.item_base + uint32_t(ty0 + y) * vd.tile_w + uint32_t(tx0 + x);
-        } else {
-          set_flag(flags, kFlagPairOverflow);
-        }
-      }
-    __syncthreads();
-    if (threadIdx.x < 64) run[threadIdx.x] += tot[threadIdx.x];
     __syncthreads();
   }
 }
