@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(32 * kRasterWarps) k_raster_fwd(
   __shared__ EntP sm_all[kRasterWarps][32];
   __shared__ float4 park_all[kRasterWarps][G::PPL * 32];
   __shared__ uint32_t park_pos_all[kRasterWarps][G::PPL * 32];
-  __shared__ float tab[128];
+  __shared__ float tab[256];
   load_exp_table(tab);
   EntP* sm = sm_all[threadIdx.x >> 5];
   float4* park = park_all[threadIdx.x >> 5];
@@ -295,7 +295,7 @@ __global__ void __launch_bounds__(32 * kRasterWarps) k_raster_fwd_aos(
   __shared__ EntP sm_all[kRasterWarps][32];
   __shared__ float4 park_all[kRasterWarps][PPL * 32];
   __shared__ uint32_t park_pos_all[kRasterWarps][PPL * 32];
-  __shared__ float tab[128];
+  __shared__ float tab[256];
   load_exp_table(tab);
   EntP* sm = sm_all[threadIdx.x >> 5];
   float4* park = park_all[threadIdx.x >> 5];
