@@ -12,6 +12,64 @@ namespace dsplat {
 // reproduce the forward bit for bit (the discrete structure -- boxes, stop
 // positions -- comes from the forward).
 // ---------------------------------------------------------------------------
+// Per-entry sums over the warp: the nine per-lane values of an entry go to
+// shared memory as nine rows of 32, and every kRedEntries entries the rows
+// are summed eight to an entry, one lane each, with 16-byte reads (rows are
+// 36 words apart, so the eight lanes of a read phase meet 32 different
+// banks).  A transposed shuffle butterfly per entry (14 shuffles with their
+// selects, 2 more for the mean, the output arithmetic in one lane group at a
+// time) cost about 72 of 240 warp-instructions per entry; with the rows and
+// the pixels in packed pairs an entry takes 189 (1,048,576 Gaussians at
+// 1920x1080, 8x8 tiles, counted by ncu).  The kernel then waits on its
+// dependency chains instead of issue slots (68% busy, was 76%): 16 views of
+// 1,048,576 Gaussians 3579 -> 3440 us, 8 at 1920x1080 of 4,194,304 6958 ->
+// 6770, one at 1280x720 of 262,144 337 -> 300.  80 registers (6 blocks of 4
+// warps per SM) are the best cap: at 72 the spills cost more than the warps
+// give (3810), at 96 the warps are missed (3590).
+constexpr int kRedEntries = 4;
+struct __align__(16) RedBuf {
+  float row[kRedEntries][9][36];
+};
+
+__device__ __forceinline__ void red_flush(const RedBuf* red, int held, int lane, float* __restrict__ gv) {
+  __syncwarp();
+  const int slot = lane >> 3, k = lane & 7;
+  const ulonglong2* r = reinterpret_cast<const ulonglong2*>(red->row[slot][k]);
+  f2 s0 = r[0].x, s1 = r[0].y;
+#pragma unroll
+  for (int i = 1; i < 8; ++i) {
+    const ulonglong2 q = r[i];
+    s0 = add2(s0, q.x);
+    s1 = add2(s1, q.y);
+  }
+  s0 = add2(s0, s1);
+  const float sum = f2_lo(s0) + f2_hi(s0);
+  // the ninth row, a quarter word per lane
+  const float4 q8 = *reinterpret_cast<const float4*>(&red->row[slot][8][4 * k]);
+  float gb = (q8.x + q8.y) + (q8.z + q8.w);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) gb += __shfl_xor_sync(0xffffffffu, gb, o);
+  const float m0 = __shfl_sync(0xffffffffu, sum, lane & 24), m1 = __shfl_sync(0xffffffffu, sum, (lane & 24) | 1);
+  const float4 c = *reinterpret_cast<const float4*>(&red->row[slot][0][32]);
+  const uint32_t g = __float_as_uint(red->row[slot][1][32]);
+  // with the w moments m_i = -op/2 (t moments): d px = -2 (A m0 + B m1),
+  // d py = -2 (B m0 + C m1), d A = m2, d B = 2 m3, d C = m4 (raw conic
+  // recovered from the staged one)
+  const float A = c.x * kInvNegHalfLog2e, B = c.y * (0.5f * kInvNegHalfLog2e), C = c.z * kInvNegHalfLog2e;
+  float out = sum;
+  if (k == 0) out = -2.f * (A * m0 + B * m1);
+  if (k == 1) out = -2.f * (B * m0 + C * m1);
+  if (k == 3) out = 2.f * sum;
+  if (k < 5) out *= 0.5f * c.w;  // the moments of t become moments of w = dL/dq (c.w = -opacity)
+  if (k > 5) out = -out;
+  if (slot < held) {
+    float* dst = gv + 12 * size_t(g);
+    atomicAdd(dst + k, out);
+    if (k == 0) atomicAdd(dst + 8, -gb);
+  }
+  __syncwarp();
+}
+
 // NT > 1 (8x8 tiles): one task covers NT horizontally adjacent tiles of one
 // superblock row (fewer where the superblock is narrower), NT x as wide with
 // NT x the pixels per lane, so that the per-entry warp reduction serves NT x
@@ -22,15 +80,18 @@ namespace dsplat {
 // tile's entries (and its stop position is a position in the shared
 // superblock list).  The forward groups tiles the same way.
 template <int TS, int PPL_, int NT>
-__global__ void __launch_bounds__(32 * kRasterWarps) k_raster_bwd(
+__global__ void __launch_bounds__(32 * kRasterWarps, NT * PPL_ <= 4 ? 6 : 4) k_raster_bwd(
     const ViewBatch b, uint32_t n, const float4* __restrict__ rec, const uint2* __restrict__ list1,
     const uint32_t* __restrict__ off1, uint32_t nchunk, uint64_t capacity, const uint32_t* __restrict__ order,
     uint32_t* __restrict__ work_counter, const float* __restrict__ grad_pix, const float* __restrict__ pix_T,
     const uint32_t* __restrict__ pix_last, float4* __restrict__ grad2d) {
   using G = TaskGeo<TS, PPL_, NT>;
-  constexpr int PPL = G::PPL;
+  constexpr int PPL = G::PPL, NP = PPL / 2;
+  static_assert(PPL % 2 == 0, "pixels are evaluated in pairs");
   __shared__ Ent sm_all[kRasterWarps][32];
+  __shared__ RedBuf red_all[kRasterWarps];
   Ent* sm = sm_all[threadIdx.x >> 5];
+  RedBuf* red = &red_all[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   const uint32_t num_tasks = b.num_items * G::SLABS;
   for (;;) {
@@ -53,27 +114,35 @@ __global__ void __launch_bounds__(32 * kRasterWarps) k_raster_bwd(
     const bool col_in = col < int(nx) * TS;
     const float fx = float(ix) + 0.5f;
     const uint32_t s = ig.s, e = ig.e;
-    // per pixel: T in front of the current entry, S = d . (colour behind it),
-    // d = dL/dpixel
-    float Tc[PPL], S[PPL], d0[PPL], d1[PPL], d2[PPL];
+    // per pixel pair: T in front of the current entry, nS = -(d . colour
+    // behind it), d = dL/dpixel; per pixel the stop position
+    f2 Tc[NP], nS[NP], d0[NP], d1[NP], d2[NP], fy2[NP];
     uint32_t last[PPL];
     uint32_t lo_min = e;
 #pragma unroll
-    for (int k = 0; k < PPL; ++k) {
-      const int iy = iy0 + k * G::ROW_STEP;
-      Tc[k] = 1.f;
-      S[k] = 0.f;
-      d0[k] = d1[k] = d2[k] = 0.f;
-      last[k] = e;  // outside pixels process nothing
-      if (col_in && ix < vd.w && iy < vd.h) {
-        const size_t p = size_t(vd.pix_base) + size_t(iy) * vd.w + ix;
-        Tc[k] = pix_T[p];
-        last[k] = pix_last[p];
-        d0[k] = grad_pix[3 * p];
-        d1[k] = grad_pix[3 * p + 1];
-        d2[k] = grad_pix[3 * p + 2];
-        lo_min = min(lo_min, last[k]);
+    for (int q = 0; q < NP; ++q) {
+      float t[2] = {1.f, 1.f}, g0[2] = {0.f, 0.f}, g1[2] = {0.f, 0.f}, g2[2] = {0.f, 0.f}, y[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int k = 2 * q + h, iy = iy0 + k * G::ROW_STEP;
+        y[h] = float(iy) + 0.5f;
+        last[k] = e;  // outside pixels process nothing
+        if (col_in && ix < vd.w && iy < vd.h) {
+          const size_t p = size_t(vd.pix_base) + size_t(iy) * vd.w + ix;
+          t[h] = pix_T[p];
+          last[k] = pix_last[p];
+          g0[h] = grad_pix[3 * p];
+          g1[h] = grad_pix[3 * p + 1];
+          g2[h] = grad_pix[3 * p + 2];
+          lo_min = min(lo_min, last[k]);
+        }
       }
+      Tc[q] = f2_make(t[0], t[1]);
+      nS[q] = f2_make(0.f, 0.f);
+      d0[q] = f2_make(g0[0], g0[1]);
+      d1[q] = f2_make(g1[0], g1[1]);
+      d2[q] = f2_make(g2[0], g2[1]);
+      fy2[q] = f2_make(y[0], y[1]);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) lo_min = min(lo_min, __shfl_xor_sync(0xffffffffu, lo_min, o));
@@ -81,6 +150,7 @@ __global__ void __launch_bounds__(32 * kRasterWarps) k_raster_bwd(
     SbWalkSpan walk{list1, ig.lx, ig.ly, nx};
     float* gv = reinterpret_cast<float*>(grad2d + 3 * size_t(ig.v) * n);
     const uint32_t lo0 = max(s, lo_min);
+    int held = 0;  // entries waiting in red
     uint2 en = lo0 < e ? walk.load(lo0 + uint32_t(lane), uint32_t(lane) < e - lo0) : make_uint2(0u, 0u);
     for (uint32_t lo = lo0; lo < e; lo += 32) {
       const int cnt = int(min(32u, e - lo));
@@ -89,96 +159,75 @@ __global__ void __launch_bounds__(32 * kRasterWarps) k_raster_bwd(
       if (lo + 32u < e) en = walk.load(lo + 32u + uint32_t(lane), uint32_t(lane) < e - (lo + 32u));
       __syncwarp();
       for (int j = 0; j < k_staged; ++j) {
-        const float4 ea = sm[j].a, eb = sm[j].b, ec = sm[j].c, ed = sm[j].d;
-        const uint32_t pos = __float_as_uint(ed.z);
-        // v[]: this lane's sums over its pixels of (t dx, t dy, t dx^2,
-        // t dx dy, t dy^2, t, dL/dr, dL/dg) with t = G dL/dalpha (its sum
-        // is dL/dop; w = dL/dq = -op/2 t); gb = dL/db
-        float v[8], gb = 0.f;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = 0.f;
+        const float4 ed = sm[j].d, ee = sm[j].e;
+        const uint32_t pos = __float_as_uint(sm[j].f.x);
+        // this lane's sums over its pixels, pair halves apart: t = G dL/dalpha
+        // (its sum is dL/dop; w = dL/dq = -op/2 t), t dy, t dy^2, and the
+        // negated dL/dcolour
+        f2 st = 0, sty = 0, styy = 0, nr = 0, ng = 0, nb = 0;
         bool any = false;
-        const float dx = fx - ea.x;
-        if (ec.y <= fx && fx <= ec.w) {
-          const float kadxdx = ea.z * dx * dx, kb2dx = ea.w * dx;
-          // moments of t = G dL/dalpha (v[5] = sum t, tdy = sum t dy, tdyy =
-          // sum t dy^2); w = dL/dq = -op/2 t, the factor is applied once per
-          // entry after the warp reduction
-          float tdy = 0.f, tdyy = 0.f;
+        const float dx = fx - ed.x;
+        if (ee.x <= fx && fx <= ee.y) {
+          const ulonglong2 qa = *reinterpret_cast<const ulonglong2*>(&sm[j].a);
+          const ulonglong2 qb = *reinterpret_cast<const ulonglong2*>(&sm[j].b);
+          const ulonglong2 qc = *reinterpret_cast<const ulonglong2*>(&sm[j].c);
+          const f2 kadxdx = f2_dup(ed.y * dx * dx), kb2dx = f2_dup(ed.z * dx);
 #pragma unroll
-          for (int k = 0; k < PPL; ++k) {
-            const float fy = float(iy0 + k * G::ROW_STEP) + 0.5f;
-            if (pos < last[k] || !(ec.z <= fy && fy <= ed.x)) continue;
+          for (int q = 0; q < NP; ++q) {
+            const float fy0 = f2_lo(fy2[q]), fy1 = f2_hi(fy2[q]);
+            const bool in0 = pos >= last[2 * q] && ee.z <= fy0 && fy0 <= ee.w;
+            const bool in1 = pos >= last[2 * q + 1] && ee.z <= fy1 && fy1 <= ee.w;
+            if (!(in0 || in1)) continue;
             any = true;
-            const float dy = fy - ea.y;
-            const float Gv = ex2_approx(quad_y(eb.x, dy, kb2dx, kadxdx));
-            const float al = Gv * eb.y;
+            const f2 dy = sub2(fy2[q], qa.x);
+            const f2 y = fma2(fma2(qa.y, dy, kb2dx), dy, kadxdx);  // k q
+            // a pixel outside the box or past its stop takes G = 0: alpha 0,
+            // 1 / (1 - alpha) = 1, every sum unchanged
+            const f2 Gv = f2_make(in0 ? ex2_approx(f2_lo(y)) : 0.f, in1 ? ex2_approx(f2_hi(y)) : 0.f);
+            const f2 nal = mul2(Gv, qb.x);  // -alpha
             // alpha < 1 is a precondition (opacity < 1); the floor only
             // keeps gradients finite if an input breaks it
-            const float iom = rcp_approx(fmaxf(1.f - al, 1e-7f));
-            Tc[k] *= iom;
-            const float wgt = al * Tc[k];
-            const float drgb = d0[k] * eb.z + d1[k] * eb.w + d2[k] * ec.x;
-            const float dLde = Tc[k] * drgb - iom * S[k];
-            S[k] += wgt * drgb;
-            v[6] += wgt * d0[k];
-            v[7] += wgt * d1[k];
-            gb += wgt * d2[k];
-            const float t = Gv * dLde;
-            v[5] += t;
-            const float tdy_p = t * dy;
-            tdy += tdy_p;
-            tdyy += tdy_p * dy;
+            const f2 om = add2(nal, f2_dup(1.f));
+            const f2 iom = f2_make(rcp_approx(fmaxf(f2_lo(om), 1e-7f)), rcp_approx(fmaxf(f2_hi(om), 1e-7f)));
+            Tc[q] = mul2(Tc[q], iom);
+            const f2 nw = mul2(nal, Tc[q]);  // -alpha T
+            const f2 drgb = fma2(d2[q], qc.y, fma2(d1[q], qc.x, mul2(d0[q], qb.y)));
+            const f2 dLde = fma2(iom, nS[q], mul2(Tc[q], drgb));
+            nS[q] = fma2(nw, drgb, nS[q]);
+            nr = fma2(nw, d0[q], nr);
+            ng = fma2(nw, d1[q], ng);
+            nb = fma2(nw, d2[q], nb);
+            const f2 t = mul2(Gv, dLde);
+            st = add2(st, t);
+            const f2 ty = mul2(t, dy);
+            sty = add2(sty, ty);
+            styy = fma2(ty, dy, styy);
           }
-          v[0] = v[5] * dx;
-          v[1] = tdy;
-          v[2] = v[0] * dx;
-          v[3] = tdy * dx;
-          v[4] = tdyy;
         }
         if (__any_sync(0xffffffffu, any)) {
-          // transposed butterfly: after the offset-16/8/4 steps lane L holds a
-          // partial sum of v[L >> 2]; offsets 2 and 1 finish it
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const bool up = lane & 16;
-            const float send = up ? v[i] : v[i + 4], keep = up ? v[i + 4] : v[i];
-            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+          const float s_t = f2_lo(st) + f2_hi(st), s_ty = f2_lo(sty) + f2_hi(sty), s_tx = s_t * dx;
+          red->row[held][0][lane] = s_tx;
+          red->row[held][1][lane] = s_ty;
+          red->row[held][2][lane] = s_tx * dx;
+          red->row[held][3][lane] = s_ty * dx;
+          red->row[held][4][lane] = f2_lo(styy) + f2_hi(styy);
+          red->row[held][5][lane] = s_t;
+          red->row[held][6][lane] = f2_lo(nr) + f2_hi(nr);
+          red->row[held][7][lane] = f2_lo(ng) + f2_hi(ng);
+          red->row[held][8][lane] = f2_lo(nb) + f2_hi(nb);
+          // what the flush needs of the entry, in the rows' padding (every
+          // lane stores the same words)
+          *reinterpret_cast<float4*>(&red->row[held][0][32]) = make_float4(ed.y, ed.z, sm[j].a.z, sm[j].b.x);
+          red->row[held][1][32] = ed.w;
+          if (++held == kRedEntries) {
+            red_flush(red, held, lane, gv);
+            held = 0;
           }
-#pragma unroll
-          for (int i = 0; i < 2; ++i) {
-            const bool up = lane & 8;
-            const float send = up ? v[i] : v[i + 2], keep = up ? v[i + 2] : v[i];
-            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
-          }
-          {
-            const bool up = lane & 4;
-            const float send = up ? v[0] : v[1], keep = up ? v[1] : v[0];
-            v[0] = keep + __shfl_xor_sync(0xffffffffu, send, 4);
-          }
-          v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
-          v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) gb += __shfl_xor_sync(0xffffffffu, gb, o);
-          const float m0 = __shfl_sync(0xffffffffu, v[0], 0), m1 = __shfl_sync(0xffffffffu, v[0], 4);
-          // with the w moments m_i = -op/2 (t moments): d px = -2 (A m0 +
-          // B m1), d py = -2 (B m0 + C m1), d A = m2, d B = 2 m3, d C = m4
-          // (raw conic recovered from the staged one)
-          const float A = ea.z * kInvNegHalfLog2e, B = ea.w * (0.5f * kInvNegHalfLog2e),
-                      C = eb.x * kInvNegHalfLog2e;
-          const int k = lane >> 2;
-          float out = v[0];
-          if (k == 0) out = -2.f * (A * m0 + B * m1);
-          if (k == 1) out = -2.f * (B * m0 + C * m1);
-          if (k == 3) out = 2.f * v[0];
-          if (k < 5) out *= -0.5f * eb.y;  // the moments of t become moments of w = dL/dq
-          float* dst = gv + 12 * size_t(__float_as_uint(ed.y));
-          if ((lane & 3) == 0) atomicAdd(dst + k, out);
-          if (lane == 1) atomicAdd(dst + 8, gb);
         }
       }
       __syncwarp();
     }
+    if (held) red_flush(red, held, lane, gv);
   }
 }
 

@@ -45,10 +45,11 @@
 // T_i = T_{i+1} / (1 - e_i), and the colour behind it is accumulated, so no
 // per-pixel list is stored.  Each lane sums its pixels' contributions in
 // registers as moments of t = G dL/dalpha (sum t, sum t dy, sum t dy^2 --
-// dx is fixed per lane; w = dL/dq = -op/2 t is applied once per entry), the warp reduces the nine per-entry sums with a
-// transposed butterfly (9 + 5 shuffles instead of 45), and nine lanes add
-// the finished 2D gradient to the per-(view, point) record with one atomic
-// instruction.
+// dx is fixed per lane; w = dL/dq = -op/2 t is applied once per entry), two
+// pixels at a time with packed f32x2 arithmetic; the warp adds the nine
+// per-lane values of an entry up in shared memory, four entries at once, and
+// adds the finished 2D gradient to the per-(view, point) record with one
+// atomic instruction for the four.
 #pragma once
 #include <type_traits>
 
@@ -66,12 +67,17 @@ static_assert(kFwdGroup8 == kBwdGroup8, "the backward runs its tasks in the forw
 constexpr float kNegHalfLog2e = -0.72134752044448170368f;
 constexpr float kInvNegHalfLog2e = -1.38629436111989061883f;  // -2 ln 2
 
-struct Ent {  // one staged list entry (64 bytes), backward
-  float4 a;   // px, py, k A, k 2B   (k = -log2(e)/2: exp(-q/2) = 2^(k q))
-  float4 b;   // k C, opacity, r, g
-  float4 c;   // b, box x0, box y0, box x1
-  float4 d;   // box y1, point index (bits), list position (bits), -
-  __device__ __forceinline__ void set_pos(uint32_t pos) { d.z = __uint_as_float(pos); }
+// A staged list entry for the backward (96 bytes): the operands of the packed
+// pixel-pair arithmetic are stored twice, so that a 64-bit half of a shared
+// load is a packed operand.
+struct Ent {
+  float4 a;  // py, py, k C, k C        (k = -log2(e)/2: exp(-q/2) = 2^(k q))
+  float4 b;  // -opacity twice, r, r
+  float4 c;  // g, g, b, b
+  float4 d;  // px, k A, k 2B, point index (bits)
+  float4 e;  // box x0, x1, y0, y1
+  float4 f;  // list position (bits), -, -, -
+  __device__ __forceinline__ void set_pos(uint32_t pos) { f.x = __uint_as_float(pos); }
 };
 
 // A staged entry for the forward, whose pixel slots are evaluated in pairs
@@ -114,11 +120,6 @@ __device__ __forceinline__ void make_entp(EntP* dst, float px, float py, float A
   dst->f = make_float4(__uint_as_float(mag < 170.f ? 1u : 0u), 0.f, 0.f, 0.f);
 }
 
-// The staged conic, scaled so that y = k q = kA dx^2 + (k2B dx + kC dy) dy.
-__device__ __forceinline__ float4 scaled_conic_a(float px, float py, float A, float B) {
-  return make_float4(px, py, fm(A, kNegHalfLog2e), fm(fa(B, B), kNegHalfLog2e));
-}
-
 template <int TS, int PPL_>
 struct Geo {
   static constexpr int PPL = PPL_;                // pixels per lane
@@ -145,10 +146,12 @@ __device__ __forceinline__ void stage_packed(Ent* dst, const float4* __restrict_
   const float4 r0 = __ldg(rec + 3 * size_t(g));
   const float4 r1 = __ldg(rec + 3 * size_t(g) + 1);
   const float4 r2 = __ldg(rec + 3 * size_t(g) + 2);
-  dst->a = scaled_conic_a(r0.x, r0.y, r0.z, r0.w);
-  dst->b = make_float4(fm(r1.x, kNegHalfLog2e), r1.y, r1.z, r1.w);
-  dst->c = make_float4(r2.x, fs(r0.x, r2.y), fs(r0.y, r2.z), fa(r0.x, r2.y));
-  dst->d = make_float4(fa(r0.y, r2.z), __uint_as_float(g), 0.f, 0.f);
+  const float kC = fm(r1.x, kNegHalfLog2e);
+  dst->a = make_float4(r0.y, r0.y, kC, kC);
+  dst->b = make_float4(-r1.y, -r1.y, r1.z, r1.z);
+  dst->c = make_float4(r1.w, r1.w, r2.x, r2.x);
+  dst->d = make_float4(r0.x, fm(r0.z, kNegHalfLog2e), fm(fa(r0.w, r0.w), kNegHalfLog2e), __uint_as_float(g));
+  dst->e = make_float4(fs(r0.x, r2.y), fa(r0.x, r2.y), fs(r0.y, r2.z), fa(r0.y, r2.z));
 }
 
 struct AosSrc {
@@ -221,12 +224,6 @@ struct SbWalkSpan {
     return __popc(bal);
   }
 };
-
-// y = k q = (kA dx) dx + (k2B dx + kC dy) dy with the conic terms staged
-// pre-scaled: kadxdx = (kA dx) dx and kb2dx = k2B dx are per entry and lane.
-__device__ __forceinline__ float quad_y(float kC, float dy, float kb2dx, float kadxdx) {
-  return ff(ff(kC, dy, kb2dx), dy, kadxdx);
-}
 
 // Copies expf_cr's 2^(j/128) table into the block's shared memory as two
 // planes, hi at [j] and rel at [128 + j] (one barrier, at kernel start).
