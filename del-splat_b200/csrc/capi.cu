@@ -25,7 +25,7 @@ __global__ void k_project_bwd_colour(uint32_t, int, const float*, const float*, 
                                      float*, float*, unsigned long long*, unsigned long long);
 __global__ void k_prepare_grad2d(const unsigned long long*, unsigned long long, float4*, size_t);
 __global__ void k_adam(size_t, float*, const float*, float*, float*, float, float, float, float, float, float);
-int raster_fwd_group(int ts);
+bool raster_in_blocks(const ViewBatch&);
 __global__ void k_pad_keys(uint32_t*, uint32_t, uint32_t, uint32_t);
 __global__ void k_sb_count(const uint32_t*, const uint2*, uint32_t, uint32_t, const ViewBatch, uint32_t*,
                            unsigned long long*);
@@ -743,7 +743,7 @@ int dsplat_gauss_batch_forward(dsplat_stream stream, const dsplat_gauss_params* 
     stage_mark(st, 3);
   }
   // longest-first raster task order (costs measured by the previous forward)
-  TRY_CUDA(order_tasks(st, b, w.lists.off1, npad / kChunk, w.item_cost, raster_fwd_group(b.ts), w.sched,
+  TRY_CUDA(order_tasks(st, b, w.lists.off1, npad / kChunk, w.item_cost, b.ts > 8 || raster_in_blocks(b) ? 1 : 2, w.sched,
                        w.task_order),
            "task order");
   TRY_CUDA(cudaMemsetAsync(w.item_cost, 0, size_t(b.num_items) * sizeof(uint32_t), st), "memset");

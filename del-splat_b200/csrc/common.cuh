@@ -247,17 +247,23 @@ template <class V>
 __device__ __forceinline__ V expf_cr_tk(V x) {
   return vfma(x, vdup<V>(kExpK), vdup<V>(kExpMagic));
 }
-// ra, rb: s + ylo rounded with ylo moved by +-kExpTie (equal: the fast path
-// holds), before the scaling by 2^(k div 128); th, rel = the table entry
+// e^x = (s + ylo) 2^(k div 128); th, rel = the table entry
 template <class V>
-__device__ __forceinline__ void expf_cr_round(V x, V tk, V th, V rel, V* ra, V* rb) {
+__device__ __forceinline__ void expf_cr_parts(V x, V tk, V th, V rel, V* s, V* ylo) {
   const V kf = vsub(tk, vdup<V>(kExpMagic));
   const V rh = vfma(kf, vdup<V>(-kExpC1), x);
   const V rlt = vfma(kf, vdup<V>(-kExpC2), rel);  // rl + R
   const V p = vfma(rh, vdup<V>(kExpP3), vdup<V>(kExpP2));
   const V tail = vfma(rh, vfma(rh, p, rlt), rlt);
-  const V s = vfma(th, rh, th);
-  const V ylo = vfma(th, tail, vfma(th, rh, vsub(th, s)));
+  *s = vfma(th, rh, th);
+  *ylo = vfma(th, tail, vfma(th, rh, vsub(th, *s)));
+}
+// ra, rb: s + ylo rounded with ylo moved by +-kExpTie (equal: the fast path
+// holds)
+template <class V>
+__device__ __forceinline__ void expf_cr_round(V x, V tk, V th, V rel, V* ra, V* rb) {
+  V s, ylo;
+  expf_cr_parts(x, tk, th, rel, &s, &ylo);
   *ra = vadd(s, vadd(ylo, vdup<V>(kExpTie)));
   *rb = vadd(s, vsub(ylo, vdup<V>(kExpTie)));
 }
@@ -293,6 +299,31 @@ __device__ __forceinline__ f2 expf_cr2(f2 x, const float* tab) {
   if (!ok) {  // rare: settle each element on its own
     if (!(f2_lo(ra) == f2_lo(rb) && fabsf(f2_lo(x)) <= kExpFastMax)) y0 = expf_cr_slow(f2_lo(x));
     if (!(f2_hi(ra) == f2_hi(rb) && fabsf(f2_hi(x)) <= kExpFastMax)) y1 = expf_cr_slow(f2_hi(x));
+  }
+  return f2_make(y0, y1);
+}
+
+// The same with the results that are not wanted left open (a pixel outside
+// the entry's box: its x has no bound, so it must not lead to the slow path)
+// and the range check folded into tie: kExpTie when the caller has bounded
+// |x| by kExpFastMax for the wanted elements, else infinity, which fails the
+// rounding test and leads to the check of x.
+__device__ __forceinline__ f2 expf_cr2_want(f2 x, f2 tie, bool want0, bool want1, const float* tab) {
+  const f2 tk = expf_cr_tk(x);
+  const float k0 = f2_lo(tk), k1 = f2_hi(tk);
+  const uint32_t j0 = __float_as_uint(k0) & 127u, j1 = __float_as_uint(k1) & 127u;
+  f2 s, ylo;
+  expf_cr_parts(x, tk, f2_make(tab[j0], tab[j1]), f2_make(tab[128 + j0], tab[128 + j1]), &s, &ylo);
+  const f2 ra = add2(s, add2(ylo, tie)), rb = add2(s, sub2(ylo, tie));
+  float y0 = expf_cr_scale(f2_lo(ra), k0), y1 = expf_cr_scale(f2_hi(ra), k1);
+  if ((want0 && !(f2_lo(ra) == f2_lo(rb))) || (want1 && !(f2_hi(ra) == f2_hi(rb)))) {  // rare; NaN comes here too
+    const f2 a = add2(s, add2(ylo, f2_dup(kExpTie))), b = add2(s, sub2(ylo, f2_dup(kExpTie)));
+    const bool ok0 = f2_lo(a) == f2_lo(b) && fabsf(f2_lo(x)) <= kExpFastMax;
+    const bool ok1 = f2_hi(a) == f2_hi(b) && fabsf(f2_hi(x)) <= kExpFastMax;
+    y0 = expf_cr_scale(f2_lo(a), k0);
+    y1 = expf_cr_scale(f2_hi(a), k1);
+    if (want0 && !ok0) y0 = expf_cr_slow(f2_lo(x));
+    if (want1 && !ok1) y1 = expf_cr_slow(f2_hi(x));
   }
   return f2_make(y0, y1);
 }

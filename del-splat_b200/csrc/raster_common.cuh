@@ -58,6 +58,9 @@
 namespace dsplat {
 
 constexpr int kRasterWarps = 4;  // warps per CTA (independent tasks)
+// a walk's cost in the schedule's units (about eight warp-instructions): list
+// batches read and entries staged
+constexpr uint32_t kCostBatch = 8, kCostEntry = 16;
 constexpr int kFwdGroup8 = 2;    // 8x8 tiles per forward task
 constexpr int kBwdGroup8 = 2;    // 8x8 tiles per backward task (4 measured slower: registers, partial overlaps)
 static_assert(kFwdGroup8 == kBwdGroup8, "the backward runs its tasks in the forward's order");
@@ -154,16 +157,6 @@ __device__ __forceinline__ void stage_packed(Ent* dst, const float4* __restrict_
   dst->e = make_float4(fs(r0.x, r2.y), fa(r0.x, r2.y), fs(r0.y, r2.z), fa(r0.y, r2.z));
 }
 
-struct AosSrc {
-  const float *xyd, *conic, *aabb, *opacity, *rgb;
-  __device__ __forceinline__ void stage(EntP* dst, uint32_t g) const {
-    const size_t i = g;
-    make_entp(dst, xyd[3 * i], xyd[3 * i + 1], conic[3 * i], conic[3 * i + 1], conic[3 * i + 2], opacity[i],
-              rgb[3 * i], rgb[3 * i + 1], rgb[3 * i + 2], aabb[4 * i], aabb[4 * i + 1], aabb[4 * i + 2],
-              aabb[4 * i + 3]);
-  }
-};
-
 struct PackedSrc {
   const float4* rec;
   __device__ __forceinline__ void stage(Ent* dst, uint32_t g) const { stage_packed(dst, rec, g); }
@@ -182,21 +175,6 @@ struct PackedSrc {
 // return how many were staged.
 // load() reads a lane's list word ahead of time (a prefetch while the
 // previous batch is walked); stage() filters and gathers from it.
-struct TileWalk {  // a per-tile list (tile2idx / idx2pnt)
-  const uint32_t* idx2pnt;
-  __device__ __forceinline__ uint2 load(uint32_t pos, bool valid) const {
-    return make_uint2(valid ? idx2pnt[pos] : 0u, 0u);
-  }
-  template <class Src, class E>
-  __device__ __forceinline__ int stage(const Src& src, E* sm, uint2 en, uint32_t pos, bool valid, int lane) const {
-    if (valid) {
-      src.stage(&sm[lane], en.x);
-      sm[lane].set_pos(pos);
-    }
-    return __popc(__ballot_sync(0xffffffffu, valid));
-  }
-};
-
 // A superblock list filtered to the tiles lx .. lx+nx-1 of one superblock row
 // (a fused-path warp task): an entry is kept if its span meets any of them;
 // ballot compaction keeps the list order.
@@ -206,14 +184,17 @@ struct SbWalkSpan {
   __device__ __forceinline__ uint2 load(uint32_t pos, bool valid) const {
     return valid ? list1[pos] : make_uint2(0u, 0u);
   }
+  __device__ __forceinline__ bool hit(uint2 en) const {
+    const uint32_t lr = en.y;
+    return lx < ((lr >> 8) & 15u) && lx + nx > (lr & 15u) && ly >= ((lr >> 4) & 15u) && ly < (lr >> 12);
+  }
   template <class Src, class E>
   __device__ __forceinline__ int stage(const Src& src, E* sm, uint2 en, uint32_t pos, bool valid, int lane) const {
     bool m = false;
     uint32_t g = 0;
     if (valid) {
       g = en.x;
-      const uint32_t lr = en.y;
-      m = lx < ((lr >> 8) & 15u) && lx + nx > (lr & 15u) && ly >= ((lr >> 4) & 15u) && ly < (lr >> 12);
+      m = hit(en);
     }
     const uint32_t bal = __ballot_sync(0xffffffffu, m);
     if (m) {

@@ -11,24 +11,24 @@
 
 namespace dsplat {
 
+cudaError_t raster_blocks(cudaStream_t, const ViewBatch&, const FwdArgs&);
+
 // ---------------------------------------------------------------------------
 // Forward walk of one slab by one warp over the list range [s, e).  Slot k of
 // every lane lies in the same row pair of the slab, so the per-slot skips
 // (pixel done, row outside the entry's box) are uniform across the warp most
 // of the time.
 // ---------------------------------------------------------------------------
-// CUDA_STOP: the stop test of the reference's CUDA kernel (alpha_sum >=
-// 0.999f, its double comparison) instead of del-splat-cpu's (> 0.999f).
 // SPLIT (a 16x8 task of two 8x8 tiles, 4 slots per lane): lane L covers
 // column L % 8 of both tiles at rows L / 8 and L / 8 + 4, slot pair 0 in the
 // left tile and pair 1 in the right one, so that an entry whose box meets
 // one tile keeps every lane of the warp busy on one pair and skips the
 // other pair warp-wide.  Otherwise lane L covers column L % TS, slot k at
 // row L / TS + k (32 / TS).
-template <int TS, int PPL_, bool CUDA_STOP, bool SPLIT, class Walk, class Src>
+template <int TS, int PPL_, bool SPLIT, class Walk, class Src>
 __device__ __forceinline__ uint32_t fwd_slab(const Walk& walk, const Src& src, EntP* sm, float4* park,
                                          uint32_t* park_pos, const float* tab, float nz,
-                                         uint32_t s, uint32_t e, int px0, int py0, int w, int h, int xend, bool accumulate,
+                                         uint32_t s, uint32_t e, int px0, int py0, int w, int h, int xend,
                                          float* __restrict__ out_rgb, size_t pix_base, float* __restrict__ out_T,
                                          uint32_t* __restrict__ out_last, const float* __restrict__ target,
                                          float* __restrict__ grad_pix, float* __restrict__ loss_slot) {
@@ -57,12 +57,6 @@ __device__ __forceinline__ uint32_t fwd_slab(const Walk& walk, const Src& src, E
     c0[k] = c1[k] = c2[k] = 0.f;
     if (ix < xend && iy < h) {
       live |= 1u << k;
-      if (accumulate) {
-        const size_t p = pix_base + size_t(iy) * w + ix;
-        c0[k] = out_rgb[3 * p];
-        c1[k] = out_rgb[3 * p + 1];
-        c2[k] = out_rgb[3 * p + 2];
-      }
     }
   }
   // slot pairs (2p, 2p+1) in packed registers during the walk
@@ -83,7 +77,7 @@ __device__ __forceinline__ uint32_t fwd_slab(const Walk& walk, const Src& src, E
   const uint32_t inside = live;
   // centres of the slab's first and last rows (the same for every lane)
   const float fy_first = float(py0) + 0.5f, fy_last = float(py0 + G::SLAB_ROWS - 1) + 0.5f;
-  uint32_t hi = e;
+  uint32_t hi = e, cost = 0;
   uint2 en = hi > s ? walk.load(hi - 1u - uint32_t(lane), uint32_t(lane) < hi - s) : make_uint2(0u, 0u);
   while (hi > s) {
     const int cnt = int(min(32u, hi - s));
@@ -156,15 +150,15 @@ __device__ __forceinline__ uint32_t fwd_slab(const Walk& walk, const Src& src, E
             // or below the threshold until it stops, so one test of the
             // pair's larger sum finds every slot that stops at this entry
             const float amax = fmaxf(f2_lo(as2[q]), f2_hi(as2[q]));
-            if (CUDA_STOP ? amax >= kAlphaStop : amax > kAlphaStop) {  // rare
+            if (amax > kAlphaStop) {  // rare
               float s0 = f2_lo(as2[q]), s1 = f2_hi(as2[q]);
-              if (CUDA_STOP ? s0 >= kAlphaStop : s0 > kAlphaStop) {
+              if (s0 > kAlphaStop) {
                 live &= ~(1u << k0);
                 park[k0 * 32 + lane] = make_float4(f2_lo(T2[q]), f2_lo(c02[q]), f2_lo(c12[q]), f2_lo(c22[q]));
                 park_pos[k0 * 32 + lane] = pos;
                 s0 = -INFINITY;
               }
-              if (CUDA_STOP ? s1 >= kAlphaStop : s1 > kAlphaStop) {
+              if (s1 > kAlphaStop) {
                 live &= ~(1u << k1);
                 park[k1 * 32 + lane] = make_float4(f2_hi(T2[q]), f2_hi(c02[q]), f2_hi(c12[q]), f2_hi(c22[q]));
                 park_pos[k1 * 32 + lane] = pos;
@@ -190,6 +184,7 @@ __device__ __forceinline__ uint32_t fwd_slab(const Walk& walk, const Src& src, E
       }
     }
     hi -= uint32_t(cnt);
+    cost += kCostBatch + uint32_t(k_staged) * kCostEntry;
     if (!__any_sync(0xffffffffu, live != 0u)) break;
     __syncwarp();
   }
@@ -229,7 +224,7 @@ __device__ __forceinline__ uint32_t fwd_slab(const Walk& walk, const Src& src, E
     for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
     if (lane == 0) *loss_slot = l;
   }
-  return e - hi;
+  return cost;
 }
 
 // ---------------------------------------------------------------------------
@@ -275,39 +270,13 @@ __global__ void __launch_bounds__(32 * kRasterWarps) k_raster_fwd(
     PackedSrc src{rec + 3 * size_t(ig.v) * n};
     SbWalkSpan walk{list1, ig.lx, ig.ly, nx};
     const int xend = min(vd.w, ig.px0 + int(nx) * TS);
-    const uint32_t walked = fwd_slab<G::GX, G::PPL, false, NT == 2 && G::PPL == 4>(
-        walk, src, sm, park, park_pos, tab, nz, ig.s, ig.e, ig.px0, ig.py0 + int(slab) * G::SLAB_ROWS, vd.w, vd.h, xend, false, out_rgb,
+    const uint32_t walked = fwd_slab<G::GX, G::PPL, NT == 2 && G::PPL == 4>(
+        walk, src, sm, park, park_pos, tab, nz, ig.s, ig.e, ig.px0, ig.py0 + int(slab) * G::SLAB_ROWS, vd.w, vd.h, xend, out_rgb,
         vd.pix_base, out_T, out_last, target, grad_pix, slab_loss ? slab_loss + size_t(item) * G::SLABS + slab : nullptr);
-    // scheduling hint for the backward and the next forward: list positions walked
+    // scheduling hint for the backward and the next forward
     if (lane == 0 && walked) atomicMax(&item_cost[item], walked);
     __syncwarp();
   }
-}
-
-// Drop-in forward (splat_gauss.rs:46-94): AoS inputs and per-tile lists,
-// accumulates into pix2rgb.
-template <int TS, int PPL, bool CUDA_STOP>
-__global__ void __launch_bounds__(32 * kRasterWarps) k_raster_fwd_aos(
-    int w, int h, int tile_w, uint32_t num_tasks, float* __restrict__ pix2rgb, AosSrc src,
-    const uint32_t* __restrict__ tile2idx, const uint32_t* __restrict__ idx2pnt, float* __restrict__ out_T,
-    uint32_t* __restrict__ out_last, float nz) {
-  using G = Geo<TS, PPL>;
-  __shared__ EntP sm_all[kRasterWarps][32];
-  __shared__ float4 park_all[kRasterWarps][PPL * 32];
-  __shared__ uint32_t park_pos_all[kRasterWarps][PPL * 32];
-  __shared__ float tab[256];
-  load_exp_table(tab);
-  EntP* sm = sm_all[threadIdx.x >> 5];
-  float4* park = park_all[threadIdx.x >> 5];
-  uint32_t* park_pos = park_pos_all[threadIdx.x >> 5];
-  const uint32_t task = blockIdx.x * kRasterWarps + (threadIdx.x >> 5);
-  if (task >= num_tasks) return;
-  const uint32_t tile = task / G::SLABS, slab = task % G::SLABS;
-  const int px0 = int(tile % uint32_t(tile_w)) * TS;
-  const int py0 = int(tile / uint32_t(tile_w)) * TS + int(slab) * G::SLAB_ROWS;
-  TileWalk walk{idx2pnt};
-  fwd_slab<TS, PPL, CUDA_STOP, false>(walk, src, sm, park, park_pos, tab, nz, tile2idx[tile], tile2idx[tile + 1], px0, py0, w, h, w, true, pix2rgb, 0, out_T,
-                    out_last, nullptr, nullptr, nullptr);
 }
 
 template <int TS, int PPL>
@@ -320,9 +289,31 @@ static void launch_fwd(cudaStream_t st, const ViewBatch& b, const FwdArgs& a) {
   count_launch();
 }
 
-int raster_fwd_group(int ts) { return ts == 8 ? kFwdGroup8 : 1; }
+// Whether a batch's forward and backward run in 8x8 blocks (raster_blocks.cu,
+// k_raster_bwd's BLOCK form) instead of the tasks here.  Blocks win while the
+// step waits for its longest walks, the tasks here once there is enough work
+// to hide them, and the earlier the larger the views are against the tasks
+// (an entry then mostly holds all of a task's pixels).  Whole steps in us,
+// tasks here -> blocks, at the configuration of 8x8 tiles:
+//   1,048,576 Gaussians, one view  1280x720   1735 -> 1457
+//   262,144,   4 views              1280x720   1686 -> 1554
+//   1,048,576, 4 views              1280x720   4026 -> 3336
+//   100,003,   8 views               640x480   1289 -> 1183
+//   1,048,576, one view             1920x1080  1722 -> 1868
+//   1,048,576, 2 views              1920x1080  2714 -> 3144
+//   262,144,   8 views              1280x720   2387 -> 2748
+//   1,048,576, 16 views, 13.5 M pixels         8878 -> 9888
+constexpr uint32_t kBlockBatchPixels = 4u << 20, kBlockViewPixels = 5u << 18;
+
+bool raster_in_blocks(const ViewBatch& b) {
+  if (b.num_pix > kBlockBatchPixels) return false;
+  for (int v = 0; v < b.num_views; ++v)
+    if (uint32_t(b.v[v].w) * uint32_t(b.v[v].h) > kBlockViewPixels) return false;
+  return true;
+}
 
 cudaError_t raster_fwd(cudaStream_t st, const ViewBatch& b, const FwdArgs& a) {
+  if (raster_in_blocks(b)) return raster_blocks(st, b, a);
 #define X(T, P)                        \
   if (b.ts == T && b.ppl == P) {       \
     launch_fwd<T, P>(st, b, a);        \
@@ -331,46 +322,6 @@ cudaError_t raster_fwd(cudaStream_t st, const ViewBatch& b, const FwdArgs& a) {
   DSPLAT_RASTER_CONFIGS(X)
 #undef X
   return cudaErrorInvalidValue;
-}
-
-template <int TS, int PPL, bool CUDA_STOP>
-static void launch_aos(cudaStream_t st, int w, int h, float* pix2rgb, const AosSrc& src, const uint32_t* tile2idx,
-                       const uint32_t* idx2pnt, float* out_T, uint32_t* out_last) {
-  const int tw = (w + TS - 1) / TS, th = (h + TS - 1) / TS;
-  const uint32_t tasks = uint32_t(tw) * uint32_t(th) * Geo<TS, PPL>::SLABS;
-  const unsigned grid = (tasks + kRasterWarps - 1) / kRasterWarps;
-  k_raster_fwd_aos<TS, PPL, CUDA_STOP><<<grid, 32 * kRasterWarps, 0, st>>>(w, h, tw, tasks, pix2rgb, src, tile2idx,
-                                                                           idx2pnt, out_T, out_last, -0.f);
-  count_launch();
-}
-
-template <bool CUDA_STOP>
-static cudaError_t launch_aos_ts(cudaStream_t st, int ts, int w, int h, float* pix2rgb, const AosSrc& src,
-                                 const uint32_t* tile2idx, const uint32_t* idx2pnt, float* out_T,
-                                 uint32_t* out_last) {
-  switch (ts) {
-    case 8:
-      launch_aos<8, 2, CUDA_STOP>(st, w, h, pix2rgb, src, tile2idx, idx2pnt, out_T, out_last);
-      break;
-    case 16:
-      launch_aos<16, 4, CUDA_STOP>(st, w, h, pix2rgb, src, tile2idx, idx2pnt, out_T, out_last);
-      break;
-    case 32:
-      launch_aos<32, 4, CUDA_STOP>(st, w, h, pix2rgb, src, tile2idx, idx2pnt, out_T, out_last);
-      break;
-    default:
-      return cudaErrorInvalidValue;
-  }
-  return cudaGetLastError();
-}
-
-cudaError_t raster_fwd_aos(cudaStream_t st, int ts, int w, int h, float* pix2rgb, const float* xyd, const float* conic,
-                           const float* aabb, const float* opacity, const float* rgb, const uint32_t* tile2idx,
-                           const uint32_t* idx2pnt, float* out_T, uint32_t* out_last, bool cuda_stop) {
-  if (w <= 0 || h <= 0) return cudaSuccess;
-  const AosSrc src{xyd, conic, aabb, opacity, rgb};
-  return cuda_stop ? launch_aos_ts<true>(st, ts, w, h, pix2rgb, src, tile2idx, idx2pnt, out_T, out_last)
-                   : launch_aos_ts<false>(st, ts, w, h, pix2rgb, src, tile2idx, idx2pnt, out_T, out_last);
 }
 
 // expf_cr elementwise (exposed so that it can be checked against a
