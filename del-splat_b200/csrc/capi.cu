@@ -136,21 +136,39 @@ struct Carver {
 // Tile lists from rank order (shared by the drop-in and batched paths):
 // stage 1 superblock multisplit, stage 2 per-tile multisplit; see tiles.cu.
 // ---------------------------------------------------------------------------
-constexpr uint32_t kChunk = 4096;  // ranks per stage-1 chunk (= kSortTile)
+// Ranks per stage-1 chunk (one block each): 4096, fewer while that leaves the
+// blocks below kChunkBlocks.  A block's time is that of its sub-passes of 512
+// ranks (about 11 us each with their barriers), so a short list of ranks is
+// cut finer; a long one is not, since every chunk has a counter for each
+// superblock to be zeroed, scanned and read.  Counts and scatter together, us,
+// chunks of 4096 -> as chosen: 16,384 points in one view 114 -> 21, 262,144
+// 103 -> 26, 1,048,576 167 -> 95, 100,003 in 8 views 137 -> 68; cut to 512 where
+// 4096 are chosen, 1,048,576 in 16 views 914 -> 966.
+constexpr uint32_t kChunkBlocks = 148 * 6;
+
+uint32_t choose_chunk(uint32_t views, uint32_t npad) {
+  uint32_t chunk = 4096;
+  while (chunk > 512 && uint64_t(views) * (npad / chunk) < kChunkBlocks) chunk /= 2;
+  return chunk;
+}
 
 struct ListsWs {
   uint32_t *cnt1, *off1, *tcnt;
   uint2* list1;
 };
 
+uint32_t num_chunks(const ViewBatch& b, uint32_t npad) {
+  return npad / choose_chunk(uint32_t(b.num_views), npad);
+}
+
 size_t lists_scan_words(const ViewBatch& b, uint32_t npad) {
-  const size_t a = size_t(b.num_sb) * (npad / kChunk) + 1, c = size_t(b.num_items) + 1;
+  const size_t a = size_t(b.num_sb) * num_chunks(b, npad) + 1, c = size_t(b.num_items) + 1;
   return a > c ? a : c;
 }
 
 void carve_lists(Carver& c, const ViewBatch& b, uint32_t npad, size_t cap, ListsWs* L, size_t* off_list1,
                  size_t* off_off1) {
-  const size_t m = size_t(b.num_sb) * (npad / kChunk) + 1;
+  const size_t m = size_t(b.num_sb) * num_chunks(b, npad) + 1;
   L->cnt1 = c.take<uint32_t>(m);
   L->off1 = c.take<uint32_t>(m, off_off1);
   L->list1 = c.take<uint2>(cap, off_list1);
@@ -162,7 +180,7 @@ void carve_lists(Carver& c, const ViewBatch& b, uint32_t npad, size_t cap, Lists
 // (capacity needed, u64); flags[0] |= overflow when they exceed capacity.
 int build_sb_lists(cudaStream_t st, const ViewBatch& b, uint32_t n, uint32_t npad, const uint32_t* order,
                    const uint2* srect, const ListsWs& L, uint32_t* scan_tmp, uint64_t capacity, uint32_t* flags) {
-  const uint32_t nchunk = npad / kChunk;
+  const uint32_t nchunk = num_chunks(b, npad);
   const size_t m = size_t(b.num_sb) * nchunk;
   const unsigned grid1 = unsigned(b.num_views) * nchunk;
   const size_t smem1 = size_t(b.max_sb) * sizeof(uint32_t);
@@ -172,7 +190,7 @@ int build_sb_lists(cudaStream_t st, const ViewBatch& b, uint32_t n, uint32_t npa
     TRY_CUDA(cudaFuncSetAttribute(k_sb_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem3)), "attr");
   }
   unsigned long long* totals = reinterpret_cast<unsigned long long*>(flags + 6);
-  k_sb_count<<<grid1, 256, smem1, st>>>(order, srect, n, npad, b, L.cnt1, totals);
+  k_sb_count<<<grid1, 256, smem1, st>>>(order, srect, npad / nchunk, npad, b, L.cnt1, totals);
   count_launch();
   TRY_CUDA(cudaMemsetAsync(L.cnt1 + m, 0, sizeof(uint32_t), st), "memset");
   TRY_CUDA(exclusive_scan(st, L.cnt1, L.off1, m + 1, scan_tmp), "scan");
@@ -186,10 +204,10 @@ int build_sb_lists(cudaStream_t st, const ViewBatch& b, uint32_t n, uint32_t npa
       TRY_CUDA(cudaFuncSetAttribute(k_sb_scatter_staged, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     int(smem_staged)),
                "attr");
-    k_sb_scatter_staged<<<grid1, 256, smem_staged, st>>>(order, srect, n, npad, b, L.off1, capacity, L.list1, flags,
+    k_sb_scatter_staged<<<grid1, 256, smem_staged, st>>>(order, srect, npad / nchunk, npad, b, L.off1, capacity, L.list1, flags,
                                                          kStageEntries);
   } else {
-    k_sb_scatter<<<grid1, 256, smem3, st>>>(order, srect, n, npad, b, L.off1, capacity, L.list1, flags);
+    k_sb_scatter<<<grid1, 256, smem3, st>>>(order, srect, npad / nchunk, npad, b, L.off1, capacity, L.list1, flags);
   }
   count_launch();
   TRY_CUDA(cudaGetLastError(), "superblock lists");
@@ -200,7 +218,7 @@ int build_sb_lists(cudaStream_t st, const ViewBatch& b, uint32_t n, uint32_t npa
 int build_tile_lists(cudaStream_t st, const ViewBatch& b, uint32_t npad, const ListsWs& L, uint32_t* segcnt,
                      uint32_t* scan_tmp, uint32_t* item_start, uint32_t* idx2pnt, uint32_t* out_tile, uint64_t capacity,
                      uint32_t* flags) {
-  const uint32_t nchunk = npad / kChunk;
+  const uint32_t nchunk = num_chunks(b, npad);
   TRY_CUDA(cudaMemsetAsync(L.tcnt + b.num_items, 0, sizeof(uint32_t), st), "memset");
   TRY_CUDA(split_tile_lists(st, L.list1, L.off1, nchunk, capacity, b, segcnt, L.tcnt), "tile counts");
   TRY_CUDA(exclusive_scan(st, L.tcnt, item_start, size_t(b.num_items) + 1, scan_tmp), "scan");
@@ -484,7 +502,7 @@ BatchWs carve_batch(void* ws, uint32_t n, const ViewBatch& b, uint64_t capacity)
   if (hw > sw) sw = hw;
   w.scan_tmp = c.take<uint32_t>(scan_tmp_words(sw));
   carve_lists(c, b, npad, cap, &w.lists, &L.off_sb_list, &L.off_sb_start);
-  L.sb_chunks = npad / kChunk;
+  L.sb_chunks = num_chunks(b, npad);
   L.num_sb = b.num_sb;
   for (int v = 0; v < b.num_views; ++v) L.sb_log2[v] = b.v[v].sb_log2;
   w.pix_T = c.take<float>(b.num_pix, &L.off_pix_T);
@@ -721,7 +739,7 @@ int dsplat_gauss_batch_forward(dsplat_stream stream, const dsplat_gauss_params* 
   stage_mark(st, 0);
   TRY_CUDA(cudaMemsetAsync(w.flags, 0, 16 * sizeof(uint32_t), st), "memset");
   if (n == 0 || pair_capacity == 0) {
-    TRY_CUDA(cudaMemsetAsync(w.lists.off1, 0, (size_t(b.num_sb) * (npad / kChunk) + 1) * 4, st), "memset");
+    TRY_CUDA(cudaMemsetAsync(w.lists.off1, 0, (size_t(b.num_sb) * w.L.sb_chunks + 1) * 4, st), "memset");
   } else {
     if (npad > n) {
       k_pad_keys<<<blocks_for(size_t(npad - n) * V, 256), 256, 0, st>>>(w.dka, n, npad, V);
@@ -743,12 +761,12 @@ int dsplat_gauss_batch_forward(dsplat_stream stream, const dsplat_gauss_params* 
     stage_mark(st, 3);
   }
   // longest-first raster task order (costs measured by the previous forward)
-  TRY_CUDA(order_tasks(st, b, w.lists.off1, npad / kChunk, w.item_cost, b.ts > 8 || raster_in_blocks(b) ? 1 : 2, w.sched,
+  TRY_CUDA(order_tasks(st, b, w.lists.off1, w.L.sb_chunks, w.item_cost, b.ts > 8 || raster_in_blocks(b) ? 1 : 2, w.sched,
                        w.task_order),
            "task order");
   TRY_CUDA(cudaMemsetAsync(w.item_cost, 0, size_t(b.num_items) * sizeof(uint32_t), st), "memset");
   stage_mark(st, 4);
-  const FwdArgs fa{n,           w.rec,   w.lists.list1, w.lists.off1, npad / kChunk, pair_capacity, w.task_order,
+  const FwdArgs fa{n,           w.rec,   w.lists.list1, w.lists.off1, w.L.sb_chunks, pair_capacity, w.task_order,
                    w.flags + 2, out_rgb, w.pix_T,       w.pix_stop,   target,        w.grad_pix,    w.slab_loss,
                    w.item_cost};
   TRY_CUDA(raster_fwd(st, b, fa),
@@ -793,7 +811,7 @@ int dsplat_gauss_batch_backward(dsplat_stream stream, const dsplat_gauss_params*
   // of the forward before it, the same measure as this forward's (equal once
   // the scene stops changing), and every order gives the same results
   stage_mark(st, 7);
-  const BwdArgs ba{n,           w.rec,    w.lists.list1,  w.lists.off1, w.L.npad / kChunk, pair_capacity,
+  const BwdArgs ba{n,           w.rec,    w.lists.list1,  w.lists.off1, w.L.sb_chunks, pair_capacity,
                    w.task_order, w.flags + 3, grad_rgb ? grad_rgb : w.grad_pix, w.pix_T, w.pix_stop, w.grad2d};
   TRY_CUDA(raster_bwd(st, b, ba),
            "raster_bwd");

@@ -337,30 +337,28 @@ __device__ __forceinline__ uint32_t local_rect(uint2 rc, int sl, int sx, int sy)
 
 constexpr int kMsThreads = 256;
 constexpr int kMsWarps = kMsThreads / 32;
-constexpr int kMsRounds = 16;
-constexpr int kMsChunk = kMsThreads * kMsRounds;  // 4096 ranks per chunk
 
 // ---------------------------------------------------------------------------
-// Stage 1a: per (chunk, superblock) counts.  Block = one chunk of 4096 ranks
-// of one view.  Output layout cnt[(sb_base[v] + s) * nchunk + c] so that an
+// Stage 1a: per (chunk, superblock) counts.  Block = one chunk of ranks (512
+// to 4096, choose_chunk in capi.cu) of one view.  Output layout cnt[(sb_base[v] + s) * nchunk + c] so that an
 // exclusive scan in index order yields (view, superblock, rank) positions.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(kMsThreads) k_sb_count(const uint32_t* __restrict__ order,
-                                                         const uint2* __restrict__ srect, uint32_t n, uint32_t npad,
+                                                         const uint2* __restrict__ srect, uint32_t chunk, uint32_t npad,
                                                          const ViewBatch b,
                                                          uint32_t* __restrict__ cnt,
                                                          unsigned long long* __restrict__ totals) {
   extern __shared__ uint32_t hist[];
-  const uint32_t nchunk = npad / kMsChunk;
+  const uint32_t nchunk = npad / chunk;
   const uint32_t v = blockIdx.x / nchunk, c = blockIdx.x % nchunk;
   const ViewDev& vd = b.v[v];
   const int sl = vd.sb_log2, sbw = sb_cols(vd), sbh = sb_rows(vd);
   const int nsb = sbw * sbh;
   for (int i = threadIdx.x; i < nsb; i += kMsThreads) hist[i] = 0;
   __syncthreads();
-  const size_t base = size_t(v) * npad + size_t(c) * kMsChunk;
+  const size_t base = size_t(v) * npad + size_t(c) * chunk;
   unsigned long long pairs = 0, entries = 0;
-  for (int i = threadIdx.x; i < kMsChunk; i += kMsThreads) {
+  for (uint32_t i = threadIdx.x; i < chunk; i += kMsThreads) {
     const uint2 rc = srect[base + i];
     int sx0, sy0, sx1, sy1;
     if (!sb_span(rc, sl, &sx0, &sy0, &sx1, &sy1)) continue;
@@ -388,34 +386,35 @@ __global__ void __launch_bounds__(kMsThreads) k_sb_count(const uint32_t* __restr
 
 // ---------------------------------------------------------------------------
 // Stage 1b: stable scatter of point indices into superblock lists.  Warp w
-// owns ranks [w*512, w*512+512) of the chunk in 16 rounds of 32.  In a round,
+// owns an eighth of the chunk's ranks in rounds of 32.  In a round,
 // each lane sets its bit in a shared mask per superblock column and row its
 // span covers; the lanes covering superblock (x, y) are then
 // colmask[x] & rowmask[y], and a lane's slot is its popcount among them.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(kMsThreads) k_sb_scatter(const uint32_t* __restrict__ order,
-                                                           const uint2* __restrict__ srect, uint32_t n, uint32_t npad,
+                                                           const uint2* __restrict__ srect, uint32_t chunk, uint32_t npad,
                                                            const ViewBatch b,
                                                            const uint32_t* __restrict__ off, uint64_t capacity,
                                                            uint2* __restrict__ list1, uint32_t* __restrict__ flags) {
   extern __shared__ uint32_t smem_ms[];  // [kMsWarps][nsb] counters, then [kMsWarps][2 * side] masks
-  const uint32_t nchunk = npad / kMsChunk;
+  const uint32_t nchunk = npad / chunk;
   const uint32_t v = blockIdx.x / nchunk, c = blockIdx.x % nchunk;
   const ViewDev& vd = b.v[v];
   const int sl = vd.sb_log2, sbw = sb_cols(vd), sbh = sb_rows(vd);
   const int nsb = sbw * sbh;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t lt = (1u << lane) - 1u;
+  const uint32_t rounds = chunk / kMsThreads;  // of 32 ranks per warp
   uint32_t* wc = smem_ms;
   const uint32_t side = b.max_sb_side;
   uint32_t* colmask = smem_ms + kMsWarps * b.max_sb + warp * 2 * side;
   uint32_t* rowmask = colmask + side;
   for (int i = threadIdx.x; i < kMsWarps * nsb; i += kMsThreads) wc[i] = 0;
   __syncthreads();
-  const size_t base = size_t(v) * npad + size_t(c) * kMsChunk + size_t(warp) * (kMsRounds * 32);
+  const size_t base = size_t(v) * npad + size_t(c) * chunk + size_t(warp) * (rounds * 32);
   uint32_t* my = wc + warp * nsb;
   // phase 1: per-warp counts
-  for (int r = 0; r < kMsRounds; ++r) {
+  for (uint32_t r = 0; r < rounds; ++r) {
     int sx0, sy0, sx1, sy1;
     if (sb_span(srect[base + r * 32 + lane], sl, &sx0, &sy0, &sx1, &sy1))
       for (int sy = sy0; sy < sy1; ++sy)
@@ -434,7 +433,7 @@ __global__ void __launch_bounds__(kMsThreads) k_sb_scatter(const uint32_t* __res
   }
   __syncthreads();
   // phase 3: stable scatter, round by round
-  for (int r = 0; r < kMsRounds; ++r) {
+  for (uint32_t r = 0; r < rounds; ++r) {
     const uint32_t g = order[base + r * 32 + lane];
     int sx0 = 0, sy0 = 0, sx1 = 0, sy1 = 0;
     const uint2 rc = srect[base + r * 32 + lane];
@@ -497,14 +496,14 @@ size_t sb_scatter_staged_smem(uint32_t max_sb, uint32_t max_side, uint32_t qcap)
 }
 
 __global__ void __launch_bounds__(kMsThreads) k_sb_scatter_staged(const uint32_t* __restrict__ order,
-                                                                  const uint2* __restrict__ srect, uint32_t n,
+                                                                  const uint2* __restrict__ srect, uint32_t chunk,
                                                                   uint32_t npad, const ViewBatch b,
                                                                   const uint32_t* __restrict__ off, uint64_t capacity,
                                                                   uint2* __restrict__ list1,
                                                                   uint32_t* __restrict__ flags, uint32_t qcap) {
   extern __shared__ uint32_t smem_ms[];
   __shared__ uint32_t sub_total;
-  const uint32_t nchunk = npad / kMsChunk;
+  const uint32_t nchunk = npad / chunk;
   const uint32_t v = blockIdx.x / nchunk, c = blockIdx.x % nchunk;
   const ViewDev& vd = b.v[v];
   const int sl = vd.sb_log2, sbw = sb_cols(vd), sbh = sb_rows(vd);
@@ -525,10 +524,10 @@ __global__ void __launch_bounds__(kMsThreads) k_sb_scatter_staged(const uint32_t
   for (int i = threadIdx.x; i < nsb; i += kMsThreads) cur[i] = off[(size_t(sb0) + i) * nchunk + c];
   const int seg = (nsb + kMsThreads - 1) / kMsThreads;
   const int s_lo = min(nsb, int(threadIdx.x) * seg), s_hi = min(nsb, s_lo + seg);
-  for (int sub = 0; sub < kMsChunk / kSubRanks; ++sub) {
+  for (uint32_t sub = 0; sub < chunk / kSubRanks; ++sub) {
     for (int i = threadIdx.x; i < kMsWarps * nsb; i += kMsThreads) wc[i] = 0;
     __syncthreads();
-    const size_t base = size_t(v) * npad + size_t(c) * kMsChunk + size_t(sub) * kSubRanks +
+    const size_t base = size_t(v) * npad + size_t(c) * chunk + size_t(sub) * kSubRanks +
                         size_t(warp) * (kSubRounds * 32);
     // per-warp counts of the sub-pass
     for (int r = 0; r < kSubRounds; ++r) {
