@@ -5,7 +5,7 @@
 Every .cu under csrc/ is compiled with nvcc for sm_100a only and linked into
 one shared library with the CUDA runtime linked statically, so the library
 does not depend on the libcudart that the host process (e.g. torch) loaded.
-project.cu, raster_fwd.cu and raster_blocks.cu are compiled with -fmad=false: their FP32
+project.cu and raster_fwd.cu are compiled with -fmad=false: their FP32
 results must match the CPU oracle bit for bit (tile spans and sort keys derive
 from the projection; the blend follows del-splat-cpu's operations), so no
 multiply-add may be fused that the source does not write as an fma.
@@ -30,8 +30,7 @@ LIB = os.path.join(OUT_DIR, "libdsplat.so")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-I", INCLUDE, "-I", CSRC,
           "--expt-relaxed-constexpr", "-Xptxas", "-v"]
-PER_FILE = {"project.cu": ["-fmad=false"], "raster_fwd.cu": ["-fmad=false"],
-            "raster_blocks.cu": ["-fmad=false"]}
+PER_FILE = {"project.cu": ["-fmad=false"], "raster_fwd.cu": ["-fmad=false"]}
 
 
 def nvcc() -> str:

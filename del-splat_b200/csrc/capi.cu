@@ -25,7 +25,6 @@ __global__ void k_project_bwd_colour(uint32_t, int, const float*, const float*, 
                                      float*, float*, unsigned long long*, unsigned long long);
 __global__ void k_prepare_grad2d(const unsigned long long*, unsigned long long, float4*, size_t);
 __global__ void k_adam(size_t, float*, const float*, float*, float*, float, float, float, float, float, float);
-bool raster_in_blocks(const ViewBatch&);
 __global__ void k_pad_keys(uint32_t*, uint32_t, uint32_t, uint32_t);
 __global__ void k_sb_count(const uint32_t*, const uint2*, uint32_t, uint32_t, const ViewBatch, uint32_t*,
                            unsigned long long*);
@@ -59,8 +58,8 @@ cudaError_t raster_bwd(cudaStream_t, const ViewBatch&, const BwdArgs&);
 bool raster_config_ok(int ts, int ppl);
 int raster_default_ppl(int ts);
 uint32_t raster_slabs_per_tile(int ts, int ppl);
-__global__ void k_order_hist(const ViewBatch, const uint32_t*, uint32_t, const uint32_t*, int, uint32_t*);
-__global__ void k_order_scatter(const ViewBatch, const uint32_t*, uint32_t, const uint32_t*, int, uint32_t*,
+__global__ void k_order_hist(const ViewBatch, const uint32_t*, uint32_t, const uint32_t*, uint32_t*);
+__global__ void k_order_scatter(const ViewBatch, const uint32_t*, uint32_t, const uint32_t*, float, uint32_t*,
                                 uint32_t*);
 cudaError_t raster_fwd_aos(cudaStream_t, int, int, int, float*, const float*, const float*, const float*, const float*,
                            const float*, const uint32_t*, const uint32_t*, float*, uint32_t*, bool);
@@ -230,13 +229,25 @@ int build_tile_lists(cudaStream_t st, const ViewBatch& b, uint32_t npad, const L
   return DSPLAT_OK;
 }
 
+// An item is heavy, walked in 8x8 blocks, when its longest task's cost is
+// above total / kHeavyShare: 0.375 of a resident warp's part (148 SMs, 24
+// warps each).  Forward and backward in us with every task whole, at 0.25, 0.5
+// and 1 of that part, and with every item heavy (8x8 tiles, SH 0):
+//   16 views, 1,048,576 Gaussians      3490 + 4730, 2930 + 3420, 2980 + 3510, 3110 + 3900, 3370 + 4390
+//   4 at 1280x720, 1,048,576           1450 + 1770, 1300 + 1480, 1300 + 1420, 1390 + 1550, 1320 + 1550
+//   one at 1280x720, 262,144            290 +  330,  215 +  244,  204 +  241,  201 +  232,  209 +  238
+//   8 at 640x480, 100,003               460 +  550,  374 +  478,  408 +  458,  444 +  511,  370 +  487
+constexpr float kHeavyShare = 148.f * 64.f;
+
 cudaError_t order_tasks(cudaStream_t st, const ViewBatch& b, const uint32_t* off1, uint32_t nchunk,
-                        const uint32_t* cost, int nt, uint32_t* sched, uint32_t* order) {
-  cudaError_t e = cudaMemsetAsync(sched, 0, 80 * sizeof(uint32_t), st);
+                        const uint32_t* cost, uint32_t* sched, uint32_t* order) {
+  cudaError_t e = cudaMemsetAsync(sched, 0, kSchedWords * sizeof(uint32_t), st);
   if (e != cudaSuccess) return e;
-  k_order_hist<<<296, 256, 0, st>>>(b, off1, nchunk, cost, nt, sched);
+  // costs are those of an item's longest task; its tasks share the total
+  const float share = kHeavyShare / float(b.ts == 8 ? 1u : raster_slabs_per_tile(b.ts, b.ppl));
+  k_order_hist<<<296, 256, 0, st>>>(b, off1, nchunk, cost, sched);
   count_launch();
-  k_order_scatter<<<296, 256, 0, st>>>(b, off1, nchunk, cost, nt, sched, order);
+  k_order_scatter<<<296, 256, 0, st>>>(b, off1, nchunk, cost, share, sched, order);
   count_launch();
   return cudaGetLastError();
 }
@@ -511,7 +522,7 @@ BatchWs carve_batch(void* ws, uint32_t n, const ViewBatch& b, uint64_t capacity)
   w.slab_loss = c.take<float>(size_t(b.num_items) * L.slabs_per_tile, &L.off_slab_loss);
   w.grad2d = c.take<float4>(3 * VN + 3, &L.off_grad2d);
   w.grad2d_tag = c.take<unsigned long long>(1);
-  w.sched = c.take<uint32_t>(80);
+  w.sched = c.take<uint32_t>(kSchedWords);
   w.task_order = c.take<uint32_t>(size_t(b.num_items) + 1);
   w.item_cost = c.take<uint32_t>(size_t(b.num_items) + 1);
   L.total_bytes = align_up(c.off, 256);
@@ -761,12 +772,11 @@ int dsplat_gauss_batch_forward(dsplat_stream stream, const dsplat_gauss_params* 
     stage_mark(st, 3);
   }
   // longest-first raster task order (costs measured by the previous forward)
-  TRY_CUDA(order_tasks(st, b, w.lists.off1, w.L.sb_chunks, w.item_cost, b.ts > 8 || raster_in_blocks(b) ? 1 : 2, w.sched,
-                       w.task_order),
+  TRY_CUDA(order_tasks(st, b, w.lists.off1, w.L.sb_chunks, w.item_cost, w.sched, w.task_order),
            "task order");
   TRY_CUDA(cudaMemsetAsync(w.item_cost, 0, size_t(b.num_items) * sizeof(uint32_t), st), "memset");
   stage_mark(st, 4);
-  const FwdArgs fa{n,           w.rec,   w.lists.list1, w.lists.off1, w.L.sb_chunks, pair_capacity, w.task_order,
+  const FwdArgs fa{n,           w.rec,   w.lists.list1, w.lists.off1, w.L.sb_chunks, pair_capacity, w.task_order, w.sched,
                    w.flags + 2, out_rgb, w.pix_T,       w.pix_stop,   target,        w.grad_pix,    w.slab_loss,
                    w.item_cost};
   TRY_CUDA(raster_fwd(st, b, fa),
@@ -812,7 +822,7 @@ int dsplat_gauss_batch_backward(dsplat_stream stream, const dsplat_gauss_params*
   // the scene stops changing), and every order gives the same results
   stage_mark(st, 7);
   const BwdArgs ba{n,           w.rec,    w.lists.list1,  w.lists.off1, w.L.sb_chunks, pair_capacity,
-                   w.task_order, w.flags + 3, grad_rgb ? grad_rgb : w.grad_pix, w.pix_T, w.pix_stop, w.grad2d};
+                   w.task_order, w.sched, w.flags + 3, grad_rgb ? grad_rgb : w.grad_pix, w.pix_T, w.pix_stop, w.grad2d};
   TRY_CUDA(raster_bwd(st, b, ba),
            "raster_bwd");
   stage_mark(st, 8);

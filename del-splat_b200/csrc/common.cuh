@@ -59,6 +59,7 @@ struct FwdArgs {
   uint32_t nchunk;
   uint64_t capacity;
   const uint32_t* order;
+  const uint32_t* sched;
   uint32_t* counter;
   float* out_rgb;
   float* out_T;
@@ -77,6 +78,7 @@ struct BwdArgs {
   uint32_t nchunk;
   uint64_t capacity;
   const uint32_t* order;
+  const uint32_t* sched;
   uint32_t* counter;
   const float* grad_pix;
   const float* pix_T;
@@ -85,6 +87,12 @@ struct BwdArgs {
 };
 
 
+
+// Words of the task schedule (order_tasks): bucket counts [0, 33), bucket
+// cursors [40, 73), and
+constexpr int kSchedCost = 74;   // u64: sum of the items' costs
+constexpr int kSchedHeavy = 76;  // leading items of the order walked in 8x8 blocks
+constexpr int kSchedWords = 80;
 
 // The five parameter tensors of one fused Adam launch (k_adam_fused).
 struct AdamSeg {

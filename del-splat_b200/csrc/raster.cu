@@ -5,8 +5,6 @@
 
 namespace dsplat {
 
-bool raster_in_blocks(const ViewBatch& b);
-
 // ---------------------------------------------------------------------------
 // Fused-path backward.  grad2d[(v*N+g)*3 + k] float4:
 //   (d px, d py, d A, d B) (d C, d opacity, d r, d g) (d b, 0, 0, 0)
@@ -81,190 +79,194 @@ __device__ __forceinline__ void red_flush(const RedBuf* red, int held, int lane,
 // the entry is in that pixel's own tile list, so each pixel sees exactly its
 // tile's entries (and its stop position is a position in the shared
 // superblock list).  The forward groups tiles the same way.
-//
-// BLOCK: the task is an 8x8-pixel block of a tile of any size instead, two
-// pixels per lane (the other template arguments then mean nothing): for
-// batches whose time is that of the longest walk.  The walks halve, the warp
-// reductions of an entry serve half the pixels: 3,000 Gaussians at 96x80 in
-// 16x16 tiles 228 -> 108 us, 262,144 at 1280x720 327 -> 233, 16 views of
-// 1,048,576 (not chosen) 3440 -> 4180.
+// Units of work as in the forward: heavy items in 8x8 blocks, two pixels per
+// lane (BlockGeo), the others in tasks of TaskGeo.  The walks of a block are
+// half as long per entry, the warp reductions of an entry serve half the
+// pixels: every unit a block, 3,000 Gaussians at 96x80 in 16x16 tiles 228 ->
+// 108 us, 262,144 at 1280x720 327 -> 233, 16 views of 1,048,576 3440 -> 4180.
 struct BlockGeo {
-  static constexpr int GX = 8, PPL = 2, ROW_STEP = 4, SLAB_ROWS = 8, SLABS = 1;
+  static constexpr int GX = 8, PPL = 2, ROW_STEP = 4;
 };
 
-template <int TS, int PPL_, int NT, bool BLOCK>
-__global__ void __launch_bounds__(32 * kRasterWarps, BLOCK || NT * PPL_ <= 4 ? 6 : 4) k_raster_bwd(
+// One task: 32 lanes over GX columns at (px0, py0), columns below xend.
+template <class GEO>
+__device__ __forceinline__ void bwd_task(const SbWalkSpan& walk, const PackedSrc& src, Ent* sm, RedBuf* red,
+                                         const ViewDev& vd, uint32_t s, uint32_t e, int px0, int py0, int xend,
+                                         const float* __restrict__ grad_pix, const float* __restrict__ pix_T,
+                                         const uint32_t* __restrict__ pix_last, float* __restrict__ gv) {
+  constexpr int PPL = GEO::PPL, NP = PPL / 2;
+  static_assert(PPL % 2 == 0, "pixels are evaluated in pairs");
+  const int lane = threadIdx.x & 31;
+  const int ix = px0 + lane % GEO::GX, iy0 = py0 + lane / GEO::GX;
+  const bool col_in = ix < xend;
+  const float fx = float(ix) + 0.5f;
+  // per pixel pair: T in front of the current entry, nS = -(d . colour
+  // behind it), d = dL/dpixel; per pixel the stop position
+  f2 Tc[NP], nS[NP], d0[NP], d1[NP], d2[NP], fy2[NP];
+  uint32_t last[PPL];
+  uint32_t lo_min = e;
+#pragma unroll
+  for (int q = 0; q < NP; ++q) {
+    float t[2] = {1.f, 1.f}, g0[2] = {0.f, 0.f}, g1[2] = {0.f, 0.f}, g2[2] = {0.f, 0.f}, y[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int k = 2 * q + h, iy = iy0 + k * GEO::ROW_STEP;
+      y[h] = float(iy) + 0.5f;
+      last[k] = e;  // outside pixels process nothing
+      if (col_in && ix < vd.w && iy < vd.h) {
+        const size_t p = size_t(vd.pix_base) + size_t(iy) * vd.w + ix;
+        t[h] = pix_T[p];
+        last[k] = pix_last[p];
+        g0[h] = grad_pix[3 * p];
+        g1[h] = grad_pix[3 * p + 1];
+        g2[h] = grad_pix[3 * p + 2];
+        lo_min = min(lo_min, last[k]);
+      }
+    }
+    Tc[q] = f2_make(t[0], t[1]);
+    nS[q] = f2_make(0.f, 0.f);
+    d0[q] = f2_make(g0[0], g0[1]);
+    d1[q] = f2_make(g1[0], g1[1]);
+    d2[q] = f2_make(g2[0], g2[1]);
+    fy2[q] = f2_make(y[0], y[1]);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) lo_min = min(lo_min, __shfl_xor_sync(0xffffffffu, lo_min, o));
+  const uint32_t lo0 = max(s, lo_min);
+  int held = 0;  // entries waiting in red
+  uint2 en = lo0 < e ? walk.load(lo0 + uint32_t(lane), uint32_t(lane) < e - lo0) : make_uint2(0u, 0u);
+  for (uint32_t lo = lo0; lo < e; lo += 32) {
+    const int cnt = int(min(32u, e - lo));
+    int k_staged;
+    if (GEO::GX == 8) {  // of the tiles' entries those whose box reaches the block's pixel centres
+      const float cx = float(px0) + 4.f, cy = float(py0) + 4.f;
+      bool hit = lane < cnt && walk.hit(en);
+      if (hit) {
+        const float4 r0 = __ldg(src.rec + 3 * size_t(en.x)), r2 = __ldg(src.rec + 3 * size_t(en.x) + 2);
+        hit = fabsf(r0.x - cx) <= r2.y + 4.f && fabsf(r0.y - cy) <= r2.z + 4.f;
+      }
+      const uint32_t bal = __ballot_sync(0xffffffffu, hit);
+      if (hit) {
+        Ent* dst = &sm[__popc(bal & ((1u << lane) - 1u))];
+        src.stage(dst, en.x);
+        dst->set_pos(lo + uint32_t(lane));
+      }
+      k_staged = __popc(bal);
+    } else {
+      k_staged = walk.stage(src, sm, en, lo + uint32_t(lane), lane < cnt, lane);
+    }
+    // the next batch's list words arrive while this batch is processed
+    if (lo + 32u < e) en = walk.load(lo + 32u + uint32_t(lane), uint32_t(lane) < e - (lo + 32u));
+    __syncwarp();
+    for (int j = 0; j < k_staged; ++j) {
+      const float4 ed = sm[j].d, ee = sm[j].e;
+      const uint32_t pos = __float_as_uint(sm[j].f.x);
+      // this lane's sums over its pixels, pair halves apart: t = G dL/dalpha
+      // (its sum is dL/dop; w = dL/dq = -op/2 t), t dy, t dy^2, and the
+      // negated dL/dcolour
+      f2 st = 0, sty = 0, styy = 0, nr = 0, ng = 0, nb = 0;
+      bool any = false;
+      const float dx = fx - ed.x;
+      if (ee.x <= fx && fx <= ee.y) {
+        const ulonglong2 qa = *reinterpret_cast<const ulonglong2*>(&sm[j].a);
+        const ulonglong2 qb = *reinterpret_cast<const ulonglong2*>(&sm[j].b);
+        const ulonglong2 qc = *reinterpret_cast<const ulonglong2*>(&sm[j].c);
+        const f2 kadxdx = f2_dup(ed.y * dx * dx), kb2dx = f2_dup(ed.z * dx);
+#pragma unroll
+        for (int q = 0; q < NP; ++q) {
+          const float fy0 = f2_lo(fy2[q]), fy1 = f2_hi(fy2[q]);
+          const bool in0 = pos >= last[2 * q] && ee.z <= fy0 && fy0 <= ee.w;
+          const bool in1 = pos >= last[2 * q + 1] && ee.z <= fy1 && fy1 <= ee.w;
+          if (!(in0 || in1)) continue;
+          any = true;
+          const f2 dy = sub2(fy2[q], qa.x);
+          const f2 y = fma2(fma2(qa.y, dy, kb2dx), dy, kadxdx);  // k q
+          // a pixel outside the box or past its stop takes G = 0: alpha 0,
+          // 1 / (1 - alpha) = 1, every sum unchanged
+          const f2 Gv = f2_make(in0 ? ex2_approx(f2_lo(y)) : 0.f, in1 ? ex2_approx(f2_hi(y)) : 0.f);
+          const f2 nal = mul2(Gv, qb.x);  // -alpha
+          // alpha < 1 is a precondition (opacity < 1); the floor only
+          // keeps gradients finite if an input breaks it
+          const f2 om = add2(nal, f2_dup(1.f));
+          const f2 iom = f2_make(rcp_approx(fmaxf(f2_lo(om), 1e-7f)), rcp_approx(fmaxf(f2_hi(om), 1e-7f)));
+          Tc[q] = mul2(Tc[q], iom);
+          const f2 nw = mul2(nal, Tc[q]);  // -alpha T
+          const f2 drgb = fma2(d2[q], qc.y, fma2(d1[q], qc.x, mul2(d0[q], qb.y)));
+          const f2 dLde = fma2(iom, nS[q], mul2(Tc[q], drgb));
+          nS[q] = fma2(nw, drgb, nS[q]);
+          nr = fma2(nw, d0[q], nr);
+          ng = fma2(nw, d1[q], ng);
+          nb = fma2(nw, d2[q], nb);
+          const f2 t = mul2(Gv, dLde);
+          st = add2(st, t);
+          const f2 ty = mul2(t, dy);
+          sty = add2(sty, ty);
+          styy = fma2(ty, dy, styy);
+        }
+      }
+      if (__any_sync(0xffffffffu, any)) {
+        const float s_t = f2_lo(st) + f2_hi(st), s_ty = f2_lo(sty) + f2_hi(sty), s_tx = s_t * dx;
+        red->row[held][0][lane] = s_tx;
+        red->row[held][1][lane] = s_ty;
+        red->row[held][2][lane] = s_tx * dx;
+        red->row[held][3][lane] = s_ty * dx;
+        red->row[held][4][lane] = f2_lo(styy) + f2_hi(styy);
+        red->row[held][5][lane] = s_t;
+        red->row[held][6][lane] = f2_lo(nr) + f2_hi(nr);
+        red->row[held][7][lane] = f2_lo(ng) + f2_hi(ng);
+        red->row[held][8][lane] = f2_lo(nb) + f2_hi(nb);
+        // what the flush needs of the entry, in the rows' padding (every
+        // lane stores the same words)
+        *reinterpret_cast<float4*>(&red->row[held][0][32]) = make_float4(ed.y, ed.z, sm[j].a.z, sm[j].b.x);
+        red->row[held][1][32] = ed.w;
+        if (++held == kRedEntries) {
+          red_flush(red, held, lane, gv);
+          held = 0;
+        }
+      }
+    }
+    __syncwarp();
+  }
+  if (held) red_flush(red, held, lane, gv);
+}
+
+template <int TS, int PPL_, int NT>
+__global__ void __launch_bounds__(32 * kRasterWarps, NT * PPL_ <= 4 ? 6 : 4) k_raster_bwd(
     const ViewBatch b, uint32_t n, const float4* __restrict__ rec, const uint2* __restrict__ list1,
     const uint32_t* __restrict__ off1, uint32_t nchunk, uint64_t capacity, const uint32_t* __restrict__ order,
-    uint32_t* __restrict__ work_counter, const float* __restrict__ grad_pix, const float* __restrict__ pix_T,
-    const uint32_t* __restrict__ pix_last, float4* __restrict__ grad2d) {
-  using G = typename std::conditional<BLOCK, BlockGeo, TaskGeo<BLOCK ? 8 : TS, BLOCK ? 2 : PPL_, NT>>::type;
-  constexpr int PPL = G::PPL, NP = PPL / 2;
-  static_assert(PPL % 2 == 0, "pixels are evaluated in pairs");
+    const uint32_t* __restrict__ sched, uint32_t* __restrict__ work_counter, const float* __restrict__ grad_pix,
+    const float* __restrict__ pix_T, const uint32_t* __restrict__ pix_last, float4* __restrict__ grad2d) {
+  using G = TaskGeo<TS, PPL_, NT>;
   __shared__ Ent sm_all[kRasterWarps][32];
   __shared__ RedBuf red_all[kRasterWarps];
   Ent* sm = sm_all[threadIdx.x >> 5];
   RedBuf* red = &red_all[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
-  const uint32_t side = BLOCK ? uint32_t(b.ts) / 8u : 1u, per_item = BLOCK ? side * side : uint32_t(G::SLABS);
-  const uint32_t num_tasks = b.num_items * per_item;
   for (;;) {
-    uint32_t task = 0;
-    if (lane == 0) task = atomicAdd(work_counter, 1u);
-    task = __shfl_sync(0xffffffffu, task, 0);
-    if (task >= num_tasks) return;
-    const uint32_t item = order[task / per_item];
-    uint32_t slab = task % per_item;
-    ItemGeo ig = item_geo(b, item, off1, nchunk, capacity);
+    uint32_t i = 0;
+    if (lane == 0) i = atomicAdd(work_counter, 1u);
+    const Task t(b, __shfl_sync(0xffffffffu, i, 0), order, sched, G::SLABS);
+    if (t.none) return;
+    const ItemGeo ig = item_geo(b, t.item, off1, nchunk, capacity);
     const ViewDev& vd = b.v[ig.v];
-    if (BLOCK) {
-      ig.px0 += int(slab % side) * 8;
-      ig.py0 += int(slab / side) * 8;
-      slab = 0;
-    }
-    // tiles of this task: 1, or 2 when the superblock holds the right neighbour
+    // tiles of the item's tasks: 1, or 2 when the superblock holds the right
+    // neighbour; the run's leftmost tile carries them
     uint32_t nx = 1;
     if (NT > 1) {
       nx = min(uint32_t(NT), 1u << vd.sb_log2);
-      if (ig.lx % nx) continue;  // the group's leftmost tile carries it
+      if (ig.lx % nx) continue;
     }
-    const int col = lane % G::GX;
-    const int ix = ig.px0 + col;
-    const int iy0 = ig.py0 + int(slab) * G::SLAB_ROWS + (lane / G::GX);
-    const bool col_in = BLOCK || col < int(nx) * TS;
-    const float fx = float(ix) + 0.5f;
-    const uint32_t s = ig.s, e = ig.e;
-    // per pixel pair: T in front of the current entry, nS = -(d . colour
-    // behind it), d = dL/dpixel; per pixel the stop position
-    f2 Tc[NP], nS[NP], d0[NP], d1[NP], d2[NP], fy2[NP];
-    uint32_t last[PPL];
-    uint32_t lo_min = e;
-#pragma unroll
-    for (int q = 0; q < NP; ++q) {
-      float t[2] = {1.f, 1.f}, g0[2] = {0.f, 0.f}, g1[2] = {0.f, 0.f}, g2[2] = {0.f, 0.f}, y[2];
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int k = 2 * q + h, iy = iy0 + k * G::ROW_STEP;
-        y[h] = float(iy) + 0.5f;
-        last[k] = e;  // outside pixels process nothing
-        if (col_in && ix < vd.w && iy < vd.h) {
-          const size_t p = size_t(vd.pix_base) + size_t(iy) * vd.w + ix;
-          t[h] = pix_T[p];
-          last[k] = pix_last[p];
-          g0[h] = grad_pix[3 * p];
-          g1[h] = grad_pix[3 * p + 1];
-          g2[h] = grad_pix[3 * p + 2];
-          lo_min = min(lo_min, last[k]);
-        }
-      }
-      Tc[q] = f2_make(t[0], t[1]);
-      nS[q] = f2_make(0.f, 0.f);
-      d0[q] = f2_make(g0[0], g0[1]);
-      d1[q] = f2_make(g1[0], g1[1]);
-      d2[q] = f2_make(g2[0], g2[1]);
-      fy2[q] = f2_make(y[0], y[1]);
+    const PackedSrc src{rec + 3 * size_t(ig.v) * n};
+    float* const gv = reinterpret_cast<float*>(grad2d + 3 * size_t(ig.v) * n);
+    if (t.block) {
+      BlockPlace p;
+      if (!block_place(b, ig, t.sub, nx, &p)) continue;
+      bwd_task<BlockGeo>(SbWalkSpan{list1, p.lx, ig.ly, 1u}, src, sm, red, vd, ig.s, ig.e, p.px0, p.py0, vd.w, grad_pix,
+                         pix_T, pix_last, gv);
+    } else {
+      bwd_task<G>(SbWalkSpan{list1, ig.lx, ig.ly, nx}, src, sm, red, vd, ig.s, ig.e, ig.px0,
+                  ig.py0 + int(t.sub) * G::SLAB_ROWS, min(vd.w, ig.px0 + int(nx) * TS), grad_pix, pix_T, pix_last, gv);
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) lo_min = min(lo_min, __shfl_xor_sync(0xffffffffu, lo_min, o));
-    PackedSrc src{rec + 3 * size_t(ig.v) * n};
-    SbWalkSpan walk{list1, ig.lx, ig.ly, nx};
-    float* gv = reinterpret_cast<float*>(grad2d + 3 * size_t(ig.v) * n);
-    const uint32_t lo0 = max(s, lo_min);
-    int held = 0;  // entries waiting in red
-    uint2 en = lo0 < e ? walk.load(lo0 + uint32_t(lane), uint32_t(lane) < e - lo0) : make_uint2(0u, 0u);
-    for (uint32_t lo = lo0; lo < e; lo += 32) {
-      const int cnt = int(min(32u, e - lo));
-      int k_staged;
-      if (BLOCK) {  // of the tile's entries those whose box reaches the block's pixel centres
-        const float cx = float(ig.px0) + 4.f, cy = float(ig.py0) + 4.f;
-        bool hit = lane < cnt && walk.hit(en);
-        if (hit && b.ts > 8) {
-          const float4 r0 = __ldg(src.rec + 3 * size_t(en.x)), r2 = __ldg(src.rec + 3 * size_t(en.x) + 2);
-          hit = fabsf(r0.x - cx) <= r2.y + 4.f && fabsf(r0.y - cy) <= r2.z + 4.f;
-        }
-        const uint32_t bal = __ballot_sync(0xffffffffu, hit);
-        if (hit) {
-          Ent* dst = &sm[__popc(bal & ((1u << lane) - 1u))];
-          src.stage(dst, en.x);
-          dst->set_pos(lo + uint32_t(lane));
-        }
-        k_staged = __popc(bal);
-      } else {
-        k_staged = walk.stage(src, sm, en, lo + uint32_t(lane), lane < cnt, lane);
-      }
-      // the next batch's list words arrive while this batch is processed
-      if (lo + 32u < e) en = walk.load(lo + 32u + uint32_t(lane), uint32_t(lane) < e - (lo + 32u));
-      __syncwarp();
-      for (int j = 0; j < k_staged; ++j) {
-        const float4 ed = sm[j].d, ee = sm[j].e;
-        const uint32_t pos = __float_as_uint(sm[j].f.x);
-        // this lane's sums over its pixels, pair halves apart: t = G dL/dalpha
-        // (its sum is dL/dop; w = dL/dq = -op/2 t), t dy, t dy^2, and the
-        // negated dL/dcolour
-        f2 st = 0, sty = 0, styy = 0, nr = 0, ng = 0, nb = 0;
-        bool any = false;
-        const float dx = fx - ed.x;
-        if (ee.x <= fx && fx <= ee.y) {
-          const ulonglong2 qa = *reinterpret_cast<const ulonglong2*>(&sm[j].a);
-          const ulonglong2 qb = *reinterpret_cast<const ulonglong2*>(&sm[j].b);
-          const ulonglong2 qc = *reinterpret_cast<const ulonglong2*>(&sm[j].c);
-          const f2 kadxdx = f2_dup(ed.y * dx * dx), kb2dx = f2_dup(ed.z * dx);
-#pragma unroll
-          for (int q = 0; q < NP; ++q) {
-            const float fy0 = f2_lo(fy2[q]), fy1 = f2_hi(fy2[q]);
-            const bool in0 = pos >= last[2 * q] && ee.z <= fy0 && fy0 <= ee.w;
-            const bool in1 = pos >= last[2 * q + 1] && ee.z <= fy1 && fy1 <= ee.w;
-            if (!(in0 || in1)) continue;
-            any = true;
-            const f2 dy = sub2(fy2[q], qa.x);
-            const f2 y = fma2(fma2(qa.y, dy, kb2dx), dy, kadxdx);  // k q
-            // a pixel outside the box or past its stop takes G = 0: alpha 0,
-            // 1 / (1 - alpha) = 1, every sum unchanged
-            const f2 Gv = f2_make(in0 ? ex2_approx(f2_lo(y)) : 0.f, in1 ? ex2_approx(f2_hi(y)) : 0.f);
-            const f2 nal = mul2(Gv, qb.x);  // -alpha
-            // alpha < 1 is a precondition (opacity < 1); the floor only
-            // keeps gradients finite if an input breaks it
-            const f2 om = add2(nal, f2_dup(1.f));
-            const f2 iom = f2_make(rcp_approx(fmaxf(f2_lo(om), 1e-7f)), rcp_approx(fmaxf(f2_hi(om), 1e-7f)));
-            Tc[q] = mul2(Tc[q], iom);
-            const f2 nw = mul2(nal, Tc[q]);  // -alpha T
-            const f2 drgb = fma2(d2[q], qc.y, fma2(d1[q], qc.x, mul2(d0[q], qb.y)));
-            const f2 dLde = fma2(iom, nS[q], mul2(Tc[q], drgb));
-            nS[q] = fma2(nw, drgb, nS[q]);
-            nr = fma2(nw, d0[q], nr);
-            ng = fma2(nw, d1[q], ng);
-            nb = fma2(nw, d2[q], nb);
-            const f2 t = mul2(Gv, dLde);
-            st = add2(st, t);
-            const f2 ty = mul2(t, dy);
-            sty = add2(sty, ty);
-            styy = fma2(ty, dy, styy);
-          }
-        }
-        if (__any_sync(0xffffffffu, any)) {
-          const float s_t = f2_lo(st) + f2_hi(st), s_ty = f2_lo(sty) + f2_hi(sty), s_tx = s_t * dx;
-          red->row[held][0][lane] = s_tx;
-          red->row[held][1][lane] = s_ty;
-          red->row[held][2][lane] = s_tx * dx;
-          red->row[held][3][lane] = s_ty * dx;
-          red->row[held][4][lane] = f2_lo(styy) + f2_hi(styy);
-          red->row[held][5][lane] = s_t;
-          red->row[held][6][lane] = f2_lo(nr) + f2_hi(nr);
-          red->row[held][7][lane] = f2_lo(ng) + f2_hi(ng);
-          red->row[held][8][lane] = f2_lo(nb) + f2_hi(nb);
-          // what the flush needs of the entry, in the rows' padding (every
-          // lane stores the same words)
-          *reinterpret_cast<float4*>(&red->row[held][0][32]) = make_float4(ed.y, ed.z, sm[j].a.z, sm[j].b.x);
-          red->row[held][1][32] = ed.w;
-          if (++held == kRedEntries) {
-            red_flush(red, held, lane, gv);
-            held = 0;
-          }
-        }
-      }
-      __syncwarp();
-    }
-    if (held) red_flush(red, held, lane, gv);
   }
 }
 
@@ -321,26 +323,20 @@ bool raster_config_ok(int ts, int ppl) {
 int raster_default_ppl(int ts) { return ts == 8 ? 2 : 4; }
 uint32_t raster_slabs_per_tile(int ts, int ppl) { return uint32_t(ts * ts / (32 * ppl)); }
 
-template <int TS, int PPL, int NT, bool BLOCK>
-static cudaError_t launch_bwd(cudaStream_t st, const ViewBatch& b, const BwdArgs& a, uint32_t tasks) {
-  k_raster_bwd<TS, PPL, NT, BLOCK>
-      <<<persistent_grid(k_raster_bwd<TS, PPL, NT, BLOCK>, tasks), 32 * kRasterWarps, 0, st>>>(
-          b, a.n, a.rec, a.list1, a.off1, a.nchunk, a.capacity, a.order, a.counter, a.grad_pix, a.pix_T, a.pix_last,
-          a.grad2d);
+template <int TS, int PPL>
+static cudaError_t launch_bwd(cudaStream_t st, const ViewBatch& b, const BwdArgs& a) {
+  constexpr int NT = TS == 8 ? kBwdGroup8 : 1;
+  k_raster_bwd<TS, PPL, NT>
+      <<<persistent_grid(k_raster_bwd<TS, PPL, NT>, max_tasks(b, TaskGeo<TS, PPL, NT>::SLABS)), 32 * kRasterWarps, 0,
+         st>>>(b, a.n, a.rec, a.list1, a.off1, a.nchunk, a.capacity, a.order, a.sched, a.counter, a.grad_pix, a.pix_T,
+               a.pix_last, a.grad2d);
   count_launch();
   return cudaGetLastError();
 }
 
 cudaError_t raster_bwd(cudaStream_t st, const ViewBatch& b, const BwdArgs& a) {
-  if (raster_in_blocks(b)) {  // the rule and its figures are in raster_fwd.cu
-    const uint32_t side = uint32_t(b.ts) / 8u;
-    return launch_bwd<8, 1, 1, true>(st, b, a, b.num_items * side * side);
-  }
-#define X(T, P)                                                                              \
-  if (b.ts == T && b.ppl == P) {                                                             \
-    constexpr int NT = T == 8 ? kBwdGroup8 : 1;                                              \
-    return launch_bwd<T, P, NT, false>(st, b, a, b.num_items * TaskGeo<T, P, NT>::SLABS);    \
-  }
+#define X(T, P) \
+  if (b.ts == T && b.ppl == P) return launch_bwd<T, P>(st, b, a);
   DSPLAT_RASTER_CONFIGS(X)
 #undef X
   return cudaErrorInvalidValue;

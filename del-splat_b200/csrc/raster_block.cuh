@@ -1,26 +1,22 @@
-// raster_blocks.cu -- the forward rasteriser for batches that do not fill the
-// GPU many times over, and the drop-in one (see raster_fwd.cu for the others,
-// for the rule between them and for the blend's arithmetic rules, which hold
-// here too; built with -fmad=false).
+// raster_block.cuh -- the forward's walk of an 8x8-pixel block (raster_fwd.cu,
+// which also has the rule for its use and the blend's arithmetic rules).
 //
-// Bound: the longest walk.  A tile of a scene's rim, whose pixels never
+// Bound: the walk's length.  A tile of a scene's rim, whose pixels never
 // saturate, walks ten times the mean list, and a warp alone on its scheduler
-// issues an instruction every four to five cycles, so such a batch takes as
-// long as its longest task.  The task here is 8x8 pixels for every tile size,
-// a pair of pixels per lane: half the instructions per entry of raster_fwd's
-// 16x8 tasks and twice the tasks, for about 15% more instructions in all.
-// Measured (us, raster_fwd's tasks -> here): 3,000 Gaussians at 96x80 in 16x16
-// tiles 200 -> 80, 262,144 at 1280x720 288 -> 211; the drop-in forward (16x16
-// tiles): 1,000 at 96x64 73 -> 34, 16,384 at 256x256 127 -> 72, 1,048,576 at
-// 1920x1080 644 -> 601.  Two entries at a time, so that their exponentials
-// overlap, were no faster for the short batches and slower for the others.
-#include <algorithm>
-
+// issues an instruction every four to five cycles, so a batch that does not
+// fill the GPU many times over takes as long as its longest tasks.  A block
+// has a pair of pixels per lane: half the instructions per entry of the 16x8
+// tasks and twice the tasks, for about 15% more instructions in all.
+// Measured (us, every task 16x8 -> every task a block): 3,000 Gaussians at
+// 96x80 in 16x16 tiles 200 -> 80, 262,144 at 1280x720 288 -> 211; the drop-in
+// forward (16x16 tiles): 1,000 at 96x64 73 -> 34, 16,384 at 256x256 127 -> 72,
+// 1,048,576 at 1920x1080 644 -> 601.  Two entries at a time, so that their
+// exponentials overlap, were no faster for the short batches and slower for
+// the others.
+#pragma once
 #include "raster_common.cuh"
 
 namespace dsplat {
-
-uint32_t raster_slabs_per_tile(int ts, int ppl);
 
 // The task: a block of 8x8 pixels, lane L at column L % 8 and rows
 // L / 8 and L / 8 + 4 (its two pixel slots), for every tile size.
@@ -161,26 +157,22 @@ struct SbWords {
 // 0.999f, its double comparison) instead of del-splat-cpu's (> 0.999f).
 // Returns the cost of the walk (in units of a few warp-instructions).
 // ---------------------------------------------------------------------------
-struct FwdWarp {  // a warp's shared memory
-  EntB ent[32];
-  float4 park[2][32];      // T, r, g, b of a stopped pixel
-  uint32_t park_pos[2][32];  // and its stop position
-};
-
 struct FwdOut {  // where a block's results go
   float* rgb;
   float* T;         // nullable
   uint32_t* last;   // nullable
-  const float* target;  // nullable; with it:
+  const float* target;  // nullable; with it grad_pix and the loss
   float* grad_pix;
-  float* loss;      // the block's partial L2 loss
-  bool loss_add;    // several blocks share the slot
 };
 
-template <bool CUDA_STOP, class Walk, class Src>
-__device__ __forceinline__ uint32_t blend_block(const Walk& walk, const Src& src, FwdWarp& sh, const float* tab, float nz,
+// ent, park (T, r, g, b of a stopped pixel) and park_pos (its stop position),
+// 32, 64 and 64 of them, are the warp's in shared memory; loss(l) takes the
+// block's partial L2 loss (lane 0).
+template <bool CUDA_STOP, class Walk, class Src, class Loss>
+__device__ __forceinline__ uint32_t blend_block(const Walk& walk, const Src& src, EntB* ent_sm, float4* park,
+                                              uint32_t* park_pos, const float* tab, float nz,
                                               uint32_t s, uint32_t e, int px0, int py0, int w, int xend, int yend,
-                                              bool accumulate, size_t pix_base, const FwdOut& out) {
+                                              bool accumulate, size_t pix_base, const FwdOut& out, const Loss& loss) {
   const int lane = threadIdx.x & 31;
   const uint32_t bit = 1u << lane;
   const int ix = px0 + (lane & 7), iy = py0 + (lane >> 3);
@@ -219,8 +211,8 @@ __device__ __forceinline__ uint32_t blend_block(const Walk& walk, const Src& src
     a = fa(a, eo);
     if (CUDA_STOP ? a >= kAlphaStop : a > kAlphaStop) {
       (k ? live1 : live0) = 0u;
-      sh.park[k][lane] = make_float4(T, r, g, b);
-      sh.park_pos[k][lane] = ent.pos;
+      park[32 * k + lane] = make_float4(T, r, g, b);
+      park_pos[32 * k + lane] = ent.pos;
       a = -INFINITY;
     }
     T2 = k ? f2_make(f2_lo(T2), T) : f2_make(T, f2_hi(T2));
@@ -245,7 +237,7 @@ __device__ __forceinline__ uint32_t blend_block(const Walk& walk, const Src& src
     const uint32_t bal = __ballot_sync(0xffffffffu, hit);
     int staged = __popc(bal);
     bool odd = false;
-    if (hit) odd = src.stage(&sh.ent[__popc(bal & (bit - 1u))], g, hi - 1u - uint32_t(lane), mask);
+    if (hit) odd = src.stage(&ent_sm[__popc(bal & (bit - 1u))], g, hi - 1u - uint32_t(lane), mask);
     const bool odd_colour = __any_sync(0xffffffffu, odd);
     hi -= cnt;
     cost += kCostBatch + uint32_t(staged) * kCostEntry;
@@ -254,14 +246,14 @@ __device__ __forceinline__ uint32_t blend_block(const Walk& walk, const Src& src
     __syncwarp();
     if (odd_colour) {
       for (int j = 0; j < staged; ++j) {
-        const EntB& ent = sh.ent[j];
+        const EntB& ent = ent_sm[j];
         if (ent.mask.x & live0) blend_one(ent, 0);
         if (ent.mask.y & live1) blend_one(ent, 1);
       }
       staged = 0;
     }
     for (int j = 0; j < staged; ++j) {
-      const EntB& ent = sh.ent[j];
+      const EntB& ent = ent_sm[j];
       // which of the lane's pixels the entry's box holds and that still blend
       const bool a0 = (ent.mask.x & live0) != 0u, a1 = (ent.mask.y & live1) != 0u;
       if (!(a0 || a1)) continue;
@@ -296,14 +288,14 @@ __device__ __forceinline__ uint32_t blend_block(const Walk& walk, const Src& src
         float s0 = f2_lo(as2), s1 = f2_hi(as2);
         if (CUDA_STOP ? s0 >= kAlphaStop : s0 > kAlphaStop) {
           live0 = 0u;
-          sh.park[0][lane] = make_float4(f2_lo(T2), f2_lo(c0), f2_lo(c1), f2_lo(c2));
-          sh.park_pos[0][lane] = ent.pos;
+          park[lane] = make_float4(f2_lo(T2), f2_lo(c0), f2_lo(c1), f2_lo(c2));
+          park_pos[lane] = ent.pos;
           s0 = -INFINITY;
         }
         if (CUDA_STOP ? s1 >= kAlphaStop : s1 > kAlphaStop) {
           live1 = 0u;
-          sh.park[1][lane] = make_float4(f2_hi(T2), f2_hi(c0), f2_hi(c1), f2_hi(c2));
-          sh.park_pos[1][lane] = ent.pos;
+          park[32 + lane] = make_float4(f2_hi(T2), f2_hi(c0), f2_hi(c1), f2_hi(c2));
+          park_pos[32 + lane] = ent.pos;
           s1 = -INFINITY;
         }
         as2 = f2_make(s0, s1);
@@ -314,24 +306,24 @@ __device__ __forceinline__ uint32_t blend_block(const Walk& walk, const Src& src
   }
   // pixels still walking at the end walked the whole list (stop position s)
   if (live0) {
-    sh.park[0][lane] = make_float4(f2_lo(T2), f2_lo(c0), f2_lo(c1), f2_lo(c2));
-    sh.park_pos[0][lane] = s;
+    park[lane] = make_float4(f2_lo(T2), f2_lo(c0), f2_lo(c1), f2_lo(c2));
+    park_pos[lane] = s;
   }
   if (live1) {
-    sh.park[1][lane] = make_float4(f2_hi(T2), f2_hi(c0), f2_hi(c1), f2_hi(c2));
-    sh.park_pos[1][lane] = s;
+    park[32 + lane] = make_float4(f2_hi(T2), f2_hi(c0), f2_hi(c1), f2_hi(c2));
+    park_pos[32 + lane] = s;
   }
   float l = 0.f;
 #pragma unroll
   for (int k = 0; k < 2; ++k) {
     if (!(k ? in1 : in0)) continue;
-    const float4 o = sh.park[k][lane];
+    const float4 o = park[32 * k + lane];
     const size_t p = k ? p1 : p0;
     out.rgb[3 * p] = o.y;
     out.rgb[3 * p + 1] = o.z;
     out.rgb[3 * p + 2] = o.w;
     if (out.T) out.T[p] = o.x;
-    if (out.last) out.last[p] = sh.park_pos[k][lane];
+    if (out.last) out.last[p] = park_pos[32 * k + lane];
     if (out.target) {
       const float d0 = o.y - out.target[3 * p], d1 = o.z - out.target[3 * p + 1], d2 = o.w - out.target[3 * p + 2];
       out.grad_pix[3 * p] = 2.f * d0;
@@ -343,106 +335,10 @@ __device__ __forceinline__ uint32_t blend_block(const Walk& walk, const Src& src
   if (out.target) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-    if (lane == 0) {
-      if (out.loss_add) atomicAdd(out.loss, l);
-      else *out.loss = l;
-    }
+    if (lane == 0) loss(l);
   }
   __syncwarp();
   return cost;
-}
-
-// ---------------------------------------------------------------------------
-// Fused-path forward: persistent, per-warp work stealing over 8x8 blocks,
-// walking each tile's entries out of its superblock list.  A tile of 16 or 32
-// pixels is 4 or 16 tasks.  slab_loss: `slots` partial L2 losses per tile
-// (when target is given; zero at the start unless slots equals the tile's
-// block count), blocks in order sharing them evenly.
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(32 * kRasterWarps, 6) k_raster_blocks(
-    const ViewBatch b, uint32_t n, const float4* __restrict__ rec, const uint2* __restrict__ list1,
-    const uint32_t* __restrict__ off1, uint32_t nchunk, uint64_t capacity, const uint32_t* __restrict__ order,
-    uint32_t* __restrict__ work_counter, float* __restrict__ out_rgb, float* __restrict__ out_T,
-    uint32_t* __restrict__ out_last, const float* __restrict__ target, float* __restrict__ grad_pix,
-    float* __restrict__ slab_loss, uint32_t slots, uint32_t* __restrict__ item_cost, float nz) {
-  __shared__ FwdWarp sh[kRasterWarps];
-  __shared__ float tab[256];
-  load_exp_table(tab);
-  const int lane = threadIdx.x & 31;
-  const uint32_t side = uint32_t(b.ts) / kBlock, blocks = side * side, num_tasks = b.num_items * blocks;
-  for (;;) {
-    uint32_t task = 0;
-    if (lane == 0) task = atomicAdd(work_counter, 1u);
-    task = __shfl_sync(0xffffffffu, task, 0);
-    if (task >= num_tasks) return;
-    const uint32_t item = order[task / blocks], blk = task % blocks;
-    const ItemGeo ig = item_geo(b, item, off1, nchunk, capacity);
-    const ViewDev& vd = b.v[ig.v];
-    const int px0 = ig.px0 + int(blk % side) * kBlock, py0 = ig.py0 + int(blk / side) * kBlock;
-    if (px0 >= vd.w || py0 >= vd.h) continue;  // a tile's blocks beyond the view
-    const PackedBlockSrc src{rec + 3 * size_t(ig.v) * n};
-    const SbWords walk{list1, ig.lx, ig.ly, 1u};
-    float* const loss = slab_loss + size_t(item) * slots + (slots >= blocks ? blk * (slots / blocks) : blk * slots / blocks);
-    const FwdOut out{out_rgb, out_T, out_last, target, grad_pix, loss, slots < blocks};
-    const uint32_t cost = blend_block<false>(walk, src, sh[threadIdx.x >> 5], tab, nz, ig.s, ig.e, px0, py0, vd.w, vd.w,
-                                           vd.h, false, vd.pix_base, out);
-    // scheduling hint for the backward and the next forward
-    if (lane == 0 && cost) atomicMax(&item_cost[item], cost);
-  }
-}
-
-// Drop-in forward (splat_gauss.rs:46-94): AoS inputs and per-tile lists,
-// accumulates into pix2rgb.
-template <bool CUDA_STOP>
-__global__ void __launch_bounds__(32 * kRasterWarps, 6) k_raster_aos(
-    int w, int h, int ts, int tile_w, uint32_t num_tasks, float* __restrict__ pix2rgb, AosBlockSrc src,
-    const uint32_t* __restrict__ tile2idx, const uint32_t* __restrict__ idx2pnt, float* __restrict__ out_T,
-    uint32_t* __restrict__ out_last, float nz) {
-  __shared__ FwdWarp sh[kRasterWarps];
-  __shared__ float tab[256];
-  load_exp_table(tab);
-  const uint32_t task = blockIdx.x * kRasterWarps + (threadIdx.x >> 5);
-  if (task >= num_tasks) return;
-  const uint32_t side = uint32_t(ts) / kBlock, tile = task / (side * side), blk = task % (side * side);
-  const int px0 = int(tile % uint32_t(tile_w)) * ts + int(blk % side) * kBlock;
-  const int py0 = int(tile / uint32_t(tile_w)) * ts + int(blk / side) * kBlock;
-  if (px0 >= w || py0 >= h) return;
-  const FwdOut out{pix2rgb, out_T, out_last, nullptr, nullptr, nullptr, false};
-  blend_block<CUDA_STOP>(TileWords{idx2pnt}, src, sh[threadIdx.x >> 5], tab, nz, tile2idx[tile], tile2idx[tile + 1], px0,
-                       py0, w, w, h, true, 0, out);
-}
-
-cudaError_t raster_blocks(cudaStream_t st, const ViewBatch& b, const FwdArgs& a) {
-  const uint32_t side = uint32_t(b.ts) / kBlock, blocks = side * side, tasks = b.num_items * blocks;
-  const uint32_t slots = raster_slabs_per_tile(b.ts, b.ppl);
-  if (a.target && slots != blocks) {
-    const cudaError_t e = cudaMemsetAsync(a.slab_loss, 0, size_t(b.num_items) * slots * sizeof(float), st);
-    if (e != cudaSuccess) return e;
-  }
-  k_raster_blocks<<<persistent_grid(k_raster_blocks, tasks), 32 * kRasterWarps, 0, st>>>(
-      b, a.n, a.rec, a.list1, a.off1, a.nchunk, a.capacity, a.order, a.counter, a.out_rgb, a.out_T, a.out_last,
-      a.target, a.grad_pix, a.slab_loss, slots, a.item_cost, -0.f);
-  count_launch();
-  return cudaGetLastError();
-}
-
-cudaError_t raster_fwd_aos(cudaStream_t st, int ts, int w, int h, float* pix2rgb, const float* xyd, const float* conic,
-                           const float* aabb, const float* opacity, const float* rgb, const uint32_t* tile2idx,
-                           const uint32_t* idx2pnt, float* out_T, uint32_t* out_last, bool cuda_stop) {
-  if (w <= 0 || h <= 0) return cudaSuccess;
-  const AosBlockSrc src{xyd, conic, aabb, opacity, rgb};
-  const uint32_t side = uint32_t(ts) / kBlock;
-  const int tw = (w + ts - 1) / ts, th = (h + ts - 1) / ts;
-  const uint32_t tasks = uint32_t(tw) * uint32_t(th) * side * side;
-  const unsigned grid = (tasks + kRasterWarps - 1) / kRasterWarps;
-  if (cuda_stop)
-    k_raster_aos<true><<<grid, 32 * kRasterWarps, 0, st>>>(w, h, ts, tw, tasks, pix2rgb, src, tile2idx, idx2pnt,
-                                                               out_T, out_last, -0.f);
-  else
-    k_raster_aos<false><<<grid, 32 * kRasterWarps, 0, st>>>(w, h, ts, tw, tasks, pix2rgb, src, tile2idx, idx2pnt,
-                                                                out_T, out_last, -0.f);
-  count_launch();
-  return cudaGetLastError();
 }
 
 }  // namespace dsplat

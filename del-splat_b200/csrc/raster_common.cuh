@@ -241,6 +241,48 @@ __device__ __forceinline__ ItemGeo item_geo(const ViewBatch& b, uint32_t item, c
   return g;
 }
 
+// One unit of a rasteriser's work: block sub of a heavy item (walked in 8x8
+// blocks: the run's tiles of 8 pixels, or the blocks of a larger tile), or
+// task sub of another.
+__host__ __device__ __forceinline__ uint32_t blocks_per_item(int ts) { return ts == 8 ? 2u : uint32_t(ts * ts) / 64u; }
+
+struct Task {
+  uint32_t item, sub;
+  bool block, none;  // none: past the last one
+  // unit i of the order, whose first sched[kSchedHeavy] items are heavy
+  __device__ __forceinline__ Task(const ViewBatch& b, uint32_t i, const uint32_t* __restrict__ order,
+                                  const uint32_t* __restrict__ sched, uint32_t slabs) {
+    const uint32_t heavy = sched[kSchedHeavy], per = blocks_per_item(b.ts), blocks = heavy * per;
+    block = i < blocks;
+    const uint32_t at = block ? i / per : heavy + (i - blocks) / slabs;
+    sub = block ? i % per : (i - blocks) % slabs;
+    none = at >= b.num_items;
+    item = none ? 0u : order[at];
+  }
+};
+
+// Where block sub of an item lies; false: outside the view or the run.
+struct BlockPlace {
+  int px0, py0;
+  uint32_t lx;
+};
+__device__ __forceinline__ bool block_place(const ViewBatch& b, const ItemGeo& g, uint32_t sub, uint32_t nx,
+                                            BlockPlace* p) {
+  p->px0 = g.px0;
+  p->py0 = g.py0;
+  p->lx = g.lx;
+  if (b.ts == 8) {
+    if (sub >= nx) return false;
+    p->px0 += 8 * int(sub);
+    p->lx += sub;
+  } else {
+    const uint32_t side = uint32_t(b.ts) / 8u;
+    p->px0 += 8 * int(sub % side);
+    p->py0 += 8 * int(sub / side);
+  }
+  return p->px0 < b.v[g.v].w && p->py0 < b.v[g.v].h;
+}
+
 // ---------------------------------------------------------------------------
 // host launch helpers
 // ---------------------------------------------------------------------------
@@ -253,6 +295,12 @@ inline int num_sms() {
     if (sms <= 0) sms = 148;
   }
   return sms;
+}
+
+// Most units of work a batch can have.
+inline uint32_t max_tasks(const ViewBatch& b, uint32_t slabs) {
+  const uint64_t t = uint64_t(b.num_items) * (blocks_per_item(b.ts) > slabs ? blocks_per_item(b.ts) : slabs);
+  return t > 0xffffffffull ? 0xffffffffu : uint32_t(t);
 }
 
 // Supported (tile size, pixels per lane) pairs; slabs per tile follow.

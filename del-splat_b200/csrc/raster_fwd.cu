@@ -7,11 +7,14 @@
 // the assembler contracts packed mul/add pairs regardless of that flag.  The
 // fused multiply-adds the exponential wants are written out (fma2) and stay
 // fused.
+#include <algorithm>
+
+#include "raster_block.cuh"
 #include "raster_common.cuh"
 
 namespace dsplat {
 
-cudaError_t raster_blocks(cudaStream_t, const ViewBatch&, const FwdArgs&);
+uint32_t raster_slabs_per_tile(int ts, int ppl);
 
 // ---------------------------------------------------------------------------
 // Forward walk of one slab by one warp over the list range [s, e).  Slot k of
@@ -25,13 +28,13 @@ cudaError_t raster_blocks(cudaStream_t, const ViewBatch&, const FwdArgs&);
 // one tile keeps every lane of the warp busy on one pair and skips the
 // other pair warp-wide.  Otherwise lane L covers column L % TS, slot k at
 // row L / TS + k (32 / TS).
-template <int TS, int PPL_, bool SPLIT, class Walk, class Src>
+template <int TS, int PPL_, bool SPLIT, class Walk, class Src, class Loss>
 __device__ __forceinline__ uint32_t fwd_slab(const Walk& walk, const Src& src, EntP* sm, float4* park,
                                          uint32_t* park_pos, const float* tab, float nz,
                                          uint32_t s, uint32_t e, int px0, int py0, int w, int h, int xend,
                                          float* __restrict__ out_rgb, size_t pix_base, float* __restrict__ out_T,
                                          uint32_t* __restrict__ out_last, const float* __restrict__ target,
-                                         float* __restrict__ grad_pix, float* __restrict__ loss_slot) {
+                                         float* __restrict__ grad_pix, const Loss& loss) {
   using G = Geo<TS, PPL_>;
   constexpr int PPL = G::PPL;
   static_assert(PPL % 2 == 0, "pixel slots are evaluated in pairs");
@@ -222,106 +225,151 @@ __device__ __forceinline__ uint32_t fwd_slab(const Walk& walk, const Src& src, E
   if (target) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-    if (lane == 0) *loss_slot = l;
+    if (lane == 0) loss(l);
   }
   return cost;
 }
 
 // ---------------------------------------------------------------------------
-// Fused-path forward: persistent, per-warp work stealing over slab tasks,
-// walking each tile's entries out of its superblock list.
-// slab_loss: one partial L2 loss per task (when target is given).
+// Fused-path forward: persistent, per-warp work stealing, walking each tile's
+// entries out of its superblock list.  The first sched[kSchedHeavy] items of
+// the order are walked in 8x8 blocks (raster_block.cuh), the others in tasks
+// of TaskGeo.  No block count is asked of the compiler: it takes 80 registers
+// by itself (6 blocks of 4 warps per SM), and 10% more instructions when told
+// to (16 views of 1,048,576 Gaussians 2890 -> 3210 us).  slab_loss: `slots` partial L2 losses per tile (when target is
+// given; zero at the start where a tile's blocks do not match its slots).
 // ---------------------------------------------------------------------------
 template <int TS, int PPL, int NT>
 __global__ void __launch_bounds__(32 * kRasterWarps) k_raster_fwd(
     const ViewBatch b, uint32_t n, const float4* __restrict__ rec, const uint2* __restrict__ list1,
     const uint32_t* __restrict__ off1, uint32_t nchunk, uint64_t capacity, const uint32_t* __restrict__ order,
-    uint32_t* __restrict__ work_counter, float* __restrict__ out_rgb, float* __restrict__ out_T,
-    uint32_t* __restrict__ out_last, const float* __restrict__ target, float* __restrict__ grad_pix,
-    float* __restrict__ slab_loss, uint32_t* __restrict__ item_cost, float nz) {
+    const uint32_t* __restrict__ sched, uint32_t* __restrict__ work_counter, float* __restrict__ out_rgb,
+    float* __restrict__ out_T, uint32_t* __restrict__ out_last, const float* __restrict__ target,
+    float* __restrict__ grad_pix, float* __restrict__ slab_loss, uint32_t slots, uint32_t* __restrict__ item_cost,
+    float nz) {
   using G = TaskGeo<TS, PPL, NT>;
-  __shared__ EntP sm_all[kRasterWarps][32];
+  static_assert(sizeof(EntB) >= sizeof(EntP), "the warps' entries of either form share their place");
+  __shared__ EntB ent_all[kRasterWarps][32];
   __shared__ float4 park_all[kRasterWarps][G::PPL * 32];
   __shared__ uint32_t park_pos_all[kRasterWarps][G::PPL * 32];
   __shared__ float tab[256];
   load_exp_table(tab);
-  EntP* sm = sm_all[threadIdx.x >> 5];
-  float4* park = park_all[threadIdx.x >> 5];
-  uint32_t* park_pos = park_pos_all[threadIdx.x >> 5];
+  EntB* const ent = ent_all[threadIdx.x >> 5];
+  float4* const park = park_all[threadIdx.x >> 5];
+  uint32_t* const park_pos = park_pos_all[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
-  const uint32_t num_tasks = b.num_items * G::SLABS;
   for (;;) {
-    uint32_t task = 0;
-    if (lane == 0) task = atomicAdd(work_counter, 1u);
-    task = __shfl_sync(0xffffffffu, task, 0);
-    if (task >= num_tasks) return;
-    const uint32_t item = order[task / G::SLABS], slab = task % G::SLABS;
-    const ItemGeo ig = item_geo(b, item, off1, nchunk, capacity);
+    uint32_t i = 0;
+    if (lane == 0) i = atomicAdd(work_counter, 1u);
+    const Task t(b, __shfl_sync(0xffffffffu, i, 0), order, sched, G::SLABS);
+    if (t.none) return;
+    const ItemGeo ig = item_geo(b, t.item, off1, nchunk, capacity);
     const ViewDev& vd = b.v[ig.v];
-    // tiles of this task (NT > 1: a run of a superblock row, see k_raster_bwd)
+    const PackedSrc src{rec + 3 * size_t(ig.v) * n};
+    // tiles of the item's tasks (NT > 1: a run of a superblock row, see
+    // k_raster_bwd, carried by its leftmost tile)
     uint32_t nx = 1;
     if (NT > 1) {
       nx = min(uint32_t(NT), 1u << vd.sb_log2);
-      if (ig.lx % nx) {  // carried by the run's leftmost tile
-        if (target && slab_loss && lane == 0) slab_loss[size_t(item) * G::SLABS + slab] = 0.f;
-        continue;
-      }
+      if (ig.lx % nx) continue;
     }
-    PackedSrc src{rec + 3 * size_t(ig.v) * n};
-    SbWalkSpan walk{list1, ig.lx, ig.ly, nx};
-    const int xend = min(vd.w, ig.px0 + int(nx) * TS);
-    const uint32_t walked = fwd_slab<G::GX, G::PPL, NT == 2 && G::PPL == 4>(
-        walk, src, sm, park, park_pos, tab, nz, ig.s, ig.e, ig.px0, ig.py0 + int(slab) * G::SLAB_ROWS, vd.w, vd.h, xend, out_rgb,
-        vd.pix_base, out_T, out_last, target, grad_pix, slab_loss ? slab_loss + size_t(item) * G::SLABS + slab : nullptr);
+    uint32_t cost;
+    if (t.block) {
+      BlockPlace p;
+      if (!block_place(b, ig, t.sub, nx, &p)) continue;
+      const FwdOut out{out_rgb, out_T, out_last, target, grad_pix};
+      cost = blend_block<false>(SbWords{list1, p.lx, ig.ly, 1u}, PackedBlockSrc{src.rec}, ent, park, park_pos, tab, nz,
+                                ig.s, ig.e, p.px0, p.py0, vd.w, vd.w, vd.h, false, vd.pix_base, out, [&](float l) {
+                                  float* const p0 = slab_loss + size_t(t.item) * slots;
+                                  constexpr uint32_t blocks = TS * TS / 64;
+                                  if (TS == 8) p0[t.sub * slots] = l;  // the run's tile t.sub
+                                  else if (slots < blocks) atomicAdd(p0 + t.sub * slots / blocks, l);
+                                  else p0[t.sub * (slots / blocks)] = l;
+                                });
+    } else {
+      SbWalkSpan walk{list1, ig.lx, ig.ly, nx};
+      const int xend = min(vd.w, ig.px0 + int(nx) * TS);
+      cost = fwd_slab<G::GX, G::PPL, NT == 2 && G::PPL == 4>(
+          walk, src, reinterpret_cast<EntP*>(ent), park, park_pos, tab, nz, ig.s, ig.e, ig.px0,
+          ig.py0 + int(t.sub) * G::SLAB_ROWS, vd.w, vd.h, xend, out_rgb, vd.pix_base, out_T, out_last, target,
+          grad_pix, [&](float l) {
+            float* const p0 = slab_loss + size_t(t.item) * G::SLABS + t.sub;
+            *p0 = l;
+            // the run's other tile has its loss in the leftmost one's slot
+            if (NT > 1 && vd.sb_log2 > 0 && ig.px0 + 8 < vd.w) p0[G::SLABS] = 0.f;
+          });
+    }
     // scheduling hint for the backward and the next forward
-    if (lane == 0 && walked) atomicMax(&item_cost[item], walked);
+    if (lane == 0 && cost) atomicMax(&item_cost[t.item], cost);
     __syncwarp();
   }
 }
 
-template <int TS, int PPL>
-static void launch_fwd(cudaStream_t st, const ViewBatch& b, const FwdArgs& a) {
-  constexpr int NT = TS == 8 ? kFwdGroup8 : 1;
-  const uint32_t tasks = b.num_items * TaskGeo<TS, PPL, NT>::SLABS;
-  k_raster_fwd<TS, PPL, NT><<<persistent_grid(k_raster_fwd<TS, PPL, NT>, tasks), 32 * kRasterWarps, 0, st>>>(
-      b, a.n, a.rec, a.list1, a.off1, a.nchunk, a.capacity, a.order, a.counter, a.out_rgb, a.out_T, a.out_last,
-      a.target, a.grad_pix, a.slab_loss, a.item_cost, -0.f);
-  count_launch();
+// Drop-in forward (splat_gauss.rs:46-94): AoS inputs and per-tile lists,
+// accumulates into pix2rgb; in 8x8 blocks (raster_block.cuh).
+template <bool CUDA_STOP>
+__global__ void __launch_bounds__(32 * kRasterWarps, 6) k_raster_fwd_aos(
+    int w, int h, int ts, int tile_w, uint32_t num_tasks, float* __restrict__ pix2rgb, AosBlockSrc src,
+    const uint32_t* __restrict__ tile2idx, const uint32_t* __restrict__ idx2pnt, float* __restrict__ out_T,
+    uint32_t* __restrict__ out_last, float nz) {
+  __shared__ EntB ent[kRasterWarps][32];
+  __shared__ float4 park[kRasterWarps][64];
+  __shared__ uint32_t park_pos[kRasterWarps][64];
+  __shared__ float tab[256];
+  load_exp_table(tab);
+  const int warp = threadIdx.x >> 5;
+  const uint32_t task = blockIdx.x * kRasterWarps + (threadIdx.x >> 5);
+  if (task >= num_tasks) return;
+  const uint32_t side = uint32_t(ts) / kBlock, tile = task / (side * side), blk = task % (side * side);
+  const int px0 = int(tile % uint32_t(tile_w)) * ts + int(blk % side) * kBlock;
+  const int py0 = int(tile / uint32_t(tile_w)) * ts + int(blk / side) * kBlock;
+  if (px0 >= w || py0 >= h) return;
+  const FwdOut out{pix2rgb, out_T, out_last, nullptr, nullptr};
+  blend_block<CUDA_STOP>(TileWords{idx2pnt}, src, ent[warp], park[warp], park_pos[warp], tab, nz, tile2idx[tile],
+                         tile2idx[tile + 1], px0, py0, w, w, h, true, 0, out, [](float) {});
 }
 
-// Whether a batch's forward and backward run in 8x8 blocks (raster_blocks.cu,
-// k_raster_bwd's BLOCK form) instead of the tasks here.  Blocks win while the
-// step waits for its longest walks, the tasks here once there is enough work
-// to hide them, and the earlier the larger the views are against the tasks
-// (an entry then mostly holds all of a task's pixels).  Whole steps in us,
-// tasks here -> blocks, at the configuration of 8x8 tiles:
-//   1,048,576 Gaussians, one view  1280x720   1735 -> 1457
-//   262,144,   4 views              1280x720   1686 -> 1554
-//   1,048,576, 4 views              1280x720   4026 -> 3336
-//   100,003,   8 views               640x480   1289 -> 1183
-//   1,048,576, one view             1920x1080  1722 -> 1868
-//   1,048,576, 2 views              1920x1080  2714 -> 3144
-//   262,144,   8 views              1280x720   2387 -> 2748
-//   1,048,576, 16 views, 13.5 M pixels         8878 -> 9888
-constexpr uint32_t kBlockBatchPixels = 4u << 20, kBlockViewPixels = 5u << 18;
-
-bool raster_in_blocks(const ViewBatch& b) {
-  if (b.num_pix > kBlockBatchPixels) return false;
-  for (int v = 0; v < b.num_views; ++v)
-    if (uint32_t(b.v[v].w) * uint32_t(b.v[v].h) > kBlockViewPixels) return false;
-  return true;
+template <int TS, int PPL>
+static cudaError_t launch_fwd(cudaStream_t st, const ViewBatch& b, const FwdArgs& a) {
+  constexpr int NT = TS == 8 ? kFwdGroup8 : 1;
+  const uint32_t slots = raster_slabs_per_tile(TS, PPL);
+  if (a.target && slots != uint32_t(TS * TS / 64)) {
+    const cudaError_t e = cudaMemsetAsync(a.slab_loss, 0, size_t(b.num_items) * slots * sizeof(float), st);
+    if (e != cudaSuccess) return e;
+  }
+  k_raster_fwd<TS, PPL, NT>
+      <<<persistent_grid(k_raster_fwd<TS, PPL, NT>, max_tasks(b, TaskGeo<TS, PPL, NT>::SLABS)), 32 * kRasterWarps, 0,
+         st>>>(b, a.n, a.rec, a.list1, a.off1, a.nchunk, a.capacity, a.order, a.sched, a.counter, a.out_rgb, a.out_T,
+               a.out_last, a.target, a.grad_pix, a.slab_loss, slots, a.item_cost, -0.f);
+  count_launch();
+  return cudaGetLastError();
 }
 
 cudaError_t raster_fwd(cudaStream_t st, const ViewBatch& b, const FwdArgs& a) {
-  if (raster_in_blocks(b)) return raster_blocks(st, b, a);
-#define X(T, P)                        \
-  if (b.ts == T && b.ppl == P) {       \
-    launch_fwd<T, P>(st, b, a);        \
-    return cudaGetLastError();         \
-  }
+#define X(T, P) \
+  if (b.ts == T && b.ppl == P) return launch_fwd<T, P>(st, b, a);
   DSPLAT_RASTER_CONFIGS(X)
 #undef X
   return cudaErrorInvalidValue;
+}
+
+cudaError_t raster_fwd_aos(cudaStream_t st, int ts, int w, int h, float* pix2rgb, const float* xyd, const float* conic,
+                           const float* aabb, const float* opacity, const float* rgb, const uint32_t* tile2idx,
+                           const uint32_t* idx2pnt, float* out_T, uint32_t* out_last, bool cuda_stop) {
+  if (w <= 0 || h <= 0) return cudaSuccess;
+  const AosBlockSrc src{xyd, conic, aabb, opacity, rgb};
+  const uint32_t side = uint32_t(ts) / kBlock;
+  const int tw = (w + ts - 1) / ts, th = (h + ts - 1) / ts;
+  const uint32_t tasks = uint32_t(tw) * uint32_t(th) * side * side;
+  const unsigned grid = (tasks + kRasterWarps - 1) / kRasterWarps;
+  if (cuda_stop)
+    k_raster_fwd_aos<true><<<grid, 32 * kRasterWarps, 0, st>>>(w, h, ts, tw, tasks, pix2rgb, src, tile2idx, idx2pnt,
+                                                               out_T, out_last, -0.f);
+  else
+    k_raster_fwd_aos<false><<<grid, 32 * kRasterWarps, 0, st>>>(w, h, ts, tw, tasks, pix2rgb, src, tile2idx, idx2pnt,
+                                                                out_T, out_last, -0.f);
+  count_launch();
+  return cudaGetLastError();
 }
 
 // expf_cr elementwise (exposed so that it can be checked against a

@@ -613,60 +613,72 @@ __global__ void __launch_bounds__(kMsThreads) k_sb_scatter_staged(const uint32_t
 }
 
 // ---------------------------------------------------------------------------
-// Longest-first task order for the rasteriser: items bucketed by floor(log2)
+// Longest-first task order for the rasterisers: items bucketed by floor(log2)
 // of their cost, heaviest bucket first, so the tail of the persistent launch
-// is made of short tasks.  The cost is the number of list positions the last
-// forward walked for the item (measured, kept in the workspace) or, where
-// none is recorded yet, its superblock-list length.  Only the schedule
-// depends on it, never the results.  sched[0..32] counts, [40..72] cursors.
+// is made of short tasks.  The cost is that of the item's longest walk in the
+// last forward (measured, kept in the workspace) or, where none is recorded
+// yet, its superblock-list length.  Only the schedule depends on it, never
+// the results.  sched: see kSchedCost in common.cuh.
+//
+// Heavy items: a task whose cost is a good part of what every resident warp
+// has to do (total / warps) ends after the others, and the GPU waits for it
+// -- the tiles of a scene's rim, whose pixels never saturate, walk ten times
+// the mean list.  The items of the buckets above that share are walked in 8x8
+// blocks (about 15% more instructions, so short tasks stay whole).
 // ---------------------------------------------------------------------------
-// Longest-first bucket of an item (0 = longest): clz of the list positions
-// its task walked in the previous forward (cost[item]), else of its
-// superblock's list length.  With nt > 1 adjacent tiles per task (8x8
-// tiles) only a group's leading tile leads a task and carries its cost; the
-// other tiles lead none (their tasks return at once) and go last.
-__device__ __forceinline__ uint32_t item_cost_bucket(const ViewBatch& b, uint32_t item, const uint32_t* off1,
-                                                     uint32_t nchunk, const uint32_t* cost, int nt) {
+__device__ __forceinline__ uint32_t item_cost(const ViewBatch& b, uint32_t item, const uint32_t* off1, uint32_t nchunk,
+                                              const uint32_t* cost) {
   int v = 0;
   for (int k = 1; k < b.num_views; ++k)
     if (item >= b.v[k].item_base) v = k;
   const ViewDev& vd = b.v[v];
   const uint32_t t = item - vd.item_base;
   const uint32_t tx = t % uint32_t(vd.tile_w), ty = t / uint32_t(vd.tile_w);
-  if (nt > 1 && tx % min(uint32_t(nt), 1u << vd.sb_log2)) return 31u;
-  const uint32_t measured = cost ? cost[item] : 0u;
-  if (measured) return uint32_t(__clz(measured));
+  // 8x8 tiles: the leftmost tile of a run carries the task of both
+  if (b.ts == 8 && tx % min(2u, 1u << vd.sb_log2)) return 0u;
+  const uint32_t measured = cost[item];
+  if (measured) return measured;
   const uint32_t sb = vd.sb_base + (ty >> vd.sb_log2) * uint32_t(sb_cols(vd)) + (tx >> vd.sb_log2);
-  const uint32_t len = off1[size_t(sb + 1) * nchunk] - off1[size_t(sb) * nchunk];
-  return len ? uint32_t(__clz(len)) : 32u;
+  return off1[size_t(sb + 1) * nchunk] - off1[size_t(sb) * nchunk];
 }
 
 __global__ void k_order_hist(const ViewBatch b, const uint32_t* __restrict__ off1, uint32_t nchunk,
-                             const uint32_t* __restrict__ cost, int nt, uint32_t* __restrict__ sched) {
+                             const uint32_t* __restrict__ cost, uint32_t* __restrict__ sched) {
   __shared__ uint32_t h[33];
   if (threadIdx.x < 33) h[threadIdx.x] = 0;
   __syncthreads();
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < b.num_items; i += gridDim.x * blockDim.x)
-    atomicAdd(&h[item_cost_bucket(b, i, off1, nchunk, cost, nt)], 1u);
+  unsigned long long sum = 0;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < b.num_items; i += gridDim.x * blockDim.x) {
+    const uint32_t c = item_cost(b, i, off1, nchunk, cost);
+    atomicAdd(&h[__clz(c)], 1u);
+    sum += c;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  if ((threadIdx.x & 31) == 0 && sum) atomicAdd(reinterpret_cast<unsigned long long*>(sched + kSchedCost), sum);
   __syncthreads();
   if (threadIdx.x < 33 && h[threadIdx.x]) atomicAdd(&sched[threadIdx.x], h[threadIdx.x]);
 }
 
 // Scatter into bucket order: each block ranks its items in shared memory and
 // takes one range per bucket from the global cursors (one global atomic per
-// bucket and block instead of one per item on 33 hot counters).  sched[0..33)
-// holds the bucket counts, sched[40..73) the cursors (zero at the start);
-// every block forms the buckets' starts from the counts itself.
+// bucket and block instead of one per item on 33 hot counters); every block
+// forms the buckets' starts from the counts itself.  heavy_share: an item
+// is heavy when its cost times that is above the total cost.
 __global__ void k_order_scatter(const ViewBatch b, const uint32_t* __restrict__ off1, uint32_t nchunk,
-                                const uint32_t* __restrict__ cost, int nt, uint32_t* __restrict__ sched,
+                                const uint32_t* __restrict__ cost, float heavy_share, uint32_t* __restrict__ sched,
                                 uint32_t* __restrict__ order) {
   __shared__ uint32_t cnt[33], base[33], start[33];
   if (threadIdx.x == 0) {
-    uint32_t run = 0;
+    const float total = float(*reinterpret_cast<const unsigned long long*>(sched + kSchedCost));
+    uint32_t run = 0, heavy = 0;
     for (int k = 0; k < 33; ++k) {
       start[k] = run;
       run += sched[k];
+      // bucket k holds the costs from 2^(31 - k) on
+      if (k < 32 && exp2f(float(31 - k)) * heavy_share > total) heavy = run;
     }
+    if (blockIdx.x == 0) sched[kSchedHeavy] = heavy;
   }
   __syncthreads();
   const uint32_t per_block = (b.num_items + gridDim.x - 1) / gridDim.x;
@@ -677,7 +689,7 @@ __global__ void k_order_scatter(const ViewBatch b, const uint32_t* __restrict__ 
     const uint32_t i = i0 + threadIdx.x;
     uint32_t bucket = 0, slot = 0;
     if (i < hi) {
-      bucket = item_cost_bucket(b, i, off1, nchunk, cost, nt);
+      bucket = uint32_t(__clz(item_cost(b, i, off1, nchunk, cost)));
       slot = atomicAdd(&cnt[bucket], 1u);
     }
     __syncthreads();
