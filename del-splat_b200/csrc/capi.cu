@@ -15,7 +15,7 @@ namespace dsplat {
 __global__ void k_gauss_project_ref(uint32_t, const float*, const float*, const float*, const float*, int, int, float*,
                                     float*, float*);
 __global__ void k_circle_project_ref(uint32_t, const float*, const float*, int, int, float, float*, float*);
-__global__ void k_prep_tiles(uint32_t, const float*, const float*, const float*, int, int, int, uint2*, uint32_t*);
+__global__ void k_prep_tiles(uint32_t, uint32_t, const float*, const float*, const float*, int, int, int, uint2*, uint32_t*);
 __global__ void k_count_pairs(uint32_t, const float*, const float*, const float*, int, int, int, unsigned long long*);
 __global__ void k_fused_project(uint32_t, uint32_t, int, const float*, const float*, const float*, const float*,
                                 const float*, const ViewBatch, float4*, uint2*, uint32_t*, uint32_t*);
@@ -23,9 +23,8 @@ __global__ void k_project_bwd_geom(uint32_t, const float*, const float*, const f
                                    float4*, float*, float*, float*, float*);
 __global__ void k_project_bwd_colour(uint32_t, int, const float*, const float*, const ViewBatch, float4*,
                                      float*, float*, unsigned long long*, unsigned long long);
-__global__ void k_prepare_grad2d(const unsigned long long*, unsigned long long, float4*, size_t);
+__global__ void k_prepare_grad2d(const unsigned long long*, unsigned long long, float4*, size_t, uint32_t*);
 __global__ void k_adam(size_t, float*, const float*, float*, float*, float, float, float, float, float, float);
-__global__ void k_pad_keys(uint32_t*, uint32_t, uint32_t, uint32_t);
 __global__ void k_sb_count(const uint32_t*, const uint2*, uint32_t, uint32_t, const ViewBatch, uint32_t*,
                            unsigned long long*);
 __global__ void k_sb_scatter(const uint32_t*, const uint2*, uint32_t, uint32_t, const ViewBatch, const uint32_t*,
@@ -38,8 +37,6 @@ cudaError_t split_tile_lists(cudaStream_t, const uint2*, const uint32_t*, uint32
                              uint32_t*, uint32_t*);
 cudaError_t scatter_tile_lists(cudaStream_t, const uint2*, const uint32_t*, uint32_t, uint64_t, const ViewBatch&,
                                const uint32_t*, const uint32_t*, uint32_t*, uint32_t*, uint32_t*);
-__global__ void k_clamp_ranges(uint32_t*, uint32_t, uint64_t, uint32_t*);
-__global__ void k_check_capacity(const unsigned long long*, uint64_t, uint32_t*);
 __global__ void k_make_keys64(const uint32_t*, const uint32_t*, const float*, const unsigned long long*, uint64_t,
                               uint64_t*);
 __global__ void k_fill_u64(uint64_t*, size_t, uint64_t);
@@ -50,17 +47,16 @@ __global__ void k_circle_resolve(size_t, const uint64_t*, const void*, int, void
 
 size_t scan_tmp_words(size_t n);
 size_t radix_hist_words(size_t n);
-cudaError_t exclusive_scan(cudaStream_t, const uint32_t*, uint32_t*, size_t, uint32_t*);
-cudaError_t radix_sort(cudaStream_t, uint32_t*, uint32_t*, uint32_t*, uint32_t*, size_t, const uint32_t*, int, uint32_t,
-                       uint32_t*, uint32_t*, bool*, const uint2*, uint32_t, uint2*, bool, uint32_t);
+cudaError_t exclusive_scan(cudaStream_t, const uint32_t*, uint32_t*, size_t, uint32_t*, uint32_t, uint32_t*);
+cudaError_t depth_sort(cudaStream_t, uint32_t*, uint32_t*, uint32_t*, uint32_t*, uint32_t, uint32_t, uint32_t*,
+                       uint32_t*, const uint2*, uint32_t, uint2*);
 cudaError_t raster_fwd(cudaStream_t, const ViewBatch&, const FwdArgs&);
 cudaError_t raster_bwd(cudaStream_t, const ViewBatch&, const BwdArgs&);
 bool raster_config_ok(int ts, int ppl);
 int raster_default_ppl(int ts);
 uint32_t raster_slabs_per_tile(int ts, int ppl);
 __global__ void k_order_hist(const ViewBatch, const uint32_t*, uint32_t, const uint32_t*, uint32_t*);
-__global__ void k_order_scatter(const ViewBatch, const uint32_t*, uint32_t, const uint32_t*, float, uint32_t*,
-                                uint32_t*);
+__global__ void k_order_scatter(const ViewBatch, const uint32_t*, uint32_t, uint32_t*, float, uint32_t*, uint32_t*);
 cudaError_t raster_fwd_aos(cudaStream_t, int, int, int, float*, const float*, const float*, const float*, const float*,
                            const float*, const uint32_t*, const uint32_t*, float*, uint32_t*, bool);
 cudaError_t expf_cr_launch(cudaStream_t, size_t, const float*, float*);
@@ -69,11 +65,6 @@ cudaError_t circle_splat_tiles(cudaStream_t, int, int, int, float*, const float*
 
 __global__ void k_adam_fused(AdamSeg, double, double, double, double, const int32_t*);
 __global__ void k_adam_step_inc(int32_t*);
-
-__global__ void k_one_minus(const float* __restrict__ T, float* __restrict__ out, size_t n) {
-  const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i < n) out[i] = 1.f - T[i];
-}
 
 namespace {
 
@@ -191,10 +182,7 @@ int build_sb_lists(cudaStream_t st, const ViewBatch& b, uint32_t n, uint32_t npa
   unsigned long long* totals = reinterpret_cast<unsigned long long*>(flags + 6);
   k_sb_count<<<grid1, 256, smem1, st>>>(order, srect, npad / nchunk, npad, b, L.cnt1, totals);
   count_launch();
-  TRY_CUDA(cudaMemsetAsync(L.cnt1 + m, 0, sizeof(uint32_t), st), "memset");
-  TRY_CUDA(exclusive_scan(st, L.cnt1, L.off1, m + 1, scan_tmp), "scan");
-  k_check_capacity<<<1, 32, 0, st>>>(totals + 1, capacity, flags);
-  count_launch();
+  TRY_CUDA(exclusive_scan(st, L.cnt1, L.off1, m, scan_tmp, 0xffffffffu, nullptr), "scan");
   // staged scatter (coalesced list stores) when its shared memory fits
   constexpr uint32_t kStageEntries = 3072;
   const size_t smem_staged = sb_scatter_staged_smem(b.max_sb, b.max_sb_side, kStageEntries);
@@ -218,13 +206,13 @@ int build_tile_lists(cudaStream_t st, const ViewBatch& b, uint32_t npad, const L
                      uint32_t* scan_tmp, uint32_t* item_start, uint32_t* idx2pnt, uint32_t* out_tile, uint64_t capacity,
                      uint32_t* flags) {
   const uint32_t nchunk = num_chunks(b, npad);
-  TRY_CUDA(cudaMemsetAsync(L.tcnt + b.num_items, 0, sizeof(uint32_t), st), "memset");
   TRY_CUDA(split_tile_lists(st, L.list1, L.off1, nchunk, capacity, b, segcnt, L.tcnt), "tile counts");
-  TRY_CUDA(exclusive_scan(st, L.tcnt, item_start, size_t(b.num_items) + 1, scan_tmp), "scan");
+  // ranges past the pair capacity are cut to it, so that readers stay in
+  // bounds (the results are then invalid and the flag is set)
+  const uint32_t limit = uint32_t(std::min<uint64_t>(capacity, 0xffffffffull));
+  TRY_CUDA(exclusive_scan(st, L.tcnt, item_start, b.num_items, scan_tmp, limit, flags), "scan");
   TRY_CUDA(scatter_tile_lists(st, L.list1, L.off1, nchunk, capacity, b, segcnt, item_start, idx2pnt, out_tile, flags),
            "tile scatter");
-  k_clamp_ranges<<<64, 256, 0, st>>>(item_start, b.num_items, capacity, flags);
-  count_launch();
   TRY_CUDA(cudaGetLastError(), "tile lists");
   return DSPLAT_OK;
 }
@@ -240,9 +228,7 @@ int build_tile_lists(cudaStream_t st, const ViewBatch& b, uint32_t npad, const L
 constexpr float kHeavyShare = 148.f * 64.f;
 
 cudaError_t order_tasks(cudaStream_t st, const ViewBatch& b, const uint32_t* off1, uint32_t nchunk,
-                        const uint32_t* cost, uint32_t* sched, uint32_t* order) {
-  cudaError_t e = cudaMemsetAsync(sched, 0, kSchedWords * sizeof(uint32_t), st);
-  if (e != cudaSuccess) return e;
+                        uint32_t* cost, uint32_t* sched, uint32_t* order) {
   // costs are those of an item's longest task; its tasks share the total
   const float share = kHeavyShare / float(b.ts == 8 ? 1u : raster_slabs_per_tile(b.ts, b.ppl));
   k_order_hist<<<296, 256, 0, st>>>(b, off1, nchunk, cost, sched);
@@ -388,18 +374,11 @@ int tiles_fill(cudaStream_t st, uint32_t n, const float* xyd, const float* aabb,
   }
   const uint32_t npad = ceil_div(n, kSortTile) * kSortTile;
   ViewBatch b = single_view_batch(img_w, img_h, int(ts), tile_w, tile_h);
-  if (npad > n) {
-    k_pad_keys<<<blocks_for(npad - n, 256), 256, 0, st>>>(t.dka, n, npad, 1);
-    count_launch();
-  }
-  k_prep_tiles<<<blocks_for(n, 256), 256, 0, st>>>(n, xyd, aabb, rad, int(ts), int(tile_w), int(tile_h), t.rect,
-                                                  t.dka);
+  k_prep_tiles<<<blocks_for(npad, 256), 256, 0, st>>>(n, npad, xyd, aabb, rad, int(ts), int(tile_w), int(tile_h),
+                                                     t.rect, t.dka);
   count_launch();
-  bool in_b = false;
-  TRY_CUDA(radix_sort(st, t.dka, t.dva, t.dkb, t.dvb, npad, nullptr, 32, 1, t.hist, t.scan_tmp, &in_b, t.rect, n,
-                      t.srect, true, n),
-           "depth sort");
-  const uint32_t* order = in_b ? t.dvb : t.dva;
+  TRY_CUDA(depth_sort(st, t.dka, t.dva, t.dkb, t.dvb, npad, 1, t.hist, t.scan_tmp, t.rect, n, t.srect), "depth sort");
+  const uint32_t* order = t.dva;
   int rc = build_sb_lists(st, b, n, npad, order, t.srect, t.lists, t.scan_tmp, capacity, t.flags);
   if (rc) return rc;
   rc = build_tile_lists(st, b, npad, t.lists, t.segcnt, t.scan_tmp, tile2idx, idx2pnt, keys64 ? t.out_tile : nullptr, capacity,
@@ -499,12 +478,13 @@ BatchWs carve_batch(void* ws, uint32_t n, const ViewBatch& b, uint64_t capacity)
   L.npad = npad;
   L.slabs_per_tile = raster_slabs_per_tile(b.ts, b.ppl);
   w.flags = c.take<uint32_t>(16, &L.off_flags);
+  w.sched = c.take<uint32_t>(kSchedWords);  // cleared with the flags
   w.rec = c.take<float4>(3 * VN + 3, &L.off_rec);
   w.rect = c.take<uint2>(VN + 1, &L.off_rect);
   w.srect = c.take<uint2>(Vp);
   w.cnt = c.take<uint32_t>(VN + 1, &L.off_cnt);
   w.dka = c.take<uint32_t>(Vp);
-  w.dva = c.take<uint32_t>(Vp, &L.off_order);  // 4 passes of 8 bits end back in (dka, dva)
+  w.dva = c.take<uint32_t>(Vp, &L.off_order);  // the depth sort ends in dva
   w.dkb = c.take<uint32_t>(Vp);
   w.dvb = c.take<uint32_t>(Vp);
   const size_t hw = radix_hist_words(Vp);
@@ -522,7 +502,6 @@ BatchWs carve_batch(void* ws, uint32_t n, const ViewBatch& b, uint64_t capacity)
   w.slab_loss = c.take<float>(size_t(b.num_items) * L.slabs_per_tile, &L.off_slab_loss);
   w.grad2d = c.take<float4>(3 * VN + 3, &L.off_grad2d);
   w.grad2d_tag = c.take<unsigned long long>(1);
-  w.sched = c.take<uint32_t>(kSchedWords);
   w.task_order = c.take<uint32_t>(size_t(b.num_items) + 1);
   w.item_cost = c.take<uint32_t>(size_t(b.num_items) + 1);
   L.total_bytes = align_up(c.off, 256);
@@ -746,27 +725,21 @@ int dsplat_gauss_batch_forward(dsplat_stream stream, const dsplat_gauss_params* 
   w = carve_batch(workspace, n, b, pair_capacity);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const uint32_t V = uint32_t(num_views), npad = w.L.npad;
-  const size_t Vp = size_t(V) * npad;
   stage_mark(st, 0);
-  TRY_CUDA(cudaMemsetAsync(w.flags, 0, 16 * sizeof(uint32_t), st), "memset");
+  TRY_CUDA(cudaMemsetAsync(w.flags, 0, size_t(reinterpret_cast<char*>(w.sched + kSchedWords) -
+                                              reinterpret_cast<char*>(w.flags)), st), "memset");
   if (n == 0 || pair_capacity == 0) {
     TRY_CUDA(cudaMemsetAsync(w.lists.off1, 0, (size_t(b.num_sb) * w.L.sb_chunks + 1) * 4, st), "memset");
   } else {
-    if (npad > n) {
-      k_pad_keys<<<blocks_for(size_t(npad - n) * V, 256), 256, 0, st>>>(w.dka, n, npad, V);
-      count_launch();
-    }
-    k_fused_project<<<blocks_for(n, 128), 128, 0, st>>>(n, npad, params->sh_degree, params->means,
+    k_fused_project<<<blocks_for(npad, 128), 128, 0, st>>>(n, npad, params->sh_degree, params->means,
                                                         params->log_scales, params->quats, params->opacity,
                                                         params->colors, b, w.rec, w.rect, w.dka, nullptr);
     count_launch();
     stage_mark(st, 1);
-    bool in_b = false;
-    TRY_CUDA(radix_sort(st, w.dka, w.dva, w.dkb, w.dvb, Vp, nullptr, 32, V, w.hist, w.scan_tmp, &in_b, w.rect, n,
-                        w.srect, true, n),
+    TRY_CUDA(depth_sort(st, w.dka, w.dva, w.dkb, w.dvb, npad, V, w.hist, w.scan_tmp, w.rect, n, w.srect),
              "depth sort");
     stage_mark(st, 2);
-    const uint32_t* order = in_b ? w.dvb : w.dva;
+    const uint32_t* order = w.dva;
     int rc2 = build_sb_lists(st, b, n, npad, order, w.srect, w.lists, w.scan_tmp, pair_capacity, w.flags);
     if (rc2) return rc2;
     stage_mark(st, 3);
@@ -774,18 +747,13 @@ int dsplat_gauss_batch_forward(dsplat_stream stream, const dsplat_gauss_params* 
   // longest-first raster task order (costs measured by the previous forward)
   TRY_CUDA(order_tasks(st, b, w.lists.off1, w.L.sb_chunks, w.item_cost, w.sched, w.task_order),
            "task order");
-  TRY_CUDA(cudaMemsetAsync(w.item_cost, 0, size_t(b.num_items) * sizeof(uint32_t), st), "memset");
   stage_mark(st, 4);
   const FwdArgs fa{n,           w.rec,   w.lists.list1, w.lists.off1, w.L.sb_chunks, pair_capacity, w.task_order, w.sched,
                    w.flags + 2, out_rgb, w.pix_T,       w.pix_stop,   target,        w.grad_pix,    w.slab_loss,
-                   w.item_cost};
+                   w.item_cost, out_alpha};
   TRY_CUDA(raster_fwd(st, b, fa),
            "raster_fwd");
   stage_mark(st, 5);
-  if (out_alpha) {
-    k_one_minus<<<blocks_for(b.num_pix, 256), 256, 0, st>>>(w.pix_T, out_alpha, b.num_pix);
-    count_launch();
-  }
   TRY_CUDA(cudaGetLastError(), "forward");
   return DSPLAT_OK;
 }
@@ -814,9 +782,8 @@ int dsplat_gauss_batch_backward(dsplat_stream stream, const dsplat_gauss_params*
   // consumes, so only a buffer not known to be clean is cleared here
   const unsigned long long tag = grad2d_tag_value(w.L, n, num_views);
   k_prepare_grad2d<<<blocks_for(3 * VN, 256) < 4096 ? blocks_for(3 * VN, 256) : 4096, 256, 0, st>>>(
-      w.grad2d_tag, tag, w.grad2d, 3 * VN);
+      w.grad2d_tag, tag, w.grad2d, 3 * VN, w.flags + 3);
   count_launch();
-  TRY_CUDA(cudaMemsetAsync(w.flags + 3, 0, sizeof(uint32_t), st), "memset");
   // the forward's longest-first task order: it ranks the tasks by the walks
   // of the forward before it, the same measure as this forward's (equal once
   // the scene stops changing), and every order gives the same results

@@ -68,6 +68,7 @@ struct FwdArgs {
   float* grad_pix;
   float* slab_loss;
   uint32_t* item_cost;
+  float* out_alpha;
 };
 
 struct BwdArgs {

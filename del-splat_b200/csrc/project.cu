@@ -277,12 +277,15 @@ __device__ __forceinline__ TileSpan tile_span(uint32_t i, const float* __restric
   return s;
 }
 
-// Span and depth key of every point.
-__global__ void k_prep_tiles(uint32_t n, const float* __restrict__ xyd, const float* __restrict__ aabb,
+// Span and depth key of every point; the keys from n to npad are all ones.
+__global__ void k_prep_tiles(uint32_t n, uint32_t npad, const float* __restrict__ xyd, const float* __restrict__ aabb,
                              const float* __restrict__ rad, int ts, int tile_w, int tile_h,
                              uint2* __restrict__ rect, uint32_t* __restrict__ dkey) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+  if (i >= n) {
+    if (i < npad) dkey[i] = 0xffffffffu;
+    return;
+  }
   const TileSpan s = tile_span(i, xyd, aabb, rad, ts, tile_w, tile_h);
   rect[i] = pack_rect(s.x0, s.y0, s.x1, s.y1);
   dkey[i] = s.count() ? depth_bits(xyd[3 * size_t(i) + 2]) : 0xffffffffu;
@@ -337,7 +340,11 @@ __global__ void __launch_bounds__(kProjThreads) k_fused_project(
     crow[(i / C) * kProjStride + (i % C)] = colors[size_t(g0) * C + i];
   __syncthreads();
   const uint32_t g = g0 + threadIdx.x;
-  if (g >= n) return;
+  if (g >= n) {  // padding keys
+    if (g < npad)
+      for (int v = 0; v < b.num_views; ++v) dkey[size_t(v) * npad + g] = 0xffffffffu;
+    return;
+  }
   const float p[3] = {means[3 * g], means[3 * g + 1], means[3 * g + 2]};
   const float s[3] = {expf_cr(log_scales[3 * g]), expf_cr(log_scales[3 * g + 1]),
                       expf_cr(log_scales[3 * g + 2])};

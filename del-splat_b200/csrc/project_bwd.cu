@@ -361,9 +361,11 @@ __global__ void __launch_bounds__(kColThreads) k_project_bwd_colour(uint32_t n, 
 
 // Clears grad2d unless the tag says it is already all zero (the previous
 // backward on this layout consumed it).  Blocks only read the tag; the
-// colour kernel of the same backward writes it.
+// colour kernel of the same backward writes it.  Also sets the backward
+// raster's work counter to zero.
 __global__ void k_prepare_grad2d(const unsigned long long* __restrict__ clean_tag, unsigned long long tag,
-                                 float4* __restrict__ grad2d, size_t count) {
+                                 float4* __restrict__ grad2d, size_t count, uint32_t* __restrict__ work_counter) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) *work_counter = 0u;
   if (*clean_tag == tag) return;
   for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += size_t(gridDim.x) * blockDim.x)
     grad2d[i] = make_float4(0.f, 0.f, 0.f, 0.f);

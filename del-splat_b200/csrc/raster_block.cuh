@@ -160,6 +160,7 @@ struct SbWords {
 struct FwdOut {  // where a block's results go
   float* rgb;
   float* T;         // nullable
+  float* alpha;     // nullable: 1 - T
   uint32_t* last;   // nullable
   const float* target;  // nullable; with it grad_pix and the loss
   float* grad_pix;
@@ -323,6 +324,7 @@ __device__ __forceinline__ uint32_t blend_block(const Walk& walk, const Src& src
     out.rgb[3 * p + 1] = o.z;
     out.rgb[3 * p + 2] = o.w;
     if (out.T) out.T[p] = o.x;
+    if (out.alpha) out.alpha[p] = 1.f - o.x;
     if (out.last) out.last[p] = park_pos[32 * k + lane];
     if (out.target) {
       const float d0 = o.y - out.target[3 * p], d1 = o.z - out.target[3 * p + 1], d2 = o.w - out.target[3 * p + 2];

@@ -33,7 +33,8 @@ __device__ __forceinline__ uint32_t fwd_slab(const Walk& walk, const Src& src, E
                                          uint32_t* park_pos, const float* tab, float nz,
                                          uint32_t s, uint32_t e, int px0, int py0, int w, int h, int xend,
                                          float* __restrict__ out_rgb, size_t pix_base, float* __restrict__ out_T,
-                                         uint32_t* __restrict__ out_last, const float* __restrict__ target,
+                                         float* __restrict__ out_alpha, uint32_t* __restrict__ out_last,
+                                         const float* __restrict__ target,
                                          float* __restrict__ grad_pix, const Loss& loss) {
   using G = Geo<TS, PPL_>;
   constexpr int PPL = G::PPL;
@@ -213,6 +214,7 @@ __device__ __forceinline__ uint32_t fwd_slab(const Walk& walk, const Src& src, E
     out_rgb[3 * p + 1] = o.z;
     out_rgb[3 * p + 2] = o.w;
     if (out_T) out_T[p] = o.x;
+    if (out_alpha) out_alpha[p] = 1.f - o.x;
     if (out_last) out_last[p] = park_pos[k * 32 + lane];
     if (target) {
       const float d0 = o.y - target[3 * p], d1 = o.z - target[3 * p + 1], d2 = o.w - target[3 * p + 2];
@@ -244,8 +246,8 @@ __global__ void __launch_bounds__(32 * kRasterWarps) k_raster_fwd(
     const ViewBatch b, uint32_t n, const float4* __restrict__ rec, const uint2* __restrict__ list1,
     const uint32_t* __restrict__ off1, uint32_t nchunk, uint64_t capacity, const uint32_t* __restrict__ order,
     const uint32_t* __restrict__ sched, uint32_t* __restrict__ work_counter, float* __restrict__ out_rgb,
-    float* __restrict__ out_T, uint32_t* __restrict__ out_last, const float* __restrict__ target,
-    float* __restrict__ grad_pix, float* __restrict__ slab_loss, uint32_t slots, uint32_t* __restrict__ item_cost,
+    float* __restrict__ out_T, float* __restrict__ out_alpha, uint32_t* __restrict__ out_last,
+    const float* __restrict__ target, float* __restrict__ grad_pix, float* __restrict__ slab_loss, uint32_t slots, uint32_t* __restrict__ item_cost,
     float nz) {
   using G = TaskGeo<TS, PPL, NT>;
   static_assert(sizeof(EntB) >= sizeof(EntP), "the warps' entries of either form share their place");
@@ -277,7 +279,7 @@ __global__ void __launch_bounds__(32 * kRasterWarps) k_raster_fwd(
     if (t.block) {
       BlockPlace p;
       if (!block_place(b, ig, t.sub, nx, &p)) continue;
-      const FwdOut out{out_rgb, out_T, out_last, target, grad_pix};
+      const FwdOut out{out_rgb, out_T, out_alpha, out_last, target, grad_pix};
       cost = blend_block<false>(SbWords{list1, p.lx, ig.ly, 1u}, PackedBlockSrc{src.rec}, ent, park, park_pos, tab, nz,
                                 ig.s, ig.e, p.px0, p.py0, vd.w, vd.w, vd.h, false, vd.pix_base, out, [&](float l) {
                                   float* const p0 = slab_loss + size_t(t.item) * slots;
@@ -291,7 +293,7 @@ __global__ void __launch_bounds__(32 * kRasterWarps) k_raster_fwd(
       const int xend = min(vd.w, ig.px0 + int(nx) * TS);
       cost = fwd_slab<G::GX, G::PPL, NT == 2 && G::PPL == 4>(
           walk, src, reinterpret_cast<EntP*>(ent), park, park_pos, tab, nz, ig.s, ig.e, ig.px0,
-          ig.py0 + int(t.sub) * G::SLAB_ROWS, vd.w, vd.h, xend, out_rgb, vd.pix_base, out_T, out_last, target,
+          ig.py0 + int(t.sub) * G::SLAB_ROWS, vd.w, vd.h, xend, out_rgb, vd.pix_base, out_T, out_alpha, out_last, target,
           grad_pix, [&](float l) {
             float* const p0 = slab_loss + size_t(t.item) * G::SLABS + t.sub;
             *p0 = l;
@@ -324,7 +326,7 @@ __global__ void __launch_bounds__(32 * kRasterWarps, 6) k_raster_fwd_aos(
   const int px0 = int(tile % uint32_t(tile_w)) * ts + int(blk % side) * kBlock;
   const int py0 = int(tile / uint32_t(tile_w)) * ts + int(blk / side) * kBlock;
   if (px0 >= w || py0 >= h) return;
-  const FwdOut out{pix2rgb, out_T, out_last, nullptr, nullptr};
+  const FwdOut out{pix2rgb, out_T, nullptr, out_last, nullptr, nullptr};
   blend_block<CUDA_STOP>(TileWords{idx2pnt}, src, ent[warp], park[warp], park_pos[warp], tab, nz, tile2idx[tile],
                          tile2idx[tile + 1], px0, py0, w, w, h, true, 0, out, [](float) {});
 }
@@ -340,7 +342,7 @@ static cudaError_t launch_fwd(cudaStream_t st, const ViewBatch& b, const FwdArgs
   k_raster_fwd<TS, PPL, NT>
       <<<persistent_grid(k_raster_fwd<TS, PPL, NT>, max_tasks(b, TaskGeo<TS, PPL, NT>::SLABS)), 32 * kRasterWarps, 0,
          st>>>(b, a.n, a.rec, a.list1, a.off1, a.nchunk, a.capacity, a.order, a.sched, a.counter, a.out_rgb, a.out_T,
-               a.out_last, a.target, a.grad_pix, a.slab_loss, slots, a.item_cost, -0.f);
+               a.out_alpha, a.out_last, a.target, a.grad_pix, a.slab_loss, slots, a.item_cost, -0.f);
   count_launch();
   return cudaGetLastError();
 }

@@ -63,50 +63,81 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t x, uint32_t* total)
   return r;
 }
 
+// This thread's kScanItems words from `base` on (base is a multiple of 8, in
+// 16-byte aligned), zero from n on.
+__device__ __forceinline__ void scan_load(const uint32_t* __restrict__ in, size_t base, size_t n, uint32_t* v) {
+  if (base + kScanItems <= n) {
+    const uint4 a = *reinterpret_cast<const uint4*>(in + base), c = *reinterpret_cast<const uint4*>(in + base + 4);
+    v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w;
+    v[4] = c.x, v[5] = c.y, v[6] = c.z, v[7] = c.w;
+  } else {
+#pragma unroll
+    for (int i = 0; i < kScanItems; ++i) v[i] = base + i < n ? in[base + i] : 0u;
+  }
+}
+
 __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const uint32_t* __restrict__ in, size_t n,
                                                               uint32_t* __restrict__ sums) {
-  const size_t base = size_t(blockIdx.x) * kScanTile + size_t(threadIdx.x) * kScanItems;
-  uint32_t s = 0;
+  uint32_t v[kScanItems], s = 0;
+  scan_load(in, size_t(blockIdx.x) * kScanTile + size_t(threadIdx.x) * kScanItems, n, v);
 #pragma unroll
-  for (int i = 0; i < kScanItems; ++i)
-    if (base + i < n) s += in[base + i];
+  for (int i = 0; i < kScanItems; ++i) s += v[i];
   __shared__ uint32_t tot;
   block_excl_scan(s, &tot);
   if (threadIdx.x == 0) sums[blockIdx.x] = tot;
 }
 
+// out[i] = sum of in[0, i) for i in [0, n], at most limit; a total above limit
+// sets the overflow flag.
 __global__ void __launch_bounds__(kScanThreads) k_scan_apply(const uint32_t* __restrict__ in,
                                                              uint32_t* __restrict__ out, size_t n,
-                                                             const uint32_t* __restrict__ sums) {
+                                                             const uint32_t* __restrict__ sums, uint32_t limit,
+                                                             uint32_t* __restrict__ flags) {
   const size_t base = size_t(blockIdx.x) * kScanTile + size_t(threadIdx.x) * kScanItems;
-  uint32_t v[kScanItems];
-  uint32_t s = 0;
+  uint32_t v[kScanItems], s = 0;
+  scan_load(in, base, n, v);
 #pragma unroll
-  for (int i = 0; i < kScanItems; ++i) {
-    v[i] = base + i < n ? in[base + i] : 0u;
-    s += v[i];
-  }
-  // the earlier blocks' totals, summed by every block itself (a few hundred
-  // words for the scans here, so no separate pass scans them)
-  uint32_t part = 0;
-  for (uint32_t i = threadIdx.x; i < blockIdx.x; i += kScanThreads) part += sums[i];
+  for (int i = 0; i < kScanItems; ++i) s += v[i];
   __shared__ uint32_t carry, tot;
-  block_excl_scan(part, &carry);
-  uint32_t p = block_excl_scan(s, &tot) + carry;
+  uint32_t p = block_excl_scan(s, &tot);
+  if (blockIdx.x > 0) {
+    // the earlier blocks' totals, summed by every block itself (a few hundred
+    // words for the scans here, so no separate pass scans them)
+    uint32_t part = 0;
+    for (uint32_t i = threadIdx.x; i < blockIdx.x; i += kScanThreads) part += sums[i];
+    block_excl_scan(part, &carry);
+    p += carry;
+  }
+  uint32_t o[kScanItems];
 #pragma unroll
   for (int i = 0; i < kScanItems; ++i) {
-    if (base + i < n) out[base + i] = p;
+    o[i] = min(p, limit);
+    if (base + i == n && p > limit) set_flag(flags, kFlagPairOverflow);
     p += v[i];
+  }
+  if (base + kScanItems <= n && (reinterpret_cast<uintptr_t>(out) & 15u) == 0) {
+    *reinterpret_cast<uint4*>(out + base) = make_uint4(o[0], o[1], o[2], o[3]);
+    *reinterpret_cast<uint4*>(out + base + 4) = make_uint4(o[4], o[5], o[6], o[7]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < kScanItems; ++i)
+      if (base + i <= n) out[base + i] = o[i];
   }
 }
 
-size_t scan_tmp_words(size_t n) { return (n + kScanTile - 1) / kScanTile + 1; }
+size_t scan_tmp_words(size_t n) { return n / kScanTile + 2; }
 
-cudaError_t exclusive_scan(cudaStream_t st, const uint32_t* in, uint32_t* out, size_t n, uint32_t* tmp) {
-  if (n == 0) return cudaSuccess;
-  const uint32_t nb = uint32_t((n + kScanTile - 1) / kScanTile);
-  k_scan_reduce<<<nb, kScanThreads, 0, st>>>(in, n, tmp); count_launch();
-  k_scan_apply<<<nb, kScanThreads, 0, st>>>(in, out, n, tmp); count_launch();
+// out[0, n] <- exclusive sums of in[0, n) and their total (one launch up to
+// kScanTile - 1 words); out may be in when the total is not wanted there.
+cudaError_t exclusive_scan(cudaStream_t st, const uint32_t* in, uint32_t* out, size_t n, uint32_t* tmp,
+                           uint32_t limit, uint32_t* flags) {
+  const uint32_t nb = uint32_t(n / kScanTile + 1);
+  if (nb > 1) {
+    k_scan_reduce<<<nb, kScanThreads, 0, st>>>(in, n, tmp);
+    count_launch();
+  }
+  k_scan_apply<<<nb, kScanThreads, 0, st>>>(in, out, n, tmp, limit, flags);
+  count_launch();
   return cudaGetLastError();
 }
 
@@ -118,12 +149,19 @@ cudaError_t exclusive_scan(cudaStream_t st, const uint32_t* in, uint32_t* out, s
 // segments never mix.
 //   upsweep:   16-byte key loads, per-warp shared histograms;
 //   downsweep: warp w ranks its 512 elements (16 rounds of 32, in index
-//              order) with match_any; the block turns the per-warp counts
-//              into local digit offsets, scatters (key, value) into shared
-//              memory in digit order, and writes each digit's run to its
-//              global offset with consecutive threads on consecutive
-//              addresses.
-// ---------------------------------------------------------------------------
+//              order) with ballots against its running digit counts; the
+//              block turns the counts into local digit offsets, scatters
+//              (key, value) into shared memory in digit order, and writes each
+//              digit's run to its global offset with consecutive threads on
+//              consecutive addresses.
+// Short segments need fewer launches, which is what bounds them:
+//   up to kRsFewBlocks blocks per segment the downsweep sums the segment's
+//   histograms itself (no scan: 8 launches instead of 16; 25 blocks in 8
+//   segments 97 -> 63 us; with 64 blocks the sums take as long as the scans,
+//   63 against 55);
+//   up to 8192 elements per segment one block sorts it in shared memory, all
+//   four digits in one launch (1,000 elements 34 us in 16 launches -> 10 in
+//   one; 3,000 -> 16).
 constexpr int kRsThreads = 256;
 constexpr int kRsWarps = kRsThreads / 32;
 constexpr int kRsRounds = 16;
@@ -163,7 +201,23 @@ __device__ __forceinline__ uint32_t peers_of_digit(uint32_t d) {
   return m;
 }
 
-__global__ void __launch_bounds__(kRsThreads) k_radix_downsweep(
+// This element's rank among its warp's elements of the same digit so far
+// (counts[d] of them in earlier rounds), which it joins.
+__device__ __forceinline__ uint32_t warp_digit_rank(uint32_t* counts, uint32_t d, int lane, uint32_t lt) {
+  const uint32_t peers = peers_of_digit(d);
+  const uint32_t before = counts[d];
+  __syncwarp();
+  if (lane == __ffs(peers) - 1) counts[d] = before + __popc(peers);
+  __syncwarp();
+  return before + __popc(peers & lt);
+}
+
+constexpr uint32_t kRsFewBlocks = 32;
+
+// FEW: offs holds the blocks' counts, which every block sums for itself;
+// otherwise their exclusive scan.
+template <bool FEW>
+__global__ void __launch_bounds__(kRsThreads, FEW ? 2 : 3) k_radix_downsweep(
     const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin, uint32_t* __restrict__ kout,
     uint32_t* __restrict__ vout, int shift, uint32_t nb_seg, const uint32_t* __restrict__ offs, int write_keys,
     const uint2* __restrict__ gather_src, uint32_t gather_n, uint2* __restrict__ gather_dst, uint32_t iota_n) {
@@ -172,6 +226,7 @@ __global__ void __launch_bounds__(kRsThreads) k_radix_downsweep(
   __shared__ uint32_t goff[256];
   __shared__ uint32_t sk[kRsTile];
   __shared__ uint32_t sv[kRsTile];
+  __shared__ uint32_t block_total;
 #pragma unroll
   for (int w = 0; w < kRsWarps; ++w) wc[w][threadIdx.x] = 0;
   __syncthreads();
@@ -196,15 +251,10 @@ __global__ void __launch_bounds__(kRsThreads) k_radix_downsweep(
       v[r] = local < iota_n ? local : 0xffffffffu;
     }
   }
-  // phase 1: per-warp digit counts (the peer masks are kept for phase 3)
-  uint32_t pm[kRsRounds];
+  // phase 1: ranks inside the warp, per-warp digit counts
+  uint32_t rank[kRsRounds];
 #pragma unroll
-  for (int r = 0; r < kRsRounds; ++r) {
-    const uint32_t d = (k[r] >> shift) & 255u;
-    pm[r] = peers_of_digit(d);
-    if (lane == __ffs(pm[r]) - 1) wc[warp][d] += __popc(pm[r]);
-    __syncwarp();
-  }
+  for (int r = 0; r < kRsRounds; ++r) rank[r] = warp_digit_rank(wc[warp], (k[r] >> shift) & 255u, lane, lt);
   __syncthreads();
   // phase 2: block-local digit starts, warp bases, global digit offsets
   {
@@ -212,8 +262,7 @@ __global__ void __launch_bounds__(kRsThreads) k_radix_downsweep(
     uint32_t tot = 0;
 #pragma unroll
     for (int w = 0; w < kRsWarps; ++w) tot += wc[w][d];
-    uint32_t all;
-    uint32_t run = block_excl_scan(tot, &all);
+    uint32_t run = block_excl_scan(tot, &block_total);
     dstart[d] = run;
 #pragma unroll
     for (int w = 0; w < kRsWarps; ++w) {
@@ -222,19 +271,25 @@ __global__ void __launch_bounds__(kRsThreads) k_radix_downsweep(
       run += t;
     }
     const uint32_t seg = blockIdx.x / nb_seg, b = blockIdx.x % nb_seg;
-    goff[d] = offs[(size_t(seg) * 256 + d) * nb_seg + b];
+    const uint32_t* h = offs + (size_t(seg) * 256 + d) * nb_seg;
+    if (!FEW) {
+      goff[d] = h[b];
+    } else {
+      uint32_t before = 0, all = 0;
+#pragma unroll 16
+      for (uint32_t i = 0; i < nb_seg; ++i) {
+        const uint32_t c = h[i];
+        if (i < b) before += c;
+        all += c;
+      }
+      goff[d] = seg * nb_seg * kRsTile + block_excl_scan(all, &block_total) + before;
+    }
   }
   __syncthreads();
   // phase 3: stable scatter into shared memory, digit-major
 #pragma unroll
   for (int r = 0; r < kRsRounds; ++r) {
-    const uint32_t d = (k[r] >> shift) & 255u;
-    const uint32_t peers = pm[r];
-    const uint32_t rb = wc[warp][d];
-    __syncwarp();
-    if (lane == __ffs(peers) - 1) wc[warp][d] = rb + __popc(peers);
-    __syncwarp();
-    const uint32_t lp = rb + __popc(peers & lt);
+    const uint32_t lp = wc[warp][(k[r] >> shift) & 255u] + rank[r];
     sk[lp] = k[r];
     sv[lp] = v[r];
   }
@@ -258,62 +313,139 @@ __global__ void __launch_bounds__(kRsThreads) k_radix_downsweep(
   }
 }
 
-size_t radix_hist_words(size_t n) { return ((n + kRsTile - 1) / kRsTile) * 256; }
+size_t radix_hist_words(size_t n) { return ((n + kRsTile - 1) / kRsTile) * 256 + 1; }
 
-// Sorts (ka, va) by bits [0, nbits) of the key, ping-ponging with (kb, vb).
-// Returns in *result_in_b whether the sorted values ended in the b buffers;
-// the keys of the last pass are not written (callers use the values only).
-// n must be a multiple of 4096 (per segment when nseg > 1); count_ptr must be
-// null (every element takes part).
-// gather_dst (nullable): the last pass also writes, per sorted position,
-// gather_src[segment * gather_n + value] (an empty record for padding).
-// iota_values: the values are the identity permutation (each segment's
-// element indices, 0xffffffff from iota_n on); va is not read, the first pass
-// forms them.
-cudaError_t radix_sort(cudaStream_t st, uint32_t* ka, uint32_t* va, uint32_t* kb, uint32_t* vb, size_t n,
-                       const uint32_t* count_ptr, int nbits, uint32_t nseg, uint32_t* hist, uint32_t* scan_tmp,
-                       bool* result_in_b, const uint2* gather_src, uint32_t gather_n, uint2* gather_dst,
-                       bool iota_values, uint32_t iota_n) {
-  if (n % kRsTile != 0 || count_ptr != nullptr || nseg == 0 || (n / kRsTile) % nseg != 0)
-    return cudaErrorInvalidValue;
-  const uint32_t nblocks = uint32_t(n / kRsTile);
-  const uint32_t nb_seg = nblocks / nseg;
-  const size_t hw = size_t(nblocks) * 256;
-  bool in_b = false;
-  if (n == 0) {
-    *result_in_b = false;
-    return cudaSuccess;
+// One block sorts a whole segment of up to THREADS * kBsRounds elements in
+// shared memory: the same ranking, four digits one after the other, every
+// warp with the same number of rounds of 32 consecutive elements.
+constexpr int kBsRounds = 8;
+
+template <int THREADS>
+struct BlockSortShared {
+  uint32_t keys[THREADS * kBsRounds];
+  uint16_t idx[THREADS * kBsRounds];
+  uint32_t wc[THREADS / 32][256];
+  uint32_t total;
+};
+
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) k_block_sort(const uint32_t* __restrict__ kin, uint32_t n, uint32_t npad,
+                                                        uint32_t* __restrict__ vout,
+                                                        const uint2* __restrict__ gather_src,
+                                                        uint2* __restrict__ gather_dst) {
+  extern __shared__ __align__(16) unsigned char bs_raw[];
+  BlockSortShared<THREADS>& sh = *reinterpret_cast<BlockSortShared<THREADS>*>(bs_raw);
+  constexpr int WARPS = THREADS / 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t lt = (1u << lane) - 1u, seg = blockIdx.x;
+  const uint32_t rounds = (n + THREADS - 1) / THREADS;  // of this segment
+  const uint32_t place0 = uint32_t(warp) * rounds * 32 + lane;
+  // places from n on hold all-ones keys, which stay behind every element
+  uint32_t k[kBsRounds], v[kBsRounds];  // v: index << 16 | rank
+#pragma unroll
+  for (int r = 0; r < kBsRounds; ++r) {
+    const uint32_t i = place0 + 32 * r;
+    k[r] = uint32_t(r) < rounds && i < n ? kin[size_t(seg) * npad + i] : 0xffffffffu;
+    v[r] = i << 16;
   }
-  for (int shift = 0; shift < nbits; shift += 8) {
-    const uint32_t* ki = in_b ? kb : ka;
-    const uint32_t* vi = iota_values && shift == 0 ? nullptr : in_b ? vb : va;
-    uint32_t* ko = in_b ? ka : kb;
-    uint32_t* vo = in_b ? va : vb;
-    k_radix_upsweep<<<nblocks, kRsThreads, 0, st>>>(ki, shift, nb_seg, hist); count_launch();
-    cudaError_t e = exclusive_scan(st, hist, hist, hw, scan_tmp);
+#pragma unroll 1
+  for (int shift = 0; shift < 32; shift += 8) {
+    for (int i = threadIdx.x; i < WARPS * 256; i += THREADS) (&sh.wc[0][0])[i] = 0;
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kBsRounds; ++r)
+      if (uint32_t(r) < rounds) v[r] |= warp_digit_rank(sh.wc[warp], (k[r] >> shift) & 255u, lane, lt);
+    __syncthreads();
+    uint32_t c[WARPS], tot = 0;  // digit threadIdx.x's counts, warp by warp
+    if (threadIdx.x < 256) {
+#pragma unroll
+      for (int w = 0; w < WARPS; ++w) {
+        c[w] = sh.wc[w][threadIdx.x];
+        tot += c[w];
+      }
+    }
+    uint32_t run = block_excl_scan(tot, &sh.total);
+    if (threadIdx.x < 256) {
+#pragma unroll
+      for (int w = 0; w < WARPS; ++w) {
+        sh.wc[w][threadIdx.x] = run;
+        run += c[w];
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kBsRounds; ++r)
+      if (uint32_t(r) < rounds) {
+        const uint32_t lp = sh.wc[warp][(k[r] >> shift) & 255u] + (v[r] & 0xffffu);
+        sh.keys[lp] = k[r];
+        sh.idx[lp] = uint16_t(v[r] >> 16);
+      }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kBsRounds; ++r)
+      if (uint32_t(r) < rounds) {
+        k[r] = sh.keys[place0 + 32 * r];
+        v[r] = uint32_t(sh.idx[place0 + 32 * r]) << 16;
+      }
+    __syncthreads();
+  }
+  for (uint32_t i = threadIdx.x; i < npad; i += THREADS) {
+    const uint32_t idx = i < rounds * THREADS ? sh.idx[i] : 0xffffu;
+    const bool real = idx < n;
+    vout[size_t(seg) * npad + i] = real ? idx : 0xffffffffu;
+    gather_dst[size_t(seg) * npad + i] = real ? gather_src[size_t(seg) * n + idx] : make_uint2(0u, 0u);
+  }
+}
+
+template <int THREADS>
+static cudaError_t block_sort(cudaStream_t st, const uint32_t* keys, uint32_t n, uint32_t npad, uint32_t nseg,
+                              uint32_t* vout, const uint2* gather_src, uint2* gather_dst) {
+  constexpr int smem = int(sizeof(BlockSortShared<THREADS>));
+  if (smem > 48 * 1024) {
+    const cudaError_t e =
+        cudaFuncSetAttribute(k_block_sort<THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    const int last = shift + 8 >= nbits;
-    k_radix_downsweep<<<nblocks, kRsThreads, 0, st>>>(ki, vi, ko, vo, shift, nb_seg, hist, last ? 0 : 1,
-                                                       gather_src, gather_n, last ? gather_dst : nullptr, iota_n);
-    count_launch();
-    in_b = !in_b;
   }
-  *result_in_b = in_b;
+  k_block_sort<THREADS><<<nseg, THREADS, smem, st>>>(keys, n, npad, vout, gather_src, gather_dst);
+  count_launch();
+  return cudaGetLastError();
+}
+
+// Stable order of every segment's n elements by their 32-bit keys in ka
+// ([nseg][npad], all-ones from n on; ka, kb and vb are scratch after): va gets
+// the elements' indices in their segment, 0xffffffff for the padding, and
+// gather_dst gather_src's record of each ([nseg][n], an empty one for the
+// padding).  npad is a multiple of 4096.
+cudaError_t depth_sort(cudaStream_t st, uint32_t* ka, uint32_t* va, uint32_t* kb, uint32_t* vb, uint32_t npad,
+                       uint32_t nseg, uint32_t* hist, uint32_t* scan_tmp, const uint2* gather_src, uint32_t n,
+                       uint2* gather_dst) {
+  if (npad == 0 || npad % kRsTile != 0 || nseg == 0) return cudaErrorInvalidValue;
+  if (n <= 512 * kBsRounds) return block_sort<512>(st, ka, n, npad, nseg, va, gather_src, gather_dst);
+  if (n <= 1024 * kBsRounds) return block_sort<1024>(st, ka, n, npad, nseg, va, gather_src, gather_dst);
+  const uint32_t nb_seg = npad / kRsTile, nblocks = nb_seg * nseg;
+  const bool few = nb_seg <= kRsFewBlocks;
+  for (int pass = 0; pass < 4; ++pass) {
+    const uint32_t* ki = pass & 1 ? kb : ka;
+    const uint32_t* vi = pass == 0 ? nullptr : pass & 1 ? vb : va;  // the first pass forms the indices
+    uint32_t* ko = pass & 1 ? ka : kb;
+    uint32_t* vo = pass & 1 ? va : vb;
+    k_radix_upsweep<<<nblocks, kRsThreads, 0, st>>>(ki, 8 * pass, nb_seg, hist);
+    count_launch();
+    if (!few) {
+      const cudaError_t e = exclusive_scan(st, hist, hist, size_t(nblocks) * 256, scan_tmp, 0xffffffffu, nullptr);
+      if (e != cudaSuccess) return e;
+    }
+    const bool last = pass == 3;  // its keys are not needed
+    (few ? k_radix_downsweep<true> : k_radix_downsweep<false>)<<<nblocks, kRsThreads, 0, st>>>(
+        ki, vi, ko, vo, 8 * pass, nb_seg, hist, last ? 0 : 1, gather_src, n, last ? gather_dst : nullptr, n);
+    count_launch();
+  }
   return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------------------
 // Rank order helpers
 // ---------------------------------------------------------------------------
-// Keys of the padding elements [n, npad) of every segment: 0xffffffff (they
-// sort last; their values are formed by the sort's first pass).
-__global__ void k_pad_keys(uint32_t* __restrict__ keys, uint32_t n, uint32_t npad, uint32_t nseg) {
-  const uint32_t pad = npad - n;
-  const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= size_t(pad) * nseg) return;
-  keys[size_t(i / pad) * npad + n + uint32_t(i % pad)] = 0xffffffffu;
-}
-
 // superblock span of a tile span (superblocks of 1 << sl tiles per side);
 // empty if no tile
 __device__ __forceinline__ bool sb_span(uint2 rc, int sl, int* sx0, int* sy0, int* sx1, int* sy1) {
@@ -391,11 +523,19 @@ __global__ void __launch_bounds__(kMsThreads) k_sb_count(const uint32_t* __restr
 // span covers; the lanes covering superblock (x, y) are then
 // colmask[x] & rowmask[y], and a lane's slot is its popcount among them.
 // ---------------------------------------------------------------------------
+// Flags a capacity overflow when the superblock lists need more entries than
+// the capacity (the 64-bit total also catches a wrapped 32-bit offset scan).
+__device__ __forceinline__ void check_capacity(uint64_t capacity, uint32_t* __restrict__ flags) {
+  if (threadIdx.x == 0 && blockIdx.x == 0 && *reinterpret_cast<const unsigned long long*>(flags + 8) > capacity)
+    set_flag(flags, kFlagPairOverflow);
+}
+
 __global__ void __launch_bounds__(kMsThreads) k_sb_scatter(const uint32_t* __restrict__ order,
                                                            const uint2* __restrict__ srect, uint32_t chunk, uint32_t npad,
                                                            const ViewBatch b,
                                                            const uint32_t* __restrict__ off, uint64_t capacity,
                                                            uint2* __restrict__ list1, uint32_t* __restrict__ flags) {
+  check_capacity(capacity, flags);
   extern __shared__ uint32_t smem_ms[];  // [kMsWarps][nsb] counters, then [kMsWarps][2 * side] masks
   const uint32_t nchunk = npad / chunk;
   const uint32_t v = blockIdx.x / nchunk, c = blockIdx.x % nchunk;
@@ -501,6 +641,7 @@ __global__ void __launch_bounds__(kMsThreads) k_sb_scatter_staged(const uint32_t
                                                                   const uint32_t* __restrict__ off, uint64_t capacity,
                                                                   uint2* __restrict__ list1,
                                                                   uint32_t* __restrict__ flags, uint32_t qcap) {
+  check_capacity(capacity, flags);
   extern __shared__ uint32_t smem_ms[];
   __shared__ uint32_t sub_total;
   const uint32_t nchunk = npad / chunk;
@@ -665,8 +806,9 @@ __global__ void k_order_hist(const ViewBatch b, const uint32_t* __restrict__ off
 // bucket and block instead of one per item on 33 hot counters); every block
 // forms the buckets' starts from the counts itself.  heavy_share: an item
 // is heavy when its cost times that is above the total cost.
+// The costs are set to zero for the next forward to measure.
 __global__ void k_order_scatter(const ViewBatch b, const uint32_t* __restrict__ off1, uint32_t nchunk,
-                                const uint32_t* __restrict__ cost, float heavy_share, uint32_t* __restrict__ sched,
+                                uint32_t* __restrict__ cost, float heavy_share, uint32_t* __restrict__ sched,
                                 uint32_t* __restrict__ order) {
   __shared__ uint32_t cnt[33], base[33], start[33];
   if (threadIdx.x == 0) {
@@ -690,6 +832,7 @@ __global__ void k_order_scatter(const ViewBatch b, const uint32_t* __restrict__ 
     uint32_t bucket = 0, slot = 0;
     if (i < hi) {
       bucket = uint32_t(__clz(item_cost(b, i, off1, nchunk, cost)));
+      cost[i] = 0u;
       slot = atomicAdd(&cnt[bucket], 1u);
     }
     __syncthreads();
@@ -701,24 +844,6 @@ __global__ void k_order_scatter(const ViewBatch b, const uint32_t* __restrict__ 
   }
 }
 
-
-// Clamp tile ranges to the pair capacity after an overflow so that readers
-// stay in bounds (the results are then invalid and the flag is set).
-__global__ void k_clamp_ranges(uint32_t* __restrict__ item_start, uint32_t num_items, uint64_t capacity,
-                               uint32_t* __restrict__ flags) {
-  const uint32_t total = item_start[num_items];
-  if (total <= capacity) return;
-  if (blockIdx.x == 0 && threadIdx.x == 0) set_flag(flags, kFlagPairOverflow);
-  for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i <= num_items; i += size_t(gridDim.x) * blockDim.x)
-    if (item_start[i] > capacity) item_start[i] = uint32_t(capacity);
-}
-
-// Flags a capacity overflow when the superblock lists need more entries than
-// the capacity (the 64-bit total also catches a wrapped 32-bit offset scan).
-__global__ void k_check_capacity(const unsigned long long* __restrict__ entries, uint64_t capacity,
-                                 uint32_t* __restrict__ flags) {
-  if (threadIdx.x == 0 && blockIdx.x == 0 && *entries > capacity) set_flag(flags, kFlagPairOverflow);
-}
 
 // keys for the drop-in API: idx2tiledepth = (tile << 32) | depth bits of the
 // point, recomputed from pnt2pixxydepth

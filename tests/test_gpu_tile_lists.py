@@ -26,3 +26,21 @@ def test_segmented_lists(orc, dev, side, n):
     assert np.array_equal(U32(t2i), o_t)
     assert np.array_equal(U32(i2p), o_i)
     assert np.array_equal(F(keys).view(np.uint64), o_k)
+
+
+@pytest.mark.parametrize("n", [512, 513, 4095, 4097, 8192, 8193, 131072, 131073])
+def test_sort_forms(orc, dev, n):
+    """Around the limits between the sort in one block (512 and 1024 threads),
+    the one whose blocks sum the digit counts and the one that scans them;
+    equal depths, points without a tile and depths below -1 among them."""
+    rng = np.random.default_rng(n)
+    xyd = np.empty((n, 3), np.float32)
+    xyd[:, :2] = rng.uniform(-30, 130, (n, 2))
+    xyd[:, 2] = np.where(rng.random(n) < 0.5, rng.uniform(-1.2, 1.2, n), rng.integers(-4, 5, n) / 4.0)
+    half = rng.uniform(0, 3, (n, 2)).astype(np.float32)
+    aabb = np.concatenate([xyd[:, :2] - half, xyd[:, :2] + half], axis=1).astype(np.float32)
+    t2i, i2p, keys = cudarc.splat_gauss_tile2idx_idx2pnt(None, (100, 90), 16, T(xyd, dev), T(aabb, dev), with_keys=True)
+    o_t, o_i, o_k = orc.tile2pnt(xyd, aabb, 100, 90, 16)
+    assert np.array_equal(U32(t2i), o_t)
+    assert np.array_equal(U32(i2p), o_i)
+    assert np.array_equal(F(keys).view(np.uint64), o_k)
