@@ -20,10 +20,11 @@ __global__ void k_count_pairs(uint32_t, const float*, const float*, const float*
 __global__ void k_fused_project(uint32_t, uint32_t, int, const float*, const float*, const float*, const float*,
                                 const float*, const ViewBatch, float4*, uint2*, uint32_t*, uint32_t*);
 __global__ void k_project_bwd_geom(uint32_t, const float*, const float*, const float*, const ViewBatch,
-                                   float4*, float*, float*, float*, float*);
-__global__ void k_project_bwd_colour(uint32_t, int, const float*, const float*, const ViewBatch, float4*,
-                                     float*, float*, unsigned long long*, unsigned long long);
-__global__ void k_prepare_grad2d(const unsigned long long*, unsigned long long, float4*, size_t, uint32_t*);
+                                   float4*, const uint8_t*, float*, float*, float*, float*);
+cudaError_t project_bwd_colour(cudaStream_t, uint32_t, int, const float*, const float*, const ViewBatch&, float4*,
+                               uint8_t*, float*, float*, unsigned long long*, unsigned long long);
+__global__ void k_prepare_grad2d(const unsigned long long*, unsigned long long, float4*, size_t, uint32_t*, size_t,
+                                 uint32_t*);
 __global__ void k_adam(size_t, float*, const float*, float*, float*, float, float, float, float, float, float);
 __global__ void k_sb_count(const uint32_t*, const uint2*, uint32_t, uint32_t, const ViewBatch, uint32_t*,
                            unsigned long long*);
@@ -409,7 +410,8 @@ struct BatchWs {
   float* grad_pix;
   float* slab_loss;
   float4* grad2d;
-  unsigned long long* grad2d_tag;  // == grad2d_tag_value(): grad2d is all zero
+  unsigned long long* grad2d_tag;  // == grad2d_tag_value(): grad2d and touched are all zero
+  uint32_t* touched;  // a byte per grad2d record
   uint32_t *sched, *task_order, *item_cost;
 };
 
@@ -502,6 +504,7 @@ BatchWs carve_batch(void* ws, uint32_t n, const ViewBatch& b, uint64_t capacity)
   w.slab_loss = c.take<float>(size_t(b.num_items) * L.slabs_per_tile, &L.off_slab_loss);
   w.grad2d = c.take<float4>(3 * VN + 3, &L.off_grad2d);
   w.grad2d_tag = c.take<unsigned long long>(1);
+  w.touched = c.take<uint32_t>((VN + 3) / 4);
   w.task_order = c.take<uint32_t>(size_t(b.num_items) + 1);
   w.item_cost = c.take<uint32_t>(size_t(b.num_items) + 1);
   L.total_bytes = align_up(c.off, 256);
@@ -782,25 +785,25 @@ int dsplat_gauss_batch_backward(dsplat_stream stream, const dsplat_gauss_params*
   // consumes, so only a buffer not known to be clean is cleared here
   const unsigned long long tag = grad2d_tag_value(w.L, n, num_views);
   k_prepare_grad2d<<<blocks_for(3 * VN, 256) < 4096 ? blocks_for(3 * VN, 256) : 4096, 256, 0, st>>>(
-      w.grad2d_tag, tag, w.grad2d, 3 * VN, w.flags + 3);
+      w.grad2d_tag, tag, w.grad2d, 3 * VN, w.touched, (VN + 3) / 4, w.flags + 3);
   count_launch();
   // the forward's longest-first task order: it ranks the tasks by the walks
   // of the forward before it, the same measure as this forward's (equal once
   // the scene stops changing), and every order gives the same results
   stage_mark(st, 7);
   const BwdArgs ba{n,           w.rec,    w.lists.list1,  w.lists.off1, w.L.sb_chunks, pair_capacity,
-                   w.task_order, w.sched, w.flags + 3, grad_rgb ? grad_rgb : w.grad_pix, w.pix_T, w.pix_stop, w.grad2d};
+                   w.task_order, w.sched, w.flags + 3, grad_rgb ? grad_rgb : w.grad_pix, w.pix_T, w.pix_stop, w.grad2d,
+                   reinterpret_cast<uint8_t*>(w.touched)};
   TRY_CUDA(raster_bwd(st, b, ba),
            "raster_bwd");
   stage_mark(st, 8);
   k_project_bwd_geom<<<blocks_for(n, 128), 128, 0, st>>>(n, params->means, params->log_scales, params->quats, b,
-                                                         w.grad2d, grads->means, grads->log_scales, grads->quats,
+                                                         w.grad2d, ba.touched, grads->means, grads->log_scales, grads->quats,
                                                          grads->opacity);
   count_launch();
-  k_project_bwd_colour<<<blocks_for(n, 128), 128, 0, st>>>(n, params->sh_degree, params->means, params->colors, b,
-                                                           w.grad2d, grads->means, grads->colors, w.grad2d_tag,
-                                                           tag);
-  count_launch();
+  TRY_CUDA(project_bwd_colour(st, n, params->sh_degree, params->means, params->colors, b, w.grad2d, ba.touched,
+                              grads->means, grads->colors, w.grad2d_tag, tag),
+           "project_bwd_colour");
   stage_mark(st, 9);
   TRY_CUDA(cudaGetLastError(), "backward");
   return DSPLAT_OK;

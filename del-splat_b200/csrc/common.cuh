@@ -85,6 +85,7 @@ struct BwdArgs {
   const float* pix_T;
   const uint32_t* pix_last;
   float4* grad2d;
+  uint8_t* touched;  // [view][point]: grad2d's record got a gradient
 };
 
 

@@ -1,13 +1,24 @@
 // project_bwd.cu -- backward of the fused projection (no reference
 // counterpart; the reference has no gradient code).
 //
-// Two kernels, one thread per Gaussian each, looping over the views of the
-// batch with the next view's 2D gradient prefetched: k_project_bwd_geom
+// Two kernels, one thread per Gaussian each, looping over the views in which
+// the point got a gradient, the next one's record prefetched: k_project_bwd_geom
 // carries the geometry chain (mean through the projection, log-scale,
 // quaternion, opacity), k_project_bwd_colour the SH coefficients and the part
 // of the mean gradient that flows through the SH view direction.  The colour
 // kernel stages its block's coefficients through shared memory, so the
 // [N, K, 3] parameter rows are read and written with coalesced accesses.
+//
+// Bound: DRAM, and the latency of the records' loads.  Most points contribute
+// to few views (the entries behind the stop positions get no gradient), so
+// the backward raster marks the (view, point) records it adds to with a byte
+// and only those are read, cleared and worked on; a point without any is not
+// read or written at all.  Colour + geometry, us: 1,048,576 points in 16 views
+// 529 + 273 -> 313 + 212, 4,194,304 in 8 1411 + 659 -> 733 + 468, 262,144 in
+// one 70 + 27 -> 36 + 26; the marks cost the backward raster 55 of 3400 and 115
+// of 6700.  5 and 6 blocks per SM (registers 96 and 80) are the best caps:
+// colour at 3, 6 and 8 blocks 404, 361 and 435 (16 views), geometry at 4, 5
+// and 8 241, 218 and 222.
 // Both add into the caller's gradient buffers (so a per-view loop
 // accumulates naturally).
 //
@@ -170,14 +181,35 @@ __device__ __forceinline__ void geometry_view(const float* p, const float* dd, c
 
 }  // namespace
 
-__global__ void __launch_bounds__(128) k_project_bwd_geom(uint32_t n, const float* __restrict__ means,
+// Bit v: the backward raster added to the record of (view v, point g).
+__device__ __forceinline__ uint32_t touched_views(const uint8_t* __restrict__ touched, uint32_t n, int views,
+                                                  uint32_t g) {
+  uint32_t m = 0;
+#pragma unroll 8
+  for (int v = 0; v < views; ++v) m |= (touched[size_t(v) * n + g] ? 1u : 0u) << v;
+  return m;
+}
+
+__global__ void __launch_bounds__(128, 6) k_project_bwd_geom(uint32_t n, const float* __restrict__ means,
                                                           const float* __restrict__ log_scales,
                                                           const float* __restrict__ quats, const ViewBatch b,
                                                           float4* __restrict__ grad2d,
+                                                          const uint8_t* __restrict__ touched,
                                                           float* __restrict__ g_means, float* __restrict__ g_ls,
                                                           float* __restrict__ g_quats, float* __restrict__ g_op) {
+  // the lanes of a warp are at different views: their constants come from
+  // shared memory (odd row stride), not from the constant bank
+  __shared__ float views[DSPLAT_MAX_VIEWS][19];
+  for (int i = threadIdx.x; i < b.num_views * 18; i += 128) {
+    const ViewDev& d = b.v[i / 18];
+    const int j = i % 18;
+    views[i / 18][j] = j < 16 ? d.mvp[j] : j == 16 ? float(d.w) : float(d.h);
+  }
+  __syncthreads();
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= n) return;
+  uint32_t todo = touched_views(touched, n, b.num_views, g);
+  if (!todo) return;
   const float p[3] = {means[3 * g], means[3 * g + 1], means[3 * g + 2]};
   const float s[3] = {expf_cr(log_scales[3 * g]), expf_cr(log_scales[3 * g + 1]), expf_cr(log_scales[3 * g + 2])};
   const float dd[3] = {s[0] * s[0], s[1] * s[1], s[2] * s[2]};
@@ -200,24 +232,26 @@ __global__ void __launch_bounds__(128) k_project_bwd_geom(uint32_t n, const floa
   float acc[16];
 #pragma unroll
   for (int k = 0; k < 16; ++k) acc[k] = 0.f;
-  float4 n0 = grad2d[3 * size_t(g)];
-  float2 n1 = *reinterpret_cast<const float2*>(grad2d + 3 * size_t(g) + 1);
-  for (int v = 0; v < b.num_views; ++v) {
+  auto record = [&](int v) { return grad2d + 3 * (size_t(v) * n + g); };
+  int v = __ffs(todo) - 1;
+  float4 n0 = record(v)[0];
+  float2 n1 = *reinterpret_cast<const float2*>(record(v) + 1);
+  while (todo) {
     const float4 g0 = n0;
     const float2 g1 = n1;
-    if (v + 1 < b.num_views) {  // prefetch the next view's record
-      const float4* gp = grad2d + 3 * (size_t(v + 1) * n + g);
-      n0 = gp[0];
-      n1 = *reinterpret_cast<const float2*>(gp + 1);
+    float4* const gp = record(v);
+    const int view = v;
+    todo &= todo - 1u;
+    if (todo) {  // prefetch the next view's record
+      v = __ffs(todo) - 1;
+      n0 = record(v)[0];
+      n1 = *reinterpret_cast<const float2*>(record(v) + 1);
     }
-    if (g0.x == 0.f && g0.y == 0.f && g0.z == 0.f && g0.w == 0.f && g1.x == 0.f && g1.y == 0.f) continue;
-    {  // consumed: leave the record's geometry part zero for the next backward
-      float4* gp = grad2d + 3 * (size_t(v) * n + g);
-      gp[0] = make_float4(0.f, 0.f, 0.f, 0.f);
-      *reinterpret_cast<float2*>(gp + 1) = make_float2(0.f, 0.f);
-    }
+    // consumed: leave the record's geometry part zero for the next backward
+    gp[0] = make_float4(0.f, 0.f, 0.f, 0.f);
+    *reinterpret_cast<float2*>(gp + 1) = make_float2(0.f, 0.f);
     float c[16];
-    geometry_view(p, dd, R, b.v[v].mvp, float(b.v[v].w), float(b.v[v].h), g0, g1, c);
+    geometry_view(p, dd, R, views[view], views[view][16], views[view][17], g0, g1, c);
 #pragma unroll
     for (int k = 0; k < 16; ++k) acc[k] += c[k];
   }
@@ -258,117 +292,147 @@ __global__ void __launch_bounds__(128) k_project_bwd_geom(uint32_t n, const floa
 constexpr int kColThreads = 128;
 constexpr int kColStride = 49;  // 48 coefficients + 1 pad (odd stride: no bank conflicts)
 
-__global__ void __launch_bounds__(kColThreads) k_project_bwd_colour(uint32_t n, int sh_deg,
+template <int DEG>
+__global__ void __launch_bounds__(kColThreads, 5) k_project_bwd_colour(uint32_t n,
                                                                     const float* __restrict__ means,
                                                                     const float* __restrict__ colors,
                                                                     const ViewBatch b,
                                                                     float4* __restrict__ grad2d,
+                                                                    uint8_t* __restrict__ touched,
                                                                     float* __restrict__ g_means,
                                                                     float* __restrict__ g_col,
                                                                     unsigned long long* __restrict__ clean_tag,
                                                                     unsigned long long tag) {
+  constexpr int K = DEG < 0 ? 1 : (DEG + 1) * (DEG + 1), C = 3 * K;
   __shared__ float rows[kColThreads * kColStride];
-  const int K = sh_deg < 0 ? 1 : (sh_deg + 1) * (sh_deg + 1);
-  const int C = 3 * K;
+  __shared__ float eyes[DSPLAT_MAX_VIEWS][3];
+  for (int i = threadIdx.x; i < b.num_views * 3; i += kColThreads) eyes[i / 3][i % 3] = b.v[i / 3].campos[i % 3];
+  __syncthreads();
   const uint32_t g0 = blockIdx.x * kColThreads;
   const uint32_t cnt = min(uint32_t(kColThreads), n - g0);
-  for (uint32_t i = threadIdx.x; i < cnt * uint32_t(C); i += kColThreads)
-    rows[(i / C) * kColStride + (i % C)] = colors[size_t(g0) * C + i];
-  __syncthreads();
   const uint32_t g = g0 + threadIdx.x;
-  const bool live = threadIdx.x < cnt;
+  uint32_t todo = threadIdx.x < cnt ? touched_views(touched, n, b.num_views, g) : 0u;
+  // the rows of a warp's own 32 points, those with a gradient
+  const int lane = threadIdx.x & 31, row0 = threadIdx.x & ~31;
+  const uint32_t used = __ballot_sync(0xffffffffu, todo != 0u);
+#pragma unroll 8
+  for (int i = lane; i < 32 * C; i += 32) {
+    const int row = i / C;
+    if ((used >> row) & 1u) rows[(row0 + row) * kColStride + i % C] = colors[size_t(g0 + row0) * C + i];
+  }
+  __syncwarp();
+  const bool live = todo != 0u;
   const float* coef = rows + threadIdx.x * kColStride;  // coef[3k + c]
-  float gcol[48];
+  float gcol[C];
 #pragma unroll
-  for (int j = 0; j < 48; ++j) gcol[j] = 0.f;
+  for (int j = 0; j < C; ++j) gcol[j] = 0.f;
   if (live) {
     float* gflat = reinterpret_cast<float*>(grad2d);
     const float p[3] = {means[3 * g], means[3 * g + 1], means[3 * g + 2]};
     float gm[3] = {0.f, 0.f, 0.f};
-    const float* r0 = gflat + 12 * size_t(g) + 6;
-    float nd0 = r0[0], nd1 = r0[1], nd2 = r0[2];
-    for (int v = 0; v < b.num_views; ++v) {
+    auto record = [&](int v) { return gflat + 12 * (size_t(v) * n + g) + 6; };
+    int v = __ffs(todo) - 1;
+    float nd0 = record(v)[0], nd1 = record(v)[1], nd2 = record(v)[2];
+    while (todo) {
       const float dc[3] = {nd0, nd1, nd2};
-      if (v + 1 < b.num_views) {  // prefetch the next view's colour gradient
-        const float* r = gflat + 12 * (size_t(v + 1) * n + g) + 6;
-        nd0 = r[0];
-        nd1 = r[1];
-        nd2 = r[2];
+      const int view = v;
+      todo &= todo - 1u;
+      if (todo) {  // prefetch the next view's colour gradient
+        v = __ffs(todo) - 1;
+        nd0 = record(v)[0];
+        nd1 = record(v)[1];
+        nd2 = record(v)[2];
       }
-      if (dc[0] == 0.f && dc[1] == 0.f && dc[2] == 0.f) continue;
-      {  // consumed: leave the record's colour part zero for the next backward
-        float* r = gflat + 12 * (size_t(v) * n + g) + 6;
+      {  // consumed: leave the record's colour part and its mark zero for the next backward
+        float* r = record(view);
         r[0] = 0.f;
         r[1] = 0.f;
         r[2] = 0.f;
+        touched[size_t(view) * n + g] = 0;
       }
-      if (sh_deg < 0) {
+      if (dc[0] == 0.f && dc[1] == 0.f && dc[2] == 0.f) continue;
+      if (DEG < 0) {
         gcol[0] += dc[0];
         gcol[1] += dc[1];
         gcol[2] += dc[2];
         continue;
       }
-      const ViewDev& vd = b.v[v];
-      const float d0 = p[0] - vd.campos[0], d1 = p[1] - vd.campos[1], d2 = p[2] - vd.campos[2];
+      const float d0 = p[0] - eyes[view][0], d1 = p[1] - eyes[view][1], d2 = p[2] - eyes[view][2];
       const float dn = sqrtf(d0 * d0 + d1 * d1 + d2 * d2);
       const float x = d0 / dn, y = d1 / dn, z = d2 / dn;
       float bs[16];
-      sh_basis(sh_deg, x, y, z, bs);
+      sh_basis(DEG, x, y, z, bs);
       float draw[3];
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         float col = 0.f;
 #pragma unroll
-        for (int k = 0; k < 16; ++k)
-          if (k < K) col += bs[k] * coef[3 * k + c];
+        for (int k = 0; k < K; ++k) col += bs[k] * coef[3 * k + c];
         draw[c] = col + 0.5f > 0.f ? dc[c] : 0.f;
       }
-      float w[16];  // w_k = sum_c coef_kc draw_c
+      float w[16] = {};  // w_k = sum_c coef_kc draw_c
 #pragma unroll
-      for (int k = 0; k < 16; ++k) {
-        w[k] = 0.f;
-        if (k < K) {
+      for (int k = 0; k < K; ++k)
 #pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            gcol[3 * k + c] += bs[k] * draw[c];
-            w[k] += coef[3 * k + c] * draw[c];
-          }
+        for (int c = 0; c < 3; ++c) {
+          gcol[3 * k + c] += bs[k] * draw[c];
+          w[k] += coef[3 * k + c] * draw[c];
         }
-      }
       float dv[3];
-      sh_weighted_grad(sh_deg, x, y, z, w, dv);
+      sh_weighted_grad(DEG, x, y, z, w, dv);
       const float dot = dv[0] * x + dv[1] * y + dv[2] * z;
       gm[0] += (dv[0] - x * dot) / dn;
       gm[1] += (dv[1] - y * dot) / dn;
       gm[2] += (dv[2] - z * dot) / dn;
     }
-    if (sh_deg >= 0) {
+    if (DEG >= 0) {
 #pragma unroll
       for (int c = 0; c < 3; ++c) g_means[3 * g + c] += gm[c];
     }
   }
-  __syncthreads();
+  __syncwarp();
   float* mine = rows + threadIdx.x * kColStride;
+  if (live) {
 #pragma unroll
-  for (int j = 0; j < 48; ++j)
-    if (j < C) mine[j] = gcol[j];
-  __syncthreads();
-  for (uint32_t i = threadIdx.x; i < cnt * uint32_t(C); i += kColThreads)
-    g_col[size_t(g0) * C + i] += rows[(i / C) * kColStride + (i % C)];
-  // after this kernel and k_project_bwd_geom every record is zero again
+    for (int j = 0; j < C; ++j) mine[j] = gcol[j];
+  }
+  __syncwarp();
+#pragma unroll 8
+  for (int i = lane; i < 32 * C; i += 32) {
+    const int row = i / C;
+    if ((used >> row) & 1u) g_col[size_t(g0 + row0) * C + i] += rows[(row0 + row) * kColStride + i % C];
+  }
+  // after this kernel and k_project_bwd_geom every record and mark is zero again
   if (blockIdx.x == 0 && threadIdx.x == 0) *clean_tag = tag;
 }
 
-// Clears grad2d unless the tag says it is already all zero (the previous
-// backward on this layout consumed it).  Blocks only read the tag; the
+cudaError_t project_bwd_colour(cudaStream_t st, uint32_t n, int sh_deg, const float* means, const float* colors,
+                               const ViewBatch& b, float4* grad2d, uint8_t* touched, float* g_means, float* g_col,
+                               unsigned long long* clean_tag, unsigned long long tag) {
+  const unsigned grid = (n + kColThreads - 1) / kColThreads;
+#define X(DEG)                                                                                                \
+  if (sh_deg == DEG)                                                                                          \
+    k_project_bwd_colour<DEG><<<grid, kColThreads, 0, st>>>(n, means, colors, b, grad2d, touched, g_means, g_col, \
+                                                            clean_tag, tag);
+  X(-1) X(0) X(1) X(2) X(3)
+#undef X
+  count_launch();
+  return cudaGetLastError();
+}
+
+// Clears grad2d and its marks unless the tag says they are already all zero
+// (the previous backward on this layout consumed them).  Blocks only read the tag; the
 // colour kernel of the same backward writes it.  Also sets the backward
 // raster's work counter to zero.
 __global__ void k_prepare_grad2d(const unsigned long long* __restrict__ clean_tag, unsigned long long tag,
-                                 float4* __restrict__ grad2d, size_t count, uint32_t* __restrict__ work_counter) {
+                                 float4* __restrict__ grad2d, size_t count, uint32_t* __restrict__ touched,
+                                 size_t touched_words, uint32_t* __restrict__ work_counter) {
   if (blockIdx.x == 0 && threadIdx.x == 0) *work_counter = 0u;
   if (*clean_tag == tag) return;
   for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += size_t(gridDim.x) * blockDim.x)
     grad2d[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < touched_words; i += size_t(gridDim.x) * blockDim.x)
+    touched[i] = 0u;
 }
 
 // Adam (Kingma & Ba 2015), bias-corrected, in place: config-4 training step.

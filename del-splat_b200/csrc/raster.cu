@@ -31,7 +31,10 @@ struct __align__(16) RedBuf {
   float row[kRedEntries][9][36];
 };
 
-__device__ __forceinline__ void red_flush(const RedBuf* red, int held, int lane, float* __restrict__ gv) {
+// base: the view's first record; touched: the marks of those that got a
+// gradient.
+__device__ __forceinline__ void red_flush(const RedBuf* red, int held, int lane, size_t base,
+                                          float4* __restrict__ grad2d, uint8_t* __restrict__ touched) {
   __syncwarp();
   const int slot = lane >> 3, k = lane & 7;
   const ulonglong2* r = reinterpret_cast<const ulonglong2*>(red->row[slot][k]);
@@ -63,9 +66,12 @@ __device__ __forceinline__ void red_flush(const RedBuf* red, int held, int lane,
   if (k < 5) out *= 0.5f * c.w;  // the moments of t become moments of w = dL/dq (c.w = -opacity)
   if (k > 5) out = -out;
   if (slot < held) {
-    float* dst = gv + 12 * size_t(g);
+    float* dst = reinterpret_cast<float*>(grad2d) + 12 * (base + g);
     atomicAdd(dst + k, out);
-    if (k == 0) atomicAdd(dst + 8, -gb);
+    if (k == 0) {
+      atomicAdd(dst + 8, -gb);
+      touched[base + g] = 1;
+    }
   }
   __syncwarp();
 }
@@ -93,7 +99,8 @@ template <class GEO>
 __device__ __forceinline__ void bwd_task(const SbWalkSpan& walk, const PackedSrc& src, Ent* sm, RedBuf* red,
                                          const ViewDev& vd, uint32_t s, uint32_t e, int px0, int py0, int xend,
                                          const float* __restrict__ grad_pix, const float* __restrict__ pix_T,
-                                         const uint32_t* __restrict__ pix_last, float* __restrict__ gv) {
+                                         const uint32_t* __restrict__ pix_last, size_t base,
+                                         float4* __restrict__ grad2d, uint8_t* __restrict__ touched) {
   constexpr int PPL = GEO::PPL, NP = PPL / 2;
   static_assert(PPL % 2 == 0, "pixels are evaluated in pairs");
   const int lane = threadIdx.x & 31;
@@ -220,14 +227,14 @@ __device__ __forceinline__ void bwd_task(const SbWalkSpan& walk, const PackedSrc
         *reinterpret_cast<float4*>(&red->row[held][0][32]) = make_float4(ed.y, ed.z, sm[j].a.z, sm[j].b.x);
         red->row[held][1][32] = ed.w;
         if (++held == kRedEntries) {
-          red_flush(red, held, lane, gv);
+          red_flush(red, held, lane, base, grad2d, touched);
           held = 0;
         }
       }
     }
     __syncwarp();
   }
-  if (held) red_flush(red, held, lane, gv);
+  if (held) red_flush(red, held, lane, base, grad2d, touched);
 }
 
 template <int TS, int PPL_, int NT>
@@ -235,7 +242,8 @@ __global__ void __launch_bounds__(32 * kRasterWarps, NT * PPL_ <= 4 ? 6 : 4) k_r
     const ViewBatch b, uint32_t n, const float4* __restrict__ rec, const uint2* __restrict__ list1,
     const uint32_t* __restrict__ off1, uint32_t nchunk, uint64_t capacity, const uint32_t* __restrict__ order,
     const uint32_t* __restrict__ sched, uint32_t* __restrict__ work_counter, const float* __restrict__ grad_pix,
-    const float* __restrict__ pix_T, const uint32_t* __restrict__ pix_last, float4* __restrict__ grad2d) {
+    const float* __restrict__ pix_T, const uint32_t* __restrict__ pix_last, float4* __restrict__ grad2d,
+    uint8_t* __restrict__ touched) {
   using G = TaskGeo<TS, PPL_, NT>;
   __shared__ Ent sm_all[kRasterWarps][32];
   __shared__ RedBuf red_all[kRasterWarps];
@@ -257,15 +265,15 @@ __global__ void __launch_bounds__(32 * kRasterWarps, NT * PPL_ <= 4 ? 6 : 4) k_r
       if (ig.lx % nx) continue;
     }
     const PackedSrc src{rec + 3 * size_t(ig.v) * n};
-    float* const gv = reinterpret_cast<float*>(grad2d + 3 * size_t(ig.v) * n);
+    const size_t base = size_t(ig.v) * n;
     if (t.block) {
       BlockPlace p;
       if (!block_place(b, ig, t.sub, nx, &p)) continue;
       bwd_task<BlockGeo>(SbWalkSpan{list1, p.lx, ig.ly, 1u}, src, sm, red, vd, ig.s, ig.e, p.px0, p.py0, vd.w, grad_pix,
-                         pix_T, pix_last, gv);
+                         pix_T, pix_last, base, grad2d, touched);
     } else {
       bwd_task<G>(SbWalkSpan{list1, ig.lx, ig.ly, nx}, src, sm, red, vd, ig.s, ig.e, ig.px0,
-                  ig.py0 + int(t.sub) * G::SLAB_ROWS, min(vd.w, ig.px0 + int(nx) * TS), grad_pix, pix_T, pix_last, gv);
+                  ig.py0 + int(t.sub) * G::SLAB_ROWS, min(vd.w, ig.px0 + int(nx) * TS), grad_pix, pix_T, pix_last, base, grad2d, touched);
     }
   }
 }
@@ -329,7 +337,7 @@ static cudaError_t launch_bwd(cudaStream_t st, const ViewBatch& b, const BwdArgs
   k_raster_bwd<TS, PPL, NT>
       <<<persistent_grid(k_raster_bwd<TS, PPL, NT>, max_tasks(b, TaskGeo<TS, PPL, NT>::SLABS)), 32 * kRasterWarps, 0,
          st>>>(b, a.n, a.rec, a.list1, a.off1, a.nchunk, a.capacity, a.order, a.sched, a.counter, a.grad_pix, a.pix_T,
-               a.pix_last, a.grad2d);
+               a.pix_last, a.grad2d, a.touched);
   count_launch();
   return cudaGetLastError();
 }
