@@ -30,9 +30,9 @@ __global__ void k_sb_count(const uint32_t*, const uint2*, uint32_t, uint32_t, co
                            unsigned long long*);
 __global__ void k_sb_scatter(const uint32_t*, const uint2*, uint32_t, uint32_t, const ViewBatch, const uint32_t*,
                              uint64_t, uint2*, uint32_t*);
-__global__ void k_sb_scatter_staged(const uint32_t*, const uint2*, uint32_t, uint32_t, const ViewBatch, const uint32_t*,
-                                    uint64_t, uint2*, uint32_t*, uint32_t);
-size_t sb_scatter_staged_smem(uint32_t max_sb, uint32_t max_side, uint32_t qcap);
+cudaError_t sb_scatter_staged(cudaStream_t, unsigned, const uint32_t*, const uint2*, uint32_t, uint32_t, const ViewBatch&,
+                              const uint32_t*, uint64_t, uint2*, uint32_t*);
+size_t sb_scatter_staged_smem(uint32_t max_sb);
 size_t tile_seg_slots(uint64_t capacity, uint32_t num_sb);
 cudaError_t split_tile_lists(cudaStream_t, const uint2*, const uint32_t*, uint32_t, uint64_t, const ViewBatch&,
                              uint32_t*, uint32_t*);
@@ -185,19 +185,13 @@ int build_sb_lists(cudaStream_t st, const ViewBatch& b, uint32_t n, uint32_t npa
   count_launch();
   TRY_CUDA(exclusive_scan(st, L.cnt1, L.off1, m, scan_tmp, 0xffffffffu, nullptr), "scan");
   // staged scatter (coalesced list stores) when its shared memory fits
-  constexpr uint32_t kStageEntries = 3072;
-  const size_t smem_staged = sb_scatter_staged_smem(b.max_sb, b.max_sb_side, kStageEntries);
-  if (smem_staged <= 100 * 1024) {
-    if (smem_staged > 48 * 1024)
-      TRY_CUDA(cudaFuncSetAttribute(k_sb_scatter_staged, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    int(smem_staged)),
-               "attr");
-    k_sb_scatter_staged<<<grid1, 256, smem_staged, st>>>(order, srect, npad / nchunk, npad, b, L.off1, capacity, L.list1, flags,
-                                                         kStageEntries);
+  if (sb_scatter_staged_smem(b.max_sb) <= 100 * 1024) {
+    TRY_CUDA(sb_scatter_staged(st, grid1, order, srect, npad / nchunk, npad, b, L.off1, capacity, L.list1, flags),
+             "superblock scatter");
   } else {
     k_sb_scatter<<<grid1, 256, smem3, st>>>(order, srect, npad / nchunk, npad, b, L.off1, capacity, L.list1, flags);
+    count_launch();
   }
-  count_launch();
   TRY_CUDA(cudaGetLastError(), "superblock lists");
   return DSPLAT_OK;
 }

@@ -613,144 +613,194 @@ __global__ void __launch_bounds__(kMsThreads) k_sb_scatter(const uint32_t* __res
 }
 
 // ---------------------------------------------------------------------------
-// Stage 1b, staged: the same result as k_sb_scatter with coalesced stores.
-// The chunk is processed in sub-passes of kSubRanks consecutive ranks (each
-// warp takes kSubRanks / 8 consecutive ranks of the sub-pass).  A sub-pass's
-// entries are ranked per superblock (per-warp counts, one block-wide scan)
-// into a shared-memory stage ordered by superblock, then each superblock's
-// run is written to its contiguous range of the superblock list (the block's
-// cursor for that superblock advances sub-pass by sub-pass).  A sub-pass
-// with more entries than the stage holds writes the same slots directly.
-// Shared memory (words): counters [8][max_sb], cursors [max_sb], stage
-// bases [max_sb + 2] (one spare word keeps the stage 8-byte aligned), masks
-// [8][2 * max_sb_side] (superblock columns, then rows), then the stage
-// (uint2[qcap]) and its superblock ids (u16[qcap]).
+// Stage 1b, staged: the same result as k_sb_scatter with coalesced stores and
+// its work spread over entries instead of ranks.  The chunk is taken in
+// sub-passes of kSubRanks consecutive ranks, a sub-pass in pieces of at most
+// kPiece entries:
+//   expand   every rank writes its superblocks, in order, to its place in the
+//            piece (ranks and places from a block-wide scan of the counts);
+//   rank     warp w takes an eighth of the piece's entries, 32 at a time: the
+//            lanes of the same superblock come from one ballot per bit of its
+//            number, earlier rounds from the warp's counters;
+//   bases    one block-wide scan over the view's superblocks;
+//   stage    the entries in superblock order in shared memory;
+//   store    each superblock's run to its contiguous range of the list (the
+//            block's cursor for it advances piece by piece).
+// Bound: the latency between its barriers, at 3 blocks per SM (4, by fewer
+// registers, were slower).  us, against every lane looping over its own rank's
+// span with coverage masks: 16 views of 1,048,576 points 816 -> 762, 8 of
+// 4,194,304 1800 -> 1650, one 76 -> 68, one of 16,384 17 -> 13.  Unrolling the
+// ballots, match.any and ranking all rounds before counting were slower (822,
+// 861, 868).
+// Shared memory: see SbScatterShared.
 // ---------------------------------------------------------------------------
-constexpr int kSubRounds = 2;
-constexpr int kSubRanks = kMsThreads * kSubRounds;  // 512 ranks per sub-pass
+constexpr int kSubRanks = 2 * kMsThreads;  // 512 ranks per sub-pass, two per thread
+constexpr int kPieceRounds = 12;
+constexpr uint32_t kPiece = kMsThreads * kPieceRounds;  // 3072 entries
 
-size_t sb_scatter_staged_smem(uint32_t max_sb, uint32_t max_side, uint32_t qcap) {
-  return (size_t(kMsWarps) * max_sb + 2 * size_t(max_sb) + 2 + size_t(kMsWarps) * 2 * max_side) * 4 +
-         size_t(qcap) * 8 +
-         ((size_t(qcap) + 1) / 2) * 4;
+struct SbScatterShared {
+  uint2 stage[kPiece];         // the piece's entries in superblock order
+  union {
+    uint32_t ent[kPiece];      // superblock x | y << 8 | rank of the sub-pass << 16, in list order
+    uint16_t stage_sb[kPiece];
+  };
+  uint2 rect[kSubRanks];       // the sub-pass's spans
+  uint32_t point[kSubRanks];   // and points
+  uint32_t first[kSubRanks + 1];  // and first entries
+  uint32_t total;
+  // then uint32_t cur[max_sb], sbase[max_sb + 1], uint16_t wc[kMsWarps][max_sb]
+};
+
+size_t sb_scatter_staged_smem(uint32_t max_sb) {
+  return sizeof(SbScatterShared) + (2 * size_t(max_sb) + 1) * 4 + size_t(kMsWarps) * max_sb * 2;
 }
 
-__global__ void __launch_bounds__(kMsThreads) k_sb_scatter_staged(const uint32_t* __restrict__ order,
+__global__ void __launch_bounds__(kMsThreads, 3) k_sb_scatter_staged(const uint32_t* __restrict__ order,
                                                                   const uint2* __restrict__ srect, uint32_t chunk,
                                                                   uint32_t npad, const ViewBatch b,
                                                                   const uint32_t* __restrict__ off, uint64_t capacity,
                                                                   uint2* __restrict__ list1,
-                                                                  uint32_t* __restrict__ flags, uint32_t qcap) {
+                                                                  uint32_t* __restrict__ flags) {
   check_capacity(capacity, flags);
-  extern __shared__ uint32_t smem_ms[];
-  __shared__ uint32_t sub_total;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  SbScatterShared& sh = *reinterpret_cast<SbScatterShared*>(smem_raw);
   const uint32_t nchunk = npad / chunk;
   const uint32_t v = blockIdx.x / nchunk, c = blockIdx.x % nchunk;
   const ViewDev& vd = b.v[v];
-  const int sl = vd.sb_log2, sbw = sb_cols(vd), sbh = sb_rows(vd);
-  const int nsb = sbw * sbh;
+  const int sl = vd.sb_log2, sbw = sb_cols(vd), nsb = sbw * sb_rows(vd);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t lt = (1u << lane) - 1u;
-  const uint32_t M = b.max_sb;
-  uint32_t* wc = smem_ms;                     // [kMsWarps][nsb]
-  uint32_t* cur = wc + kMsWarps * M;          // [nsb]
-  uint32_t* sbase = cur + M;                  // [nsb + 1]
-  const uint32_t side = b.max_sb_side;
-  uint32_t* colmask = sbase + M + 2 + warp * 2 * side;
-  uint32_t* rowmask = colmask + side;
-  uint2* stage = reinterpret_cast<uint2*>(sbase + M + 2 + kMsWarps * 2 * side);  // 10 M + 2 + 16 side words: 8-byte aligned
-  uint16_t* stage_sb = reinterpret_cast<uint16_t*>(stage + qcap);
-  uint32_t* my = wc + warp * nsb;
-  const uint32_t sb0 = vd.sb_base;
-  for (int i = threadIdx.x; i < nsb; i += kMsThreads) cur[i] = off[(size_t(sb0) + i) * nchunk + c];
+  uint32_t* const cur = reinterpret_cast<uint32_t*>(smem_raw + sizeof(SbScatterShared));
+  uint32_t* const sbase = cur + b.max_sb;
+  uint16_t* const wc = reinterpret_cast<uint16_t*>(sbase + b.max_sb + 1);
+  uint16_t* const my = wc + warp * nsb;
+  int bits = 1;  // of a superblock's number
+  while ((1 << bits) < nsb) ++bits;
+  for (int i = threadIdx.x; i < nsb; i += kMsThreads) cur[i] = off[(size_t(vd.sb_base) + i) * nchunk + c];
   const int seg = (nsb + kMsThreads - 1) / kMsThreads;
   const int s_lo = min(nsb, int(threadIdx.x) * seg), s_hi = min(nsb, s_lo + seg);
   for (uint32_t sub = 0; sub < chunk / kSubRanks; ++sub) {
-    for (int i = threadIdx.x; i < kMsWarps * nsb; i += kMsThreads) wc[i] = 0;
-    __syncthreads();
-    const size_t base = size_t(v) * npad + size_t(c) * chunk + size_t(sub) * kSubRanks +
-                        size_t(warp) * (kSubRounds * 32);
-    // per-warp counts of the sub-pass
-    for (int r = 0; r < kSubRounds; ++r) {
-      int sx0, sy0, sx1, sy1;
-      if (sb_span(srect[base + r * 32 + lane], sl, &sx0, &sy0, &sx1, &sy1))
-        for (int sy = sy0; sy < sy1; ++sy)
-          for (int sx = sx0; sx < sx1; ++sx) atomicAdd(&my[sy * sbw + sx], 1u);
-    }
-    __syncthreads();
-    // stage layout: superblock-major, then warp (= rank order)
-    uint32_t loc = 0;
-    for (int sb = s_lo; sb < s_hi; ++sb)
+    const size_t base = size_t(v) * npad + size_t(c) * chunk + size_t(sub) * kSubRanks + 2 * threadIdx.x;
+    // this thread's two ranks
+    const uint4 rr = *reinterpret_cast<const uint4*>(srect + base);
+    const uint2 pp = *reinterpret_cast<const uint2*>(order + base);
+    const uint2 rc[2] = {make_uint2(rr.x, rr.y), make_uint2(rr.z, rr.w)};
+    int sx0[2], sy0[2], sx1[2], sy1[2];
+    uint32_t count[2];
 #pragma unroll
-      for (int w = 0; w < kMsWarps; ++w) loc += wc[w * nsb + sb];
-    uint32_t run = block_excl_scan(loc, &sub_total);
-    for (int sb = s_lo; sb < s_hi; ++sb) {
-      sbase[sb] = run;
-#pragma unroll
-      for (int w = 0; w < kMsWarps; ++w) {
-        const uint32_t t = wc[w * nsb + sb];
-        wc[w * nsb + sb] = run;
-        run += t;
-      }
-    }
-    if (threadIdx.x == 0) sbase[nsb] = sub_total;
+    for (int k = 0; k < 2; ++k)
+      count[k] = sb_span(rc[k], sl, &sx0[k], &sy0[k], &sx1[k], &sy1[k])
+                     ? uint32_t(sx1[k] - sx0[k]) * uint32_t(sy1[k] - sy0[k]) : 0u;
+    const uint32_t first = block_excl_scan(count[0] + count[1], &sh.total);
+    *reinterpret_cast<uint4*>(&sh.rect[2 * threadIdx.x]) = rr;
+    *reinterpret_cast<uint2*>(&sh.point[2 * threadIdx.x]) = pp;
+    sh.first[2 * threadIdx.x] = first;
+    sh.first[2 * threadIdx.x + 1] = first + count[0];
+    if (threadIdx.x == 0) sh.first[kSubRanks] = sh.total;
     __syncthreads();
-    const uint32_t total = sub_total;
-    const bool staged = total <= qcap;
-    for (int r = 0; r < kSubRounds; ++r) {
-      const uint32_t g = order[base + r * 32 + lane];
-      int sx0 = 0, sy0 = 0, sx1 = 0, sy1 = 0;
-      const uint2 rc = srect[base + r * 32 + lane];
-      const bool has = sb_span(rc, sl, &sx0, &sy0, &sx1, &sy1);
-      if (has) {
-        for (int x = sx0; x < sx1; ++x) colmask[x] = 0u;
-        for (int y = sy0; y < sy1; ++y) rowmask[y] = 0u;
+    const uint32_t total = sh.total;
+    // pieces of whole ranks: a rank has at most nsb <= kPiece entries
+    for (uint32_t r0 = 0, e0 = 0; e0 < total;) {
+      uint32_t r1 = kSubRanks, e1 = total;
+      if (total - e0 > kPiece) {  // the last rank that still fits, the same search in every thread
+        uint32_t lo = r0 + 1, hi = kSubRanks;
+        while (lo < hi) {
+          const uint32_t mid = (lo + hi + 1) / 2;
+          if (sh.first[mid] - e0 <= kPiece) lo = mid;
+          else hi = mid - 1;
+        }
+        r1 = lo;
+        e1 = sh.first[r1];
       }
-      __syncwarp();
-      if (has) {
-        for (int x = sx0; x < sx1; ++x) atomicOr(&colmask[x], 1u << lane);
-        for (int y = sy0; y < sy1; ++y) atomicOr(&rowmask[y], 1u << lane);
+      for (int i = threadIdx.x; i < (kMsWarps * nsb + 1) / 2; i += kMsThreads) reinterpret_cast<uint32_t*>(wc)[i] = 0;
+      uint32_t at = first - e0;
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const uint32_t rank = 2 * threadIdx.x + k;
+        if (count[k] && rank >= r0 && rank < r1) {
+          uint32_t o = at;
+          for (int sy = sy0[k]; sy < sy1[k]; ++sy)
+            for (int sx = sx0[k]; sx < sx1[k]; ++sx) sh.ent[o++] = uint32_t(sx) | uint32_t(sy) << 8 | rank << 16;
+        }
+        at += count[k];
       }
-      __syncwarp();
-      for (int sy = sy0; sy < sy1; ++sy) {
-        const uint32_t rm = rowmask[sy];
-        for (int sx = sx0; sx < sx1; ++sx) {
-          const int sb = sy * sbw + sx;
-          const uint32_t sp = my[sb] + uint32_t(__popc(colmask[sx] & rm & lt));
-          const uint2 en = make_uint2(g, local_rect(rc, sl, sx, sy));
-          if (staged) {
-            stage[sp] = en;
-            stage_sb[sp] = uint16_t(sb);
-          } else {
-            const uint64_t dst = uint64_t(cur[sb]) + (sp - sbase[sb]);
-            if (dst < capacity) list1[dst] = en;
-            else set_flag(flags, kFlagPairOverflow);
-          }
+      __syncthreads();
+      const uint32_t n_piece = e1 - e0, rounds = (n_piece + kMsThreads - 1) / kMsThreads;
+      const uint32_t i0 = uint32_t(warp) * rounds * 32 + lane;
+      uint32_t e[kPieceRounds], place[kPieceRounds];  // place: superblock << 16 | rank among the warp's of it
+#pragma unroll
+      for (int r = 0; r < kPieceRounds; ++r) {
+        if (uint32_t(r) >= rounds) break;
+        const bool in = i0 + 32 * r < n_piece;
+        e[r] = in ? sh.ent[i0 + 32 * r] : 0u;
+        const uint32_t sb = in ? ((e[r] >> 8) & 255u) * uint32_t(sbw) + (e[r] & 255u) : 0u;
+        uint32_t peers = __ballot_sync(0xffffffffu, in);
+        for (int bit = 0; bit < bits; ++bit) {
+          const uint32_t m = __ballot_sync(0xffffffffu, (sb >> bit) & 1u);
+          peers &= ((sb >> bit) & 1u) ? m : ~m;
+        }
+        uint32_t before = 0;
+        if (in) before = my[sb];
+        __syncwarp();
+        if (in && lane == __ffs(peers) - 1) my[sb] = uint16_t(before + __popc(peers));
+        __syncwarp();
+        place[r] = sb << 16 | (before + __popc(peers & lt));
+      }
+      __syncthreads();
+      // stage layout: superblock-major, then warp (= list order)
+      uint32_t loc = 0;
+      for (int sb = s_lo; sb < s_hi; ++sb)
+#pragma unroll
+        for (int w = 0; w < kMsWarps; ++w) loc += wc[w * nsb + sb];
+      uint32_t run = block_excl_scan(loc, &sh.total);
+      for (int sb = s_lo; sb < s_hi; ++sb) {
+        sbase[sb] = run;
+#pragma unroll
+        for (int w = 0; w < kMsWarps; ++w) {
+          const uint32_t t = wc[w * nsb + sb];
+          wc[w * nsb + sb] = uint16_t(run);
+          run += t;
         }
       }
-      __syncwarp();
-      for (int sy = sy0; sy < sy1; ++sy) {
-        const uint32_t rm = rowmask[sy];
-        for (int sx = sx0; sx < sx1; ++sx) {
-          const uint32_t m = colmask[sx] & rm;
-          if ((m >> lane) == 1u) my[sy * sbw + sx] += uint32_t(__popc(m));
+      if (threadIdx.x == 0) sbase[nsb] = n_piece;
+      __syncthreads();
+#pragma unroll
+      for (int r = 0; r < kPieceRounds; ++r) {
+        if (uint32_t(r) >= rounds) break;
+        if (i0 + 32 * r < n_piece) {
+          const uint32_t sb = place[r] >> 16, rank = e[r] >> 16, pos = my[sb] + (place[r] & 0xffffu);
+          sh.stage[pos] = make_uint2(sh.point[rank], local_rect(sh.rect[rank], sl, int(e[r] & 255u),
+                                                                int((e[r] >> 8) & 255u)));
+          sh.stage_sb[pos] = uint16_t(sb);
         }
       }
-      __syncwarp();
-    }
-    __syncthreads();
-    if (staged) {
-      for (uint32_t i = threadIdx.x; i < total; i += kMsThreads) {
-        const int sb = stage_sb[i];
+      __syncthreads();
+      for (uint32_t i = threadIdx.x; i < n_piece; i += kMsThreads) {
+        const int sb = sh.stage_sb[i];
         const uint64_t dst = uint64_t(cur[sb]) + (i - sbase[sb]);
-        if (dst < capacity) list1[dst] = stage[i];
+        if (dst < capacity) list1[dst] = sh.stage[i];
         else set_flag(flags, kFlagPairOverflow);
       }
+      __syncthreads();
+      for (int sb = threadIdx.x; sb < nsb; sb += kMsThreads) cur[sb] += sbase[sb + 1] - sbase[sb];
+      r0 = r1;
+      e0 = e1;
+      __syncthreads();
     }
-    __syncthreads();
-    for (int sb = threadIdx.x; sb < nsb; sb += kMsThreads) cur[sb] += sbase[sb + 1] - sbase[sb];
-    __syncthreads();
   }
+}
+
+cudaError_t sb_scatter_staged(cudaStream_t st, unsigned grid, const uint32_t* order, const uint2* srect, uint32_t chunk,
+                              uint32_t npad, const ViewBatch& b, const uint32_t* off, uint64_t capacity, uint2* list1,
+                              uint32_t* flags) {
+  const size_t smem = sb_scatter_staged_smem(b.max_sb);
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(k_sb_scatter_staged, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    if (e != cudaSuccess) return e;
+  }
+  k_sb_scatter_staged<<<grid, kMsThreads, smem, st>>>(order, srect, chunk, npad, b, off, capacity, list1, flags);
+  count_launch();
+  return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------------------
