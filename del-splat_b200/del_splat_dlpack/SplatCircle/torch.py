@@ -25,12 +25,12 @@ def from_project_spheres(
     from .. import SplatCircle
 
     SplatCircle.from_project_spheres(
-        util_torch.to_dlpack_safe(pnt2xyz, stream_ptr),
+        util_torch.to_kernel(pnt2xyz, stream_ptr),
         radius,
-        util_torch.to_dlpack_safe(transform_world2ndc, stream_ptr),
+        util_torch.to_kernel(transform_world2ndc, stream_ptr),
         img_shape,
-        util_torch.to_dlpack_safe(pnt2pixxyndcz, stream_ptr),
-        util_torch.to_dlpack_safe(pnt2pixrad, stream_ptr),
+        util_torch.to_kernel(pnt2pixxyndcz, stream_ptr),
+        util_torch.to_kernel(pnt2pixrad, stream_ptr),
         stream_ptr)
     return pnt2pixxyndcz, pnt2pixrad
 

@@ -25,9 +25,9 @@ def rasterize_pix(
     from .. import SplatPoint
 
     SplatPoint.rasterize_pix(
-        util_torch.to_dlpack_safe(pnt2pixxyndcz, stream_ptr),
-        util_torch.to_dlpack_safe(pnt2rgb, stream_ptr),
-        util_torch.to_dlpack_safe(pix2rgb, stream_ptr),
+        util_torch.to_kernel(pnt2pixxyndcz, stream_ptr),
+        util_torch.to_kernel(pnt2rgb, stream_ptr),
+        util_torch.to_kernel(pix2rgb, stream_ptr),
         stream_ptr)
     return pix2rgb
 
@@ -48,9 +48,9 @@ def rasterize_pix_zbuffer(
     from .. import SplatPoint
 
     SplatPoint.rasterize_pix_zbuffer(
-        util_torch.to_dlpack_safe(pnt2pixxyndcz, stream_ptr),
-        util_torch.to_dlpack_safe(pnt2rgb, stream_ptr),
-        util_torch.to_dlpack_safe(pix2rgb, stream_ptr),
-        util_torch.to_dlpack_safe(pix2unitdepth, stream_ptr),
+        util_torch.to_kernel(pnt2pixxyndcz, stream_ptr),
+        util_torch.to_kernel(pnt2rgb, stream_ptr),
+        util_torch.to_kernel(pix2rgb, stream_ptr),
+        util_torch.to_kernel(pix2unitdepth, stream_ptr),
         stream_ptr)
     return pix2rgb
