@@ -21,6 +21,8 @@
 // Filtering a rank-ordered superblock list by tile keeps rank order, so every
 // tile list is the reference's order, (tile, depth bits, point index)
 // ascending, bit for bit; no 64-bit pair key is sorted.
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace dsplat {
@@ -143,32 +145,43 @@ cudaError_t exclusive_scan(cudaStream_t st, const uint32_t* in, uint32_t* out, s
 
 // ---------------------------------------------------------------------------
 // Stable LSD radix sort of (u32 key, u32 value), 8-bit digits.
-// Each block owns a tile of 4096 consecutive elements.  Segmented form: with
-// nb_seg blocks per segment the histogram is laid out (segment, digit, block)
-// so that one exclusive scan yields every block's output offset per digit and
-// segments never mix.
+// Each block owns a tile of 4096 consecutive elements, or of 2048.  Segmented
+// form: with nb_seg blocks per segment the histogram is laid out (segment,
+// digit, block) so that one exclusive scan yields every block's output offset
+// per digit and segments never mix.
 //   upsweep:   16-byte key loads, per-warp shared histograms;
-//   downsweep: warp w ranks its 512 elements (16 rounds of 32, in index
+//   downsweep: warp w ranks its elements (16 or 8 rounds of 32, in index
 //              order) with ballots against its running digit counts; the
 //              block turns the counts into local digit offsets, scatters
 //              (key, value) into shared memory in digit order, and writes each
 //              digit's run to its global offset with consecutive threads on
 //              consecutive addresses.
-// Short segments need fewer launches, which is what bounds them:
-//   up to kRsFewBlocks blocks per segment the downsweep sums the segment's
-//   histograms itself (no scan: 8 launches instead of 16; 25 blocks in 8
-//   segments 97 -> 63 us; with 64 blocks the sums take as long as the scans,
-//   63 against 55);
+// Short sorts are bound by the chain of launches and, in each, by the chain of
+// rounds (us of all sort and scan launches of one sort below, before -> after):
+//   up to kRsShortBlocks tiles of 2048 (two for each SM) the tiles are 2048:
+//   half the rounds, and every block still resident at once.  16,384 keys 46
+//   -> 35, 50,021 50 -> 37, 262,144 72 -> 66; from 8 x 100,003 on the halved
+//   tiles only add histograms (66 with tiles of 4096, 72 with 2048; 16 x
+//   1,048,576: 550 and 645);
+//   up to kRsFewRows rows of counts read by all blocks together (blocks per
+//   segment x blocks) the downsweep sums its segment's counts itself: no scan,
+//   8 launches instead of 16.  One row per block then, so that the reads are
+//   coalesced.  262,144 keys 66 -> 42, 1,048,576 92 -> 77, 8 x 262,144 110 ->
+//   104; past the limit the rows take as long as the scans (2 x 1,048,576:
+//   72 + 32 for downsweeps and scans, 110 + 7 with rows);
 //   up to 8192 elements per segment one block sorts it in shared memory, all
 //   four digits in one launch (1,000 elements 34 us in 16 launches -> 10 in
 //   one; 3,000 -> 16).
 constexpr int kRsThreads = 256;
 constexpr int kRsWarps = kRsThreads / 32;
 constexpr int kRsRounds = 16;
-constexpr int kRsTile = kRsThreads * kRsRounds;  // 4096
+constexpr int kRsShortRounds = 8;
 
+// FEW: a row of 256 counts per block, otherwise a row of nb_seg per digit
+template <int ROUNDS, bool FEW>
 __global__ void __launch_bounds__(kRsThreads) k_radix_upsweep(const uint32_t* __restrict__ keys, int shift,
                                                               uint32_t nb_seg, uint32_t* __restrict__ hist) {
+  constexpr int kRsTile = kRsThreads * ROUNDS;
   __shared__ uint32_t h[kRsWarps][256];
   for (int i = threadIdx.x; i < kRsWarps * 256; i += kRsThreads) (&h[0][0])[i] = 0;
   __syncthreads();
@@ -187,7 +200,7 @@ __global__ void __launch_bounds__(kRsThreads) k_radix_upsweep(const uint32_t* __
 #pragma unroll
   for (int w = 0; w < kRsWarps; ++w) sum += h[w][threadIdx.x];
   const uint32_t seg = blockIdx.x / nb_seg, b = blockIdx.x % nb_seg;
-  hist[(size_t(seg) * 256 + threadIdx.x) * nb_seg + b] = sum;
+  hist[FEW ? size_t(blockIdx.x) * 256 + threadIdx.x : (size_t(seg) * 256 + threadIdx.x) * nb_seg + b] = sum;
 }
 
 // lanes of the warp whose 8-bit digit equals this lane's (one ballot per bit)
@@ -212,19 +225,23 @@ __device__ __forceinline__ uint32_t warp_digit_rank(uint32_t* counts, uint32_t d
   return before + __popc(peers & lt);
 }
 
-constexpr uint32_t kRsFewBlocks = 32;
+constexpr uint64_t kRsFewRows = 1u << 16;
+constexpr uint32_t kRsShortBlocks = 296;
+constexpr uint32_t kRsSumRows = 8;  // in flight per thread (4: 63 us for 57 with 256 rows, 16: the same)
 
 // FEW: offs holds the blocks' counts, which every block sums for itself;
 // otherwise their exclusive scan.
-template <bool FEW>
+template <int ROUNDS, bool FEW>
 __global__ void __launch_bounds__(kRsThreads, FEW ? 2 : 3) k_radix_downsweep(
     const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin, uint32_t* __restrict__ kout,
     uint32_t* __restrict__ vout, int shift, uint32_t nb_seg, const uint32_t* __restrict__ offs, int write_keys,
     const uint2* __restrict__ gather_src, uint32_t gather_n, uint2* __restrict__ gather_dst, uint32_t iota_n) {
+  constexpr int kRsTile = kRsThreads * ROUNDS;
+  static_assert(kRsTile >= 8 * 256, "sk holds eight rows of sums");
   __shared__ uint32_t wc[kRsWarps][256];
   __shared__ uint32_t dstart[256];
   __shared__ uint32_t goff[256];
-  __shared__ uint32_t sk[kRsTile];
+  __shared__ __align__(16) uint32_t sk[kRsTile];
   __shared__ uint32_t sv[kRsTile];
   __shared__ uint32_t block_total;
 #pragma unroll
@@ -232,29 +249,54 @@ __global__ void __launch_bounds__(kRsThreads, FEW ? 2 : 3) k_radix_downsweep(
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t lt = (1u << lane) - 1u;
-  const size_t base = size_t(blockIdx.x) * kRsTile + size_t(warp) * (kRsRounds * 32);
-  uint32_t k[kRsRounds], v[kRsRounds];
+  const size_t base = size_t(blockIdx.x) * kRsTile + size_t(warp) * (ROUNDS * 32);
+  uint32_t k[ROUNDS], v[ROUNDS];
   // vin null (first pass of a sort of the identity permutation): an
   // element's value is its index in its segment, 0xffffffff from iota_n on
   if (vin) {
 #pragma unroll
-    for (int r = 0; r < kRsRounds; ++r) {
+    for (int r = 0; r < ROUNDS; ++r) {
       k[r] = kin[base + r * 32 + lane];
       v[r] = vin[base + r * 32 + lane];
     }
   } else {
-    const uint32_t local0 = (blockIdx.x % nb_seg) * kRsTile + uint32_t(warp) * (kRsRounds * 32) + uint32_t(lane);
+    const uint32_t local0 = (blockIdx.x % nb_seg) * kRsTile + uint32_t(warp) * (ROUNDS * 32) + uint32_t(lane);
 #pragma unroll
-    for (int r = 0; r < kRsRounds; ++r) {
+    for (int r = 0; r < ROUNDS; ++r) {
       k[r] = kin[base + r * 32 + lane];
       const uint32_t local = local0 + uint32_t(r) * 32u;
       v[r] = local < iota_n ? local : 0xffffffffu;
     }
   }
-  // phase 1: ranks inside the warp, per-warp digit counts
-  uint32_t rank[kRsRounds];
+  // FEW: the digits' counts in the segment's blocks, all and those before this
+  // one; threads 64 g .. take every fourth row, four digits each, and leave
+  // their sums in sk until phase 2
+  if (FEW) {
+    const uint32_t b = blockIdx.x % nb_seg, g = threadIdx.x >> 6, q = threadIdx.x & 63u;
+    const uint4* h = reinterpret_cast<const uint4*>(offs) + size_t(blockIdx.x - b) * 64 + q;
+    uint4 before = make_uint4(0u, 0u, 0u, 0u), all = before;
+    for (uint32_t i0 = g; i0 < nb_seg; i0 += 4 * kRsSumRows)
 #pragma unroll
-  for (int r = 0; r < kRsRounds; ++r) rank[r] = warp_digit_rank(wc[warp], (k[r] >> shift) & 255u, lane, lt);
+      for (uint32_t j = 0; j < kRsSumRows; ++j) {
+        const uint32_t i = i0 + 4 * j;
+        const uint4 c = i < nb_seg ? h[size_t(i) * 64] : make_uint4(0u, 0u, 0u, 0u);
+        const uint32_t m = i < b ? 0xffffffffu : 0u;
+        before.x += c.x & m;
+        before.y += c.y & m;
+        before.z += c.z & m;
+        before.w += c.w & m;
+        all.x += c.x;
+        all.y += c.y;
+        all.z += c.z;
+        all.w += c.w;
+      }
+    reinterpret_cast<uint4*>(sk)[g * 64 + q] = all;
+    reinterpret_cast<uint4*>(sk)[256 + g * 64 + q] = before;
+  }
+  // phase 1: ranks inside the warp, per-warp digit counts
+  uint32_t rank[ROUNDS];
+#pragma unroll
+  for (int r = 0; r < ROUNDS; ++r) rank[r] = warp_digit_rank(wc[warp], (k[r] >> shift) & 255u, lane, lt);
   __syncthreads();
   // phase 2: block-local digit starts, warp bases, global digit offsets
   {
@@ -271,24 +313,18 @@ __global__ void __launch_bounds__(kRsThreads, FEW ? 2 : 3) k_radix_downsweep(
       run += t;
     }
     const uint32_t seg = blockIdx.x / nb_seg, b = blockIdx.x % nb_seg;
-    const uint32_t* h = offs + (size_t(seg) * 256 + d) * nb_seg;
-    if (!FEW) {
-      goff[d] = h[b];
-    } else {
-      uint32_t before = 0, all = 0;
-#pragma unroll 16
-      for (uint32_t i = 0; i < nb_seg; ++i) {
-        const uint32_t c = h[i];
-        if (i < b) before += c;
-        all += c;
-      }
+    if (FEW) {
+      const uint32_t all = sk[d] + sk[256 + d] + sk[512 + d] + sk[768 + d];
+      const uint32_t before = sk[1024 + d] + sk[1280 + d] + sk[1536 + d] + sk[1792 + d];
       goff[d] = seg * nb_seg * kRsTile + block_excl_scan(all, &block_total) + before;
+    } else {
+      goff[d] = offs[(size_t(seg) * 256 + d) * nb_seg + b];
     }
   }
   __syncthreads();
   // phase 3: stable scatter into shared memory, digit-major
 #pragma unroll
-  for (int r = 0; r < kRsRounds; ++r) {
+  for (int r = 0; r < ROUNDS; ++r) {
     const uint32_t lp = wc[warp][(k[r] >> shift) & 255u] + rank[r];
     sk[lp] = k[r];
     sv[lp] = v[r];
@@ -313,7 +349,16 @@ __global__ void __launch_bounds__(kRsThreads, FEW ? 2 : 3) k_radix_downsweep(
   }
 }
 
-size_t radix_hist_words(size_t n) { return ((n + kRsTile - 1) / kRsTile) * 256 + 1; }
+// n: keys of all segments together
+static int radix_rounds(size_t n) {
+  return n <= size_t(kRsThreads) * kRsShortRounds * kRsShortBlocks ? kRsShortRounds : kRsRounds;
+}
+// (a workspace of n keys also serves fewer)
+size_t radix_hist_words(size_t n) {
+  const size_t shrt = std::min<size_t>((n + kRsThreads * kRsShortRounds - 1) / (kRsThreads * kRsShortRounds),
+                                       kRsShortBlocks);
+  return std::max(shrt, (n + kRsThreads * kRsRounds - 1) / (kRsThreads * kRsRounds)) * 256 + 1;
+}
 
 // One block sorts a whole segment of up to THREADS * kBsRounds elements in
 // shared memory: the same ranking, four digits one after the other, every
@@ -411,6 +456,32 @@ static cudaError_t block_sort(cudaStream_t st, const uint32_t* keys, uint32_t n,
   return cudaGetLastError();
 }
 
+template <int ROUNDS>
+static cudaError_t radix_sort(cudaStream_t st, uint32_t* ka, uint32_t* va, uint32_t* kb, uint32_t* vb, uint32_t npad,
+                              uint32_t nseg, uint32_t* hist, uint32_t* scan_tmp, const uint2* gather_src, uint32_t n,
+                              uint2* gather_dst) {
+  const uint32_t nb_seg = npad / (kRsThreads * ROUNDS), nblocks = nb_seg * nseg;
+  const bool few = uint64_t(nb_seg) * nblocks <= kRsFewRows;
+  for (int pass = 0; pass < 4; ++pass) {
+    const uint32_t* ki = pass & 1 ? kb : ka;
+    const uint32_t* vi = pass == 0 ? nullptr : pass & 1 ? vb : va;  // the first pass forms the indices
+    uint32_t* ko = pass & 1 ? ka : kb;
+    uint32_t* vo = pass & 1 ? va : vb;
+    (few ? k_radix_upsweep<ROUNDS, true> : k_radix_upsweep<ROUNDS, false>)<<<nblocks, kRsThreads, 0, st>>>(
+        ki, 8 * pass, nb_seg, hist);
+    count_launch();
+    if (!few) {
+      const cudaError_t e = exclusive_scan(st, hist, hist, size_t(nblocks) * 256, scan_tmp, 0xffffffffu, nullptr);
+      if (e != cudaSuccess) return e;
+    }
+    const bool last = pass == 3;  // its keys are not needed
+    (few ? k_radix_downsweep<ROUNDS, true> : k_radix_downsweep<ROUNDS, false>)<<<nblocks, kRsThreads, 0, st>>>(
+        ki, vi, ko, vo, 8 * pass, nb_seg, hist, last ? 0 : 1, gather_src, n, last ? gather_dst : nullptr, n);
+    count_launch();
+  }
+  return cudaGetLastError();
+}
+
 // Stable order of every segment's n elements by their 32-bit keys in ka
 // ([nseg][npad], all-ones from n on; ka, kb and vb are scratch after): va gets
 // the elements' indices in their segment, 0xffffffff for the padding, and
@@ -419,28 +490,12 @@ static cudaError_t block_sort(cudaStream_t st, const uint32_t* keys, uint32_t n,
 cudaError_t depth_sort(cudaStream_t st, uint32_t* ka, uint32_t* va, uint32_t* kb, uint32_t* vb, uint32_t npad,
                        uint32_t nseg, uint32_t* hist, uint32_t* scan_tmp, const uint2* gather_src, uint32_t n,
                        uint2* gather_dst) {
-  if (npad == 0 || npad % kRsTile != 0 || nseg == 0) return cudaErrorInvalidValue;
+  if (npad == 0 || npad % (kRsThreads * kRsRounds) != 0 || nseg == 0) return cudaErrorInvalidValue;
   if (n <= 512 * kBsRounds) return block_sort<512>(st, ka, n, npad, nseg, va, gather_src, gather_dst);
   if (n <= 1024 * kBsRounds) return block_sort<1024>(st, ka, n, npad, nseg, va, gather_src, gather_dst);
-  const uint32_t nb_seg = npad / kRsTile, nblocks = nb_seg * nseg;
-  const bool few = nb_seg <= kRsFewBlocks;
-  for (int pass = 0; pass < 4; ++pass) {
-    const uint32_t* ki = pass & 1 ? kb : ka;
-    const uint32_t* vi = pass == 0 ? nullptr : pass & 1 ? vb : va;  // the first pass forms the indices
-    uint32_t* ko = pass & 1 ? ka : kb;
-    uint32_t* vo = pass & 1 ? va : vb;
-    k_radix_upsweep<<<nblocks, kRsThreads, 0, st>>>(ki, 8 * pass, nb_seg, hist);
-    count_launch();
-    if (!few) {
-      const cudaError_t e = exclusive_scan(st, hist, hist, size_t(nblocks) * 256, scan_tmp, 0xffffffffu, nullptr);
-      if (e != cudaSuccess) return e;
-    }
-    const bool last = pass == 3;  // its keys are not needed
-    (few ? k_radix_downsweep<true> : k_radix_downsweep<false>)<<<nblocks, kRsThreads, 0, st>>>(
-        ki, vi, ko, vo, 8 * pass, nb_seg, hist, last ? 0 : 1, gather_src, n, last ? gather_dst : nullptr, n);
-    count_launch();
-  }
-  return cudaGetLastError();
+  if (radix_rounds(size_t(npad) * nseg) == kRsShortRounds)
+    return radix_sort<kRsShortRounds>(st, ka, va, kb, vb, npad, nseg, hist, scan_tmp, gather_src, n, gather_dst);
+  return radix_sort<kRsRounds>(st, ka, va, kb, vb, npad, nseg, hist, scan_tmp, gather_src, n, gather_dst);
 }
 
 // ---------------------------------------------------------------------------

@@ -44,3 +44,19 @@ def test_sort_forms(orc, dev, n):
     assert np.array_equal(U32(t2i), o_t)
     assert np.array_equal(U32(i2p), o_i)
     assert np.array_equal(F(keys).view(np.uint64), o_k)
+
+
+@pytest.mark.parametrize("n", [524288, 524289, 606208, 606209, 1048576, 1048577])
+def test_sort_tiles(orc, dev, n):
+    """Around the limits between tiles of 2048 and 4096 keys and between blocks
+    that sum their segment's counts and the scan of them; equal depths among
+    the keys."""
+    rng = np.random.default_rng(n)
+    xyd = np.empty((n, 3), np.float32)
+    xyd[:, :2] = rng.uniform(-30, 130, (n, 2))
+    xyd[:, 2] = np.where(rng.random(n) < 0.5, rng.uniform(-1.2, 1.2, n), rng.integers(-4, 5, n) / 4.0)
+    aabb = np.concatenate([xyd[:, :2] - 1, xyd[:, :2] + 1], axis=1).astype(np.float32)
+    t2i, i2p = cudarc.splat_gauss_tile2idx_idx2pnt(None, (100, 90), 16, T(xyd, dev), T(aabb, dev))
+    o_t, o_i, _ = orc.tile2pnt(xyd, aabb, 100, 90, 16)
+    assert np.array_equal(U32(t2i), o_t)
+    assert np.array_equal(U32(i2p), o_i)
