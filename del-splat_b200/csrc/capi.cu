@@ -17,8 +17,8 @@ __global__ void k_gauss_project_ref(uint32_t, const float*, const float*, const 
 __global__ void k_circle_project_ref(uint32_t, const float*, const float*, int, int, float, float*, float*);
 __global__ void k_prep_tiles(uint32_t, uint32_t, const float*, const float*, const float*, int, int, int, uint2*, uint32_t*);
 __global__ void k_count_pairs(uint32_t, const float*, const float*, const float*, int, int, int, unsigned long long*);
-__global__ void k_fused_project(uint32_t, uint32_t, int, const float*, const float*, const float*, const float*,
-                                const float*, const ViewBatch, float4*, uint2*, uint32_t*, uint32_t*);
+cudaError_t fused_project(cudaStream_t, uint32_t, uint32_t, int, const float*, const float*, const float*,
+                          const float*, const float*, const ViewBatch&, float4*, uint2*, uint32_t*);
 __global__ void k_project_bwd_geom(uint32_t, const float*, const float*, const float*, const ViewBatch,
                                    float4*, const uint8_t*, float*, float*, float*, float*);
 cudaError_t project_bwd_colour(cudaStream_t, uint32_t, int, const float*, const float*, const ViewBatch&, float4*,
@@ -728,10 +728,9 @@ int dsplat_gauss_batch_forward(dsplat_stream stream, const dsplat_gauss_params* 
   if (n == 0 || pair_capacity == 0) {
     TRY_CUDA(cudaMemsetAsync(w.lists.off1, 0, (size_t(b.num_sb) * w.L.sb_chunks + 1) * 4, st), "memset");
   } else {
-    k_fused_project<<<blocks_for(npad, 128), 128, 0, st>>>(n, npad, params->sh_degree, params->means,
-                                                        params->log_scales, params->quats, params->opacity,
-                                                        params->colors, b, w.rec, w.rect, w.dka, nullptr);
-    count_launch();
+    TRY_CUDA(fused_project(st, n, npad, params->sh_degree, params->means, params->log_scales, params->quats,
+                           params->opacity, params->colors, b, w.rec, w.rect, w.dka),
+             "projection");
     stage_mark(st, 1);
     TRY_CUDA(depth_sort(st, w.dka, w.dva, w.dkb, w.dvb, npad, V, w.hist, w.scan_tmp, w.rect, n, w.srect),
              "depth sort");

@@ -316,52 +316,77 @@ __global__ void __launch_bounds__(256) k_count_pairs(uint32_t n, const float* __
 // Fused projection for a batch of views.  One thread per Gaussian reads its
 // parameters once and writes, for every view v:
 //   rec[v*N+g]   3 x float4 = (px, py, A, B) (C, opacity, r, g) (b, hx, hy, ndcz)
-//   rect[v*N+g]  packed tile span, cnt[v*N+g] = #tiles (cnt nullable)
+//   rect[v*N+g]  packed tile span
 //   dkey[v*Npad+g] depth key bits(max(ndc_z+1,0)); 0xffffffff when no tile
-// sh_deg < 0: colors are RGB [N,3]; else SH coefficients [N,(deg+1)^2,3].
+// DEG < 0: colors are RGB [N,3]; else SH coefficients [N,(DEG+1)^2,3].
+//
+// Bound: instruction issue (about 750 instructions per view and point, the
+// reference's arithmetic kept operation for operation; 79% of the issue
+// slots), and for one or two views the parameters' way in.  With the degree a
+// template argument the rows' copy divides by a constant, and a thread has 16
+// of its words and all its other parameters in flight at once: 16 views of
+// 1,048,576 points 392 -> 361 us, 8 of 4,194,304 880 -> 765 (61% of what its
+// 3.0 GB take at the copy rate), one of 262,144 30.5 -> 25.9, 8 of 100,003
+// 32 -> 29.  8 words in flight 769 (4,194,304 points), 24 784, 48 912.
 // ---------------------------------------------------------------------------
 constexpr int kProjThreads = 128;
-constexpr int kProjStride = 49;  // 48 coefficients + 1 pad (odd stride: conflict-free rows)
+constexpr int kProjLoads = 16;  // words of the colour rows in flight per thread
 
+template <int DEG>
 __global__ void __launch_bounds__(kProjThreads) k_fused_project(
-    uint32_t n, uint32_t npad, int sh_deg, const float* __restrict__ means,
-    const float* __restrict__ log_scales, const float* __restrict__ quats,
-    const float* __restrict__ opacity, const float* __restrict__ colors, const ViewBatch b,
-    float4* __restrict__ rec, uint2* __restrict__ rect, uint32_t* __restrict__ dkey,
-    uint32_t* __restrict__ cnt) {
+    uint32_t n, uint32_t npad, const float* __restrict__ means, const float* __restrict__ log_scales,
+    const float* __restrict__ quats, const float* __restrict__ opacity, const float* __restrict__ colors,
+    const ViewBatch b, float4* __restrict__ rec, uint2* __restrict__ rect, uint32_t* __restrict__ dkey) {
   // the block's colour rows (128 Gaussians x 3K floats, contiguous) are
   // loaded coalesced into shared memory, padded to an odd stride
-  __shared__ float crow[kProjThreads * kProjStride];
-  const int K = sh_deg < 0 ? 1 : (sh_deg + 1) * (sh_deg + 1);
-  const int C = 3 * K;
+  constexpr int K = DEG < 0 ? 1 : (DEG + 1) * (DEG + 1);
+  constexpr int C = 3 * K, kStride = C | 1;
+  __shared__ float crow[kProjThreads * kStride];
   const uint32_t g0 = blockIdx.x * kProjThreads;
-  const uint32_t cnt_blk = n > g0 ? min(uint32_t(kProjThreads), n - g0) : 0u;
-  for (uint32_t i = threadIdx.x; i < cnt_blk * uint32_t(C); i += kProjThreads)
-    crow[(i / C) * kProjStride + (i % C)] = colors[size_t(g0) * C + i];
-  __syncthreads();
+  const uint32_t words = (n > g0 ? min(uint32_t(kProjThreads), n - g0) : 0u) * uint32_t(C);
+  const float* src = colors + size_t(g0) * C;
+  // the point's other parameters arrive beside them
   const uint32_t g = g0 + threadIdx.x;
+  const size_t gl = min(g, n - 1u);
+  const float p[3] = {means[3 * gl], means[3 * gl + 1], means[3 * gl + 2]};
+  const float ls[3] = {log_scales[3 * gl], log_scales[3 * gl + 1], log_scales[3 * gl + 2]};
+  const float q[4] = {quats[4 * gl], quats[4 * gl + 1], quats[4 * gl + 2], quats[4 * gl + 3]};
+  const float op = opacity[gl];
+#pragma unroll
+  for (int k0 = 0; k0 < C; k0 += kProjLoads) {
+    float r[kProjLoads];
+#pragma unroll
+    for (int k = 0; k < kProjLoads; ++k) {
+      const uint32_t i = uint32_t(k0 + k) * kProjThreads + threadIdx.x;
+      if (k0 + k < C && i < words) r[k] = src[i];
+    }
+#pragma unroll
+    for (int k = 0; k < kProjLoads; ++k) {
+      const uint32_t i = uint32_t(k0 + k) * kProjThreads + threadIdx.x;
+      if (k0 + k < C && i < words) crow[(i / C) * kStride + (i % C)] = r[k];
+    }
+  }
+  __syncthreads();
   if (g >= n) {  // padding keys
     if (g < npad)
       for (int v = 0; v < b.num_views; ++v) dkey[size_t(v) * npad + g] = 0xffffffffu;
     return;
   }
-  const float p[3] = {means[3 * g], means[3 * g + 1], means[3 * g + 2]};
-  const float s[3] = {expf_cr(log_scales[3 * g]), expf_cr(log_scales[3 * g + 1]),
-                      expf_cr(log_scales[3 * g + 2])};
-  const float q[4] = {quats[4 * g], quats[4 * g + 1], quats[4 * g + 2], quats[4 * g + 3]};
+  const float s[3] = {expf_cr(ls[0]), expf_cr(ls[1]), expf_cr(ls[2])};
   const float nrm = sqrtf(q[0] * q[0] + q[1] * q[1] + q[2] * q[2] + q[3] * q[3]);
   const float qn[4] = {q[0] / nrm, q[1] / nrm, q[2] / nrm, q[3] / nrm};
   float r[9];
   quat_to_mat3(qn, r);
-  const float op = opacity[g];
-  const float* coef = crow + threadIdx.x * kProjStride;  // read per view from shared memory
+  // volatile: the compiler would keep the row in registers for all views, at
+  // half the resident warps (16 views 460 us)
+  const volatile float* coef = crow + threadIdx.x * kStride;
   const float tsf = tile_inv(b.ts);
   for (int v = 0; v < b.num_views; ++v) {
     const ViewDev& vd = b.v[v];
     Proj o;
     project_core(p, r, s, vd.mvp, vd.w, vd.h, &o);
     float col[3];
-    if (sh_deg < 0) {
+    if (DEG < 0) {
       col[0] = coef[0];
       col[1] = coef[1];
       col[2] = coef[2];
@@ -369,13 +394,12 @@ __global__ void __launch_bounds__(kProjThreads) k_fused_project(
       const float d0 = p[0] - vd.campos[0], d1 = p[1] - vd.campos[1], d2 = p[2] - vd.campos[2];
       const float dn = sqrtf(d0 * d0 + d1 * d1 + d2 * d2);
       float bs[16];
-      sh_basis(sh_deg, d0 / dn, d1 / dn, d2 / dn, bs);
+      sh_basis(DEG, d0 / dn, d1 / dn, d2 / dn, bs);
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         float acc = 0.f;
 #pragma unroll
-        for (int k = 0; k < 16; ++k)
-          if (k < K) acc += bs[k] * coef[k * 3 + c];
+        for (int k = 0; k < K; ++k) acc += bs[k] * coef[k * 3 + c];
         acc += 0.5f;
         col[c] = acc > 0.f ? acc : 0.f;
       }
@@ -393,9 +417,22 @@ __global__ void __launch_bounds__(kProjThreads) k_fused_project(
       rec[3 * o_idx + 2] = make_float4(col[2], o.hx, o.hy, o.ndcz);
     }
     rect[o_idx] = pack_rect(x0, y0, x1, y1);
-    if (cnt) cnt[o_idx] = c;
     dkey[size_t(v) * npad + g] = c ? depth_bits(o.ndcz) : 0xffffffffu;
   }
+}
+
+cudaError_t fused_project(cudaStream_t st, uint32_t n, uint32_t npad, int sh_deg, const float* means,
+                          const float* log_scales, const float* quats, const float* opacity, const float* colors,
+                          const ViewBatch& b, float4* rec, uint2* rect, uint32_t* dkey) {
+  const unsigned grid = (npad + kProjThreads - 1) / kProjThreads;
+#define X(DEG)                                                                                                   \
+  if (sh_deg == DEG)                                                                                             \
+    k_fused_project<DEG><<<grid, kProjThreads, 0, st>>>(n, npad, means, log_scales, quats, opacity, colors, b, rec, \
+                                                        rect, dkey);
+  X(-1) X(0) X(1) X(2) X(3)
+#undef X
+  count_launch();
+  return cudaGetLastError();
 }
 
 }  // namespace dsplat

@@ -11,7 +11,10 @@
 // B200 structure: the unit of work is a warp task.  With 8x8 tiles a task
 // covers two horizontally adjacent tiles of one superblock (16x8 pixels, 4
 // per lane); with 16x16 or 32x32 tiles a slab of one tile (32 lanes x 2..8
-// pixels).  A lane's pixels share its column.  A warp stages 32 list entries
+// pixels).  A lane's pixels share its column.  The items whose walk is a good
+// part of what a resident warp has to do (see the task order in tiles.cu), and
+// the drop-in forward's tiles, are walked in blocks of 8x8 pixels instead
+// (raster_block.cuh).  A warp stages 32 list entries
 // at a time into its own shared-memory slots (one coalesced index load + one
 // 48-byte record gather per lane; the next batch's index loads are issued
 // before the current batch is walked), then every lane walks them with
