@@ -202,7 +202,8 @@ __device__ __forceinline__ f2 mul2_rn(f2 a, f2 b, f2 nz) { return fma2(a, b, nz)
 //     scaled by 2^(k div 128) exactly.
 // Otherwise (|x| > 87, NaN, or the rounding test failed -- about 1e-4 of
 // the inputs), expf_cr_slow evaluates the reduction in double precision
-// (64-entry table, degree-6 polynomial) and rounds the double once to float, which also produces subnormal results, 0 and infinity.
+// (64-entry table, degree-6 polynomial) and rounds the double once to float,
+// which also produces subnormal results, 0 and infinity.
 // With 64 entries the polynomial needs another term, and with ln2/128 in
 // three short parts the reduction another step (17 operations); 128 entries
 // also halve the error, so fewer inputs fail the rounding test.  Measured on
