@@ -7,7 +7,7 @@
 // of kSegEntries in the whole list, so that the work is spread over the GPU
 // whatever the lists' lengths (one block per superblock left the long lists
 // of the view's middle to a few blocks: 1308 us for 1,048,576 Gaussians at
-// 1920x1080 and 16x16 tiles, 510 superblocks; by segments 148 us):
+// 1920x1080 and 16x16 tiles, 510 superblocks; by segments 137 us):
 //   k_seg_count    per (segment, tile) entry counts;
 //   k_seg_scan     per superblock: each tile's counts become exclusive
 //                  prefixes over its segments, their sum the tile's length;
@@ -254,8 +254,14 @@ __global__ void __launch_bounds__(kSegThreads) k_seg_scatter(const uint2* __rest
 }
 
 namespace {
-unsigned seg_grid(uint64_t capacity, uint32_t num_sb) {
-  return unsigned(std::min<size_t>(tile_seg_slots(capacity, num_sb), 148 * 8));
+// Blocks of a kernel over the segments: more of them even out what the
+// segments take (how many tiles their entries cover), each pays for the search
+// of its first segment.  1,048,576 Gaussians at 1920x1080, us for 8, 24, 32,
+// 64 and 256 blocks per SM: scatter 105, 94, 94, 97, 150; count, whose
+// segments all take the same, 40, 40 (12 per SM), 43 (32).
+constexpr size_t kSegCountBlocks = 148 * 8, kSegScatterBlocks = 148 * 24;
+unsigned seg_grid(uint64_t capacity, uint32_t num_sb, size_t most) {
+  return unsigned(std::min<size_t>(tile_seg_slots(capacity, num_sb), most));
 }
 }  // namespace
 
@@ -263,7 +269,7 @@ unsigned seg_grid(uint64_t capacity, uint32_t num_sb) {
 // tile_seg_slots() times the superblock's tile count words (64 at most).
 cudaError_t split_tile_lists(cudaStream_t st, const uint2* list1, const uint32_t* off1, uint32_t nchunk,
                              uint64_t capacity, const ViewBatch& b, uint32_t* segcnt, uint32_t* tcnt) {
-  const unsigned grid = seg_grid(capacity, b.num_sb);
+  const unsigned grid = seg_grid(capacity, b.num_sb, kSegCountBlocks);
   switch (b.v[0].sb_log2) {
     case 0: k_seg_count<0><<<grid, kSegThreads, 0, st>>>(list1, off1, nchunk, capacity, b.num_sb, segcnt); break;
     case 1: k_seg_count<1><<<grid, kSegThreads, 0, st>>>(list1, off1, nchunk, capacity, b.num_sb, segcnt); break;
@@ -279,7 +285,7 @@ cudaError_t split_tile_lists(cudaStream_t st, const uint2* list1, const uint32_t
 cudaError_t scatter_tile_lists(cudaStream_t st, const uint2* list1, const uint32_t* off1, uint32_t nchunk,
                                uint64_t capacity, const ViewBatch& b, const uint32_t* segcnt,
                                const uint32_t* item_start, uint32_t* idx2pnt, uint32_t* out_tile, uint32_t* flags) {
-  const unsigned grid = seg_grid(capacity, b.num_sb);
+  const unsigned grid = seg_grid(capacity, b.num_sb, kSegScatterBlocks);
 #define X(SL)                                                                                                       \
   k_seg_scatter<SL><<<grid, kSegThreads, 0, st>>>(list1, off1, nchunk, capacity, b.num_sb, b.v[0], segcnt,           \
                                                   item_start, idx2pnt, out_tile, flags)
