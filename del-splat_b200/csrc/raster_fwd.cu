@@ -278,7 +278,12 @@ __global__ void __launch_bounds__(32 * kRasterWarps) k_raster_fwd(
     uint32_t cost;
     if (t.block) {
       BlockPlace p;
-      if (!block_place(b, ig, t.sub, nx, &p)) continue;
+      if (!block_place(b, ig, t.sub, nx, &p)) {
+        // a block of a larger tile outside the view: its slot of the tile is
+        // its own where a tile has as many slots as blocks
+        if (TS > 8 && target && lane == 0 && slots == TS * TS / 64) slab_loss[size_t(t.item) * slots + t.sub] = 0.f;
+        continue;
+      }
       const FwdOut out{out_rgb, out_T, out_alpha, out_last, target, grad_pix};
       cost = blend_block<false>(SbWords{list1, p.lx, ig.ly, 1u}, PackedBlockSrc{src.rec}, ent, park, park_pos, tab, nz,
                                 ig.s, ig.e, p.px0, p.py0, vd.w, vd.w, vd.h, false, vd.pix_base, out, [&](float l) {
