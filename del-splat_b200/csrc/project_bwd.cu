@@ -250,6 +250,9 @@ __global__ void __launch_bounds__(128, 6) k_project_bwd_geom(uint32_t n, const f
     // consumed: leave the record's geometry part zero for the next backward
     gp[0] = make_float4(0.f, 0.f, 0.f, 0.f);
     *reinterpret_cast<float2*>(gp + 1) = make_float2(0.f, 0.f);
+    // nothing flows through a zero record, also where the chain's factors are
+    // infinite (a needle's determinant can be 0 in float32)
+    if (g0.x == 0.f && g0.y == 0.f && g0.z == 0.f && g0.w == 0.f && g1.x == 0.f && g1.y == 0.f) continue;
     float c[16];
     geometry_view(p, dd, R, views[view], views[view][16], views[view][17], g0, g1, c);
 #pragma unroll
