@@ -18,13 +18,13 @@ __global__ void k_circle_project_ref(uint32_t, const float*, const float*, int, 
 __global__ void k_prep_tiles(uint32_t, uint32_t, const float*, const float*, const float*, int, int, int, uint2*, uint32_t*);
 __global__ void k_count_pairs(uint32_t, const float*, const float*, const float*, int, int, int, unsigned long long*);
 cudaError_t fused_project(cudaStream_t, uint32_t, uint32_t, int, const float*, const float*, const float*,
-                          const float*, const float*, const ViewBatch&, float4*, uint2*, uint32_t*);
+                          const float*, const float*, const ViewBatch&, float4*, uint2*, uint32_t*, uint32_t*);
 __global__ void k_project_bwd_geom(uint32_t, const float*, const float*, const float*, const ViewBatch,
                                    float4*, const uint8_t*, float*, float*, float*, float*);
 cudaError_t project_bwd_colour(cudaStream_t, uint32_t, int, const float*, const float*, const ViewBatch&, float4*,
                                uint8_t*, float*, float*, unsigned long long*, unsigned long long);
 __global__ void k_prepare_grad2d(const unsigned long long*, unsigned long long, float4*, size_t, uint32_t*, size_t,
-                                 uint32_t*);
+                                 uint32_t*, const float*, size_t, uint32_t*);
 __global__ void k_adam(size_t, float*, const float*, float*, float*, float, float, float, float, float, float);
 __global__ void k_sb_count(const uint32_t*, const uint2*, uint32_t, uint32_t, const ViewBatch, uint32_t*,
                            unsigned long long*);
@@ -729,7 +729,7 @@ int dsplat_gauss_batch_forward(dsplat_stream stream, const dsplat_gauss_params* 
     TRY_CUDA(cudaMemsetAsync(w.lists.off1, 0, (size_t(b.num_sb) * w.L.sb_chunks + 1) * 4, st), "memset");
   } else {
     TRY_CUDA(fused_project(st, n, npad, params->sh_degree, params->means, params->log_scales, params->quats,
-                           params->opacity, params->colors, b, w.rec, w.rect, w.dka),
+                           params->opacity, params->colors, b, w.rec, w.rect, w.dka, w.sched + kSchedOdd),
              "projection");
     stage_mark(st, 1);
     TRY_CUDA(depth_sort(st, w.dka, w.dva, w.dkb, w.dvb, npad, V, w.hist, w.scan_tmp, w.rect, n, w.srect),
@@ -778,7 +778,8 @@ int dsplat_gauss_batch_backward(dsplat_stream stream, const dsplat_gauss_params*
   // consumes, so only a buffer not known to be clean is cleared here
   const unsigned long long tag = grad2d_tag_value(w.L, n, num_views);
   k_prepare_grad2d<<<blocks_for(3 * VN, 256) < 4096 ? blocks_for(3 * VN, 256) : 4096, 256, 0, st>>>(
-      w.grad2d_tag, tag, w.grad2d, 3 * VN, w.touched, (VN + 3) / 4, w.flags + 3);
+      w.grad2d_tag, tag, w.grad2d, 3 * VN, w.touched, (VN + 3) / 4, w.flags + 3, grad_rgb, size_t(b.num_pix) * 3,
+      w.sched + kSchedOdd);
   count_launch();
   // the forward's longest-first task order: it ranks the tasks by the walks
   // of the forward before it, the same measure as this forward's (equal once

@@ -59,7 +59,7 @@ struct FwdArgs {
   uint32_t nchunk;
   uint64_t capacity;
   const uint32_t* order;
-  const uint32_t* sched;
+  uint32_t* sched;
   uint32_t* counter;
   float* out_rgb;
   float* out_T;
@@ -94,7 +94,23 @@ struct BwdArgs {
 // cursors [40, 73), and
 constexpr int kSchedCost = 74;   // u64: sum of the items' costs
 constexpr int kSchedHeavy = 76;  // leading items of the order walked in 8x8 blocks
+constexpr int kSchedOdd = 77;    // not 0: the batch has something odd (see kBwdLarge)
 constexpr int kSchedWords = 80;
+
+// What the backward raster's packed pairs may meet (bwd_task): nothing that is
+// not finite, and no product that overflows, since a zero alpha has to stay a
+// zero gradient.  Opacities are at most 1, colours and upstream gradients at
+// most kBwdLarge, and the conic's terms at the box's corner at most kBwdTerms
+// (an axis ratio of 670 at 45 degrees): beyond it the exponent's roundings can
+// turn an alpha into e times itself (2.5e-7 kBwdTerms = 1), and a pixel's walk
+// overflows once five of its entries have been held at 1 / (1 - alpha) = 1e7
+// that way.
+constexpr float kBwdLarge = 3e5f, kBwdTerms = 4e6f;
+__device__ __forceinline__ bool odd_record(const float* conic, float hx, float hy, float opacity, const float* rgb) {
+  const float terms = fabsf(conic[0]) * hx * hx + 2.f * fabsf(conic[1]) * hx * hy + fabsf(conic[2]) * hy * hy;
+  return !(terms <= kBwdTerms && fabsf(opacity) <= 1.f && fabsf(rgb[0]) <= kBwdLarge && fabsf(rgb[1]) <= kBwdLarge &&
+           fabsf(rgb[2]) <= kBwdLarge);
+}
 
 // The five parameter tensors of one fused Adam launch (k_adam_fused).
 struct AdamSeg {

@@ -317,6 +317,7 @@ __global__ void __launch_bounds__(256) k_count_pairs(uint32_t n, const float* __
 // parameters once and writes, for every view v:
 //   rec[v*N+g]   3 x float4 = (px, py, A, B) (C, opacity, r, g) (b, hx, hy, ndcz)
 //   rect[v*N+g]  packed tile span
+//   odd          set to 1 where a record is odd (odd_record); the caller clears it
 //   dkey[v*Npad+g] depth key bits(max(ndc_z+1,0)); 0xffffffff when no tile
 // DEG < 0: colors are RGB [N,3]; else SH coefficients [N,(DEG+1)^2,3].
 //
@@ -336,7 +337,8 @@ template <int DEG>
 __global__ void __launch_bounds__(kProjThreads) k_fused_project(
     uint32_t n, uint32_t npad, const float* __restrict__ means, const float* __restrict__ log_scales,
     const float* __restrict__ quats, const float* __restrict__ opacity, const float* __restrict__ colors,
-    const ViewBatch b, float4* __restrict__ rec, uint2* __restrict__ rect, uint32_t* __restrict__ dkey) {
+    const ViewBatch b, float4* __restrict__ rec, uint2* __restrict__ rect, uint32_t* __restrict__ dkey,
+    uint32_t* __restrict__ odd) {
   // the block's colour rows (128 Gaussians x 3K floats, contiguous) are
   // loaded coalesced into shared memory, padded to an odd stride
   constexpr int K = DEG < 0 ? 1 : (DEG + 1) * (DEG + 1);
@@ -415,6 +417,7 @@ __global__ void __launch_bounds__(kProjThreads) k_fused_project(
       rec[3 * o_idx + 0] = make_float4(o.px, o.py, o.conic[0], o.conic[1]);
       rec[3 * o_idx + 1] = make_float4(o.conic[2], op, col[0], col[1]);
       rec[3 * o_idx + 2] = make_float4(col[2], o.hx, o.hy, o.ndcz);
+      if (odd_record(o.conic, o.hx, o.hy, op, col)) *odd = 1u;
     }
     rect[o_idx] = pack_rect(x0, y0, x1, y1);
     dkey[size_t(v) * npad + g] = c ? depth_bits(o.ndcz) : 0xffffffffu;
@@ -423,12 +426,12 @@ __global__ void __launch_bounds__(kProjThreads) k_fused_project(
 
 cudaError_t fused_project(cudaStream_t st, uint32_t n, uint32_t npad, int sh_deg, const float* means,
                           const float* log_scales, const float* quats, const float* opacity, const float* colors,
-                          const ViewBatch& b, float4* rec, uint2* rect, uint32_t* dkey) {
+                          const ViewBatch& b, float4* rec, uint2* rect, uint32_t* dkey, uint32_t* odd) {
   const unsigned grid = (npad + kProjThreads - 1) / kProjThreads;
 #define X(DEG)                                                                                                   \
   if (sh_deg == DEG)                                                                                             \
     k_fused_project<DEG><<<grid, kProjThreads, 0, st>>>(n, npad, means, log_scales, quats, opacity, colors, b, rec, \
-                                                        rect, dkey);
+                                                        rect, dkey, odd);
   X(-1) X(0) X(1) X(2) X(3)
 #undef X
   count_launch();

@@ -426,11 +426,20 @@ cudaError_t project_bwd_colour(cudaStream_t st, uint32_t n, int sh_deg, const fl
 // Clears grad2d and its marks unless the tag says they are already all zero
 // (the previous backward on this layout consumed them).  Blocks only read the tag; the
 // colour kernel of the same backward writes it.  Also sets the backward
-// raster's work counter to zero.
+// raster's work counter to zero, and marks the batch where the caller's upstream
+// gradient (nullable) has something odd.
 __global__ void k_prepare_grad2d(const unsigned long long* __restrict__ clean_tag, unsigned long long tag,
                                  float4* __restrict__ grad2d, size_t count, uint32_t* __restrict__ touched,
-                                 size_t touched_words, uint32_t* __restrict__ work_counter) {
+                                 size_t touched_words, uint32_t* __restrict__ work_counter,
+                                 const float* __restrict__ grad_rgb, size_t grad_words, uint32_t* __restrict__ odd) {
   if (blockIdx.x == 0 && threadIdx.x == 0) *work_counter = 0u;
+  if (grad_rgb) {
+    bool large = false;
+#pragma unroll 4
+    for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < grad_words; i += size_t(gridDim.x) * blockDim.x)
+      large = large || !(fabsf(grad_rgb[i]) <= kBwdLarge);
+    if (large) *odd = 1u;
+  }
   if (*clean_tag == tag) return;
   for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += size_t(gridDim.x) * blockDim.x)
     grad2d[i] = make_float4(0.f, 0.f, 0.f, 0.f);

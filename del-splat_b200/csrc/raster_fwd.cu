@@ -232,6 +232,10 @@ __device__ __forceinline__ uint32_t fwd_slab(const Walk& walk, const Src& src, E
   return cost;
 }
 
+// A task's loss from which on one of its upstream gradients 2 (image - target)
+// can be above kBwdLarge.
+constexpr float kLargeLoss = 0.25f * kBwdLarge * kBwdLarge;
+
 // ---------------------------------------------------------------------------
 // Fused-path forward: persistent, per-warp work stealing, walking each tile's
 // entries out of its superblock list.  The first sched[kSchedHeavy] items of
@@ -245,7 +249,7 @@ template <int TS, int PPL, int NT>
 __global__ void __launch_bounds__(32 * kRasterWarps) k_raster_fwd(
     const ViewBatch b, uint32_t n, const float4* __restrict__ rec, const uint2* __restrict__ list1,
     const uint32_t* __restrict__ off1, uint32_t nchunk, uint64_t capacity, const uint32_t* __restrict__ order,
-    const uint32_t* __restrict__ sched, uint32_t* __restrict__ work_counter, float* __restrict__ out_rgb,
+    uint32_t* __restrict__ sched, uint32_t* __restrict__ work_counter, float* __restrict__ out_rgb,
     float* __restrict__ out_T, float* __restrict__ out_alpha, uint32_t* __restrict__ out_last,
     const float* __restrict__ target, float* __restrict__ grad_pix, float* __restrict__ slab_loss, uint32_t slots, uint32_t* __restrict__ item_cost,
     float nz) {
@@ -287,6 +291,7 @@ __global__ void __launch_bounds__(32 * kRasterWarps) k_raster_fwd(
       const FwdOut out{out_rgb, out_T, out_alpha, out_last, target, grad_pix};
       cost = blend_block<false>(SbWords{list1, p.lx, ig.ly, 1u}, PackedBlockSrc{src.rec}, ent, park, park_pos, tab, nz,
                                 ig.s, ig.e, p.px0, p.py0, vd.w, vd.w, vd.h, false, vd.pix_base, out, [&](float l) {
+                                  if (!(l <= kLargeLoss)) sched[kSchedOdd] = 1u;
                                   float* const p0 = slab_loss + size_t(t.item) * slots;
                                   constexpr uint32_t blocks = TS * TS / 64;
                                   if (TS == 8) p0[t.sub * slots] = l;  // the run's tile t.sub
@@ -300,6 +305,7 @@ __global__ void __launch_bounds__(32 * kRasterWarps) k_raster_fwd(
           walk, src, reinterpret_cast<EntP*>(ent), park, park_pos, tab, nz, ig.s, ig.e, ig.px0,
           ig.py0 + int(t.sub) * G::SLAB_ROWS, vd.w, vd.h, xend, out_rgb, vd.pix_base, out_T, out_alpha, out_last, target,
           grad_pix, [&](float l) {
+            if (!(l <= kLargeLoss)) sched[kSchedOdd] = 1u;
             float* const p0 = slab_loss + size_t(t.item) * G::SLABS + t.sub;
             *p0 = l;
             // the run's other tile has its loss in the leftmost one's slot

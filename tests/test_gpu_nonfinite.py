@@ -27,3 +27,49 @@ def test_zero_gradient_through_a_needle_is_zero(dev):
     batch.backward(p, grads, torch.zeros_like(batch.out_rgb))
     for k in GROUPS:
         assert not F(grads[k]).any(), k  # NaN counts as non-zero
+
+
+def _pixel_scene(w=48, h=40):
+    """One Gaussian per pixel, its box inside the pixel; a random half of them far, the others near."""
+    rng = np.random.default_rng(9)
+    n = w * h
+    far = rng.random(n) < 0.5
+    y, x = np.divmod(np.arange(n), w)
+    means = np.stack([(x + 0.5) * 2 / w - 1, 1 - (y + 0.5) * 2 / h, np.where(far, -0.5, 0.5)], 1).astype(np.float32)
+    ls = np.full((n, 3), np.log(0.1 / max(w, h)), np.float32)
+    quats = np.tile(np.array([[0, 0, 0, 1]], np.float32), (n, 1))
+    cam = scenes.Camera(w, h, np.eye(4, dtype=np.float32).reshape(16), np.zeros(3, np.float32))
+    sc = scenes.GaussScene(means, ls, quats, np.full(n, 0.5, np.float32), rng.uniform(0, 1, (n, 3)).astype(np.float32),
+                           -1, [cam], 8)
+    return sc, far
+
+
+@pytest.mark.parametrize("ts,ppl", CONFIGS)
+@pytest.mark.parametrize("what", ["inf colour", "nan colour", "inf opacity", "nan opacity", "nan upstream"])
+def test_backward_keeps_it_in_its_pixels(dev, ts, ppl, what):
+    """Half of the pixels hold something that is not finite; the Gaussians of
+    the other pixels get the gradients that they get without it."""
+    sc, far = _pixel_scene()
+    up = np.random.default_rng(4).uniform(-1, 1, (sc.n, 3)).astype(np.float32)
+    results = []
+    for odd in (False, True):
+        p = params_of(sc, dev)
+        grad_rgb = torch.from_numpy(up).to(dev)
+        sel = torch.from_numpy(far).to(dev)
+        if odd:
+            value = float(what.split()[0])
+            (p["colors"] if "colour" in what else p["opacity"] if "opacity" in what else grad_rgb)[sel] = value
+        batch = GaussBatch(sc.n, sc.cameras, ts, -1, pair_capacity=1 << 16, device=dev, pixels_per_lane=ppl)
+        batch.ensure_capacity(p)
+        res = []
+        for blocks in masks(batch):
+            set_blocks(batch, blocks)
+            batch.forward(p)
+            grads = {k: torch.zeros_like(v) for k, v in p.items()}
+            batch.backward(p, grads, grad_rgb.reshape(-1))
+            res.append({k: F(grads[k])[~far] for k in GROUPS})
+        results.append(res)
+    for a, b in zip(*results):
+        assert np.abs(a["colors"]).min() > 0
+        for k in GROUPS:
+            assert np.isfinite(a[k]).all() and np.array_equal(a[k], b[k]), k
