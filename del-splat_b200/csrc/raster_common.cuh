@@ -97,7 +97,7 @@ struct EntP {                // conic (A, B, C) staged times -1/2 (see make_entp
   float4 c;  // r, r, g, g
   float4 d;  // b, b, px, -A/2
   float4 e;  // box x0, box x1, box y0, box y1
-  float4 f;  // exponent in expf_cr's fast range (0/1 bits), list position (bits), -, -
+  float4 f;  // plain entry (0/1 bits, see make_entp), list position (bits), -, -
   __device__ __forceinline__ void set_pos(uint32_t pos) { f.y = __uint_as_float(pos); }
 };
 
@@ -107,7 +107,9 @@ __device__ __forceinline__ void make_entp(EntP* dst, float px, float py, float A
   // bounded in magnitude by the same sum of absolute terms at the box's
   // farthest corner; below 170 (rounding adds far less than the margin to
   // 174) every exponent -q/2 of the entry lies in expf_cr's fast range and
-  // the per-pixel range check is skipped.  NaN or infinite terms fail it.
+  // the per-pixel range check is skipped.  NaN or infinite terms fail it.  So
+  // does an infinite or NaN colour, which must not meet the alpha of 0 that a
+  // pixel outside the box takes: the form with the range check leaves it out.
   //
   // The conic is staged times -1/2 (exact), so that the walk forms the
   // exponent -q/2 directly: every product and sum of q scaled by -1/2 is the
@@ -123,7 +125,8 @@ __device__ __forceinline__ void make_entp(EntP* dst, float px, float py, float A
   dst->c = make_float4(r, r, g, g);
   dst->d = make_float4(b, b, px, hA);
   dst->e = make_float4(x0, x1, y0, y1);
-  dst->f = make_float4(__uint_as_float(mag < 170.f ? 1u : 0u), 0.f, 0.f, 0.f);
+  const bool plain = mag < 170.f && fabsf(r) < INFINITY && fabsf(g) < INFINITY && fabsf(b) < INFINITY;
+  dst->f = make_float4(__uint_as_float(plain ? 1u : 0u), 0.f, 0.f, 0.f);
 }
 
 template <int TS, int PPL_>

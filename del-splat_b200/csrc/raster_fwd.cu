@@ -118,8 +118,9 @@ __device__ __forceinline__ uint32_t fwd_slab(const Walk& walk, const Src& src, E
         if (!SPLIT) col_terms(fxp[0], &adxdx2_1, &dx2_1);
         const uint32_t pos = __float_as_uint(ef.y);
         // all instances compute the same bits: `inrange` skips expf_cr's
-        // range check (proven by the entry's staged flag), `rows` the row
-        // test of an entry whose box holds every row of the slab
+        // range check and the care for colours that are not finite (proven by
+        // the entry's staged flag), `rows` the row test of an entry whose box
+        // holds every row of the slab
         auto blend_slots = [&](auto inrange, auto rows) {
 #pragma unroll
           for (int q = 0; q < NP; ++q) {
@@ -144,9 +145,15 @@ __device__ __forceinline__ uint32_t fwd_slab(const Walk& walk, const Src& src, E
             // state is unchanged
             const f2 e2 = decltype(rows)::value ? al : f2_make(a0 ? f2_lo(al) : 0.f, a1 ? f2_hi(al) : 0.f);
             const f2 eo2 = mul2_rn(T2[q], e2, nz2);
-            c02[q] = add2(c02[q], mul2_rn(qc.x, eo2, nz2));
-            c12[q] = add2(c12[q], mul2_rn(qc.y, eo2, nz2));
-            c22[q] = add2(c22[q], mul2_rn(qbl, eo2, nz2));
+            // of an entry that may have an infinite colour, a pixel outside
+            // the box takes colour 0
+            auto colour = [&](f2 c) {
+              return decltype(inrange)::value || decltype(rows)::value
+                         ? c : f2_make(a0 ? f2_lo(c) : 0.f, a1 ? f2_hi(c) : 0.f);
+            };
+            c02[q] = add2(c02[q], mul2_rn(colour(qc.x), eo2, nz2));
+            c12[q] = add2(c12[q], mul2_rn(colour(qc.y), eo2, nz2));
+            c22[q] = add2(c22[q], mul2_rn(colour(qbl), eo2, nz2));
             T2[q] = mul2(T2[q], sub2(f2_dup(1.f), e2));
             as2[q] = add2(as2[q], eo2);
             // a stopped slot's alpha sum is parked at -inf (it stays -inf

@@ -73,3 +73,24 @@ def test_backward_keeps_it_in_its_pixels(dev, ts, ppl, what):
         assert np.abs(a["colors"]).min() > 0
         for k in GROUPS:
             assert np.isfinite(a[k]).all() and np.array_equal(a[k], b[k]), k
+
+
+@pytest.mark.parametrize("ts,ppl", CONFIGS)
+def test_batched_image_keeps_odd_colours_in_their_boxes(orc, dev, ts, ppl):
+    """Infinite and NaN colours, every item walked in both shapes: the
+    oracle's image, bit for bit."""
+    sc = scenes.config0(seed=5, n=300, size=(90, 60))
+    sc.colors[::7] = np.inf
+    sc.colors[3::11, 1] = np.nan
+    cam = sc.cameras[0]
+    p = params_of(sc, dev)
+    batch = GaussBatch(sc.n, sc.cameras, ts, -1, pair_capacity=1 << 16, device=dev, pixels_per_lane=ppl)
+    batch.ensure_capacity(p)
+    xyd, conic, aabb, rgb = orc.fused_project(sc.means, sc.log_scales, sc.quats, sc.colors, -1, cam.mvp, cam.campos, 90, 60)
+    t2i, i2p, _ = orc.tile2pnt(xyd, aabb, 90, 60, ts)
+    want, _, _ = orc.gauss_rasterize_tiled(90, 60, ts, t2i, i2p, xyd, conic, aabb, sc.opacity, rgb)
+    assert np.isfinite(want).any() and not np.isfinite(want).all()
+    for blocks in masks(batch):
+        set_blocks(batch, blocks)
+        batch.forward(p)
+        assert np.array_equal(F(batch.images()[0]), want, equal_nan=True)
