@@ -497,7 +497,7 @@ BatchWs carve_batch(void* ws, uint32_t n, const ViewBatch& b, uint64_t capacity)
   w.grad_pix = c.take<float>(size_t(b.num_pix) * 3, &L.off_grad_pix);
   w.slab_loss = c.take<float>(size_t(b.num_items) * L.slabs_per_tile, &L.off_slab_loss);
   w.grad2d = c.take<float4>(3 * VN + 3, &L.off_grad2d);
-  w.grad2d_tag = c.take<unsigned long long>(1);
+  w.grad2d_tag = c.take<unsigned long long>(1);  // here for callers who clear it (dsplat.h)
   w.touched = c.take<uint32_t>((VN + 3) / 4);
   w.task_order = c.take<uint32_t>(size_t(b.num_items) + 1);
   w.item_cost = c.take<uint32_t>(size_t(b.num_items) + 1);

@@ -85,6 +85,10 @@ class GaussBatch:
                                                   self.capacity, ctypes.byref(L)), "batch_layout")
         self.layout = L
         self.ws = torch.empty(int(L.total_bytes), dtype=torch.uint8, device=self.device)
+        # the mark that the 2D gradients are zero: memory of an earlier batch
+        # can hold it while other tensors have written over the gradients
+        mark = int(L.off_grad2d) + 48 * (self.num_views * self.n + 1)
+        self._ws((mark + 255) // 256 * 256, 1, torch.int64).zero_()
         self.out_rgb = torch.empty(int(L.num_pix) * 3, dtype=torch.float32, device=self.device)
 
     def ensure_capacity(self, params: Dict[str, torch.Tensor], slack: float = 1.05) -> int:
