@@ -56,6 +56,7 @@ cudaError_t raster_bwd(cudaStream_t, const ViewBatch&, const BwdArgs&);
 bool raster_config_ok(int ts, int ppl);
 int raster_default_ppl(int ts);
 uint32_t raster_slabs_per_tile(int ts, int ppl);
+uint32_t loss_units_per_slab(int ts, int ppl);
 __global__ void k_order_hist(const ViewBatch, const uint32_t*, uint32_t, const uint32_t*, uint32_t*);
 __global__ void k_order_scatter(const ViewBatch, const uint32_t*, uint32_t, uint32_t*, float, uint32_t*, uint32_t*);
 cudaError_t raster_fwd_aos(cudaStream_t, int, int, int, float*, const float*, const float*, const float*, const float*,
@@ -403,6 +404,7 @@ struct BatchWs {
   uint32_t* pix_stop;
   float* grad_pix;
   float* slab_loss;
+  float* unit_loss;  // slab_loss's parts (tiles above 8x8)
   float4* grad2d;
   unsigned long long* grad2d_tag;  // == grad2d_tag_value(): grad2d and touched are all zero
   uint32_t* touched;  // a byte per grad2d record
@@ -496,6 +498,8 @@ BatchWs carve_batch(void* ws, uint32_t n, const ViewBatch& b, uint64_t capacity)
   w.pix_stop = c.take<uint32_t>(b.num_pix, &L.off_pix_stop);
   w.grad_pix = c.take<float>(size_t(b.num_pix) * 3, &L.off_grad_pix);
   w.slab_loss = c.take<float>(size_t(b.num_items) * L.slabs_per_tile, &L.off_slab_loss);
+  w.unit_loss = c.take<float>(
+      b.ts == 8 ? 0 : size_t(b.num_items) * L.slabs_per_tile * loss_units_per_slab(b.ts, b.ppl));
   w.grad2d = c.take<float4>(3 * VN + 3, &L.off_grad2d);
   w.grad2d_tag = c.take<unsigned long long>(1);  // here for callers who clear it (dsplat.h)
   w.touched = c.take<uint32_t>((VN + 3) / 4);
@@ -746,7 +750,7 @@ int dsplat_gauss_batch_forward(dsplat_stream stream, const dsplat_gauss_params* 
   stage_mark(st, 4);
   const FwdArgs fa{n,           w.rec,   w.lists.list1, w.lists.off1, w.L.sb_chunks, pair_capacity, w.task_order, w.sched,
                    w.flags + 2, out_rgb, w.pix_T,       w.pix_stop,   target,        w.grad_pix,    w.slab_loss,
-                   w.item_cost, out_alpha};
+                   w.unit_loss, w.item_cost, out_alpha};
   TRY_CUDA(raster_fwd(st, b, fa),
            "raster_fwd");
   stage_mark(st, 5);

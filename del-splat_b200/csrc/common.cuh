@@ -67,6 +67,7 @@ struct FwdArgs {
   const float* target;
   float* grad_pix;
   float* slab_loss;
+  float* unit_loss;  // of tiles above 8x8
   uint32_t* item_cost;
   float* out_alpha;
 };

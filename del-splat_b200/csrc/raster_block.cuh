@@ -167,9 +167,10 @@ struct FwdOut {  // where a block's results go
 };
 
 // ent, park (T, r, g, b of a stopped pixel) and park_pos (its stop position),
-// 32, 64 and 64 of them, are the warp's in shared memory; loss(l) takes the
-// block's partial L2 loss (lane 0).
-template <bool CUDA_STOP, class Walk, class Src, class Loss>
+// 32, 64 and 64 of them, are the warp's in shared memory; loss(k, l) takes the
+// L2 loss of the block's loss unit k (one, or an upper and a lower half: see
+// loss_rows in raster_fwd.cu).
+template <bool CUDA_STOP, int LOSS_ROWS, class Walk, class Src, class Loss>
 __device__ __forceinline__ uint32_t blend_block(const Walk& walk, const Src& src, EntB* ent_sm, float4* park,
                                               uint32_t* park_pos, const float* tab, float nz,
                                               uint32_t s, uint32_t e, int px0, int py0, int w, int xend, int yend,
@@ -314,7 +315,7 @@ __device__ __forceinline__ uint32_t blend_block(const Walk& walk, const Src& src
     park[32 + lane] = make_float4(f2_hi(T2), f2_hi(c0), f2_hi(c1), f2_hi(c2));
     park_pos[32 + lane] = s;
   }
-  float l = 0.f;
+  float l[2] = {0.f, 0.f};
 #pragma unroll
   for (int k = 0; k < 2; ++k) {
     if (!(k ? in1 : in0)) continue;
@@ -331,13 +332,18 @@ __device__ __forceinline__ uint32_t blend_block(const Walk& walk, const Src& src
       out.grad_pix[3 * p] = 2.f * d0;
       out.grad_pix[3 * p + 1] = 2.f * d1;
       out.grad_pix[3 * p + 2] = 2.f * d2;
-      l += d0 * d0 + d1 * d1 + d2 * d2;
+      l[k] = d0 * d0 + d1 * d1 + d2 * d2;
     }
   }
   if (out.target) {
+    constexpr int units = 8 / LOSS_ROWS;
+    if (units == 1) l[0] += l[1];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-    if (lane == 0) loss(l);
+    for (int k = 0; k < units; ++k) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) l[k] += __shfl_xor_sync(0xffffffffu, l[k], o);
+      if (lane == 0) loss(k, l[k]);
+    }
   }
   __syncwarp();
   return cost;

@@ -16,6 +16,11 @@ namespace dsplat {
 
 uint32_t raster_slabs_per_tile(int ts, int ppl);
 
+// The L2 loss is summed in units of 8 columns and as many rows, 8 or, where a
+// slab has only four, 4, in the same order of pixels in a slab as in an 8x8
+// block, so that its bits do not depend on the shape an item is walked in.
+__host__ __device__ constexpr int loss_rows(int slab_rows) { return slab_rows < 8 ? slab_rows : 8; }
+
 // ---------------------------------------------------------------------------
 // Forward walk of one slab by one warp over the list range [s, e).  Slot k of
 // every lane lies in the same row pair of the slab, so the per-slot skips
@@ -211,7 +216,7 @@ __device__ __forceinline__ uint32_t fwd_slab(const Walk& walk, const Src& src, E
       park_pos[(2 * q + 1) * 32 + lane] = s;
     }
   }
-  float l = 0.f;
+  float l[PPL] = {};
 #pragma unroll
   for (int k = 0; k < PPL; ++k) {
     if (!((inside >> k) & 1u)) continue;
@@ -228,13 +233,42 @@ __device__ __forceinline__ uint32_t fwd_slab(const Walk& walk, const Src& src, E
       grad_pix[3 * p] = 2.f * d0;
       grad_pix[3 * p + 1] = 2.f * d1;
       grad_pix[3 * p + 2] = 2.f * d2;
-      l += d0 * d0 + d1 * d1 + d2 * d2;
+      l[k] = d0 * d0 + d1 * d1 + d2 * d2;
     }
   }
-  if (target) {
+  if (target) {  // the loss units, each summed in a block's order
+    constexpr int ROWS = loss_rows(G::SLAB_ROWS);
+    if (SPLIT) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-    if (lane == 0) loss(l);
+      for (int q = 0; q < 2; ++q) {
+        float v = l[2 * q] + l[2 * q + 1];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (lane == 0) loss(q, v);
+      }
+    } else {
+      constexpr int SLOTS = ROWS / G::ROW_STEP;  // of a unit
+#pragma unroll
+      for (int u = 0; u < PPL / SLOTS; ++u) {
+        // row r and, in a unit of 8, r + 4; then r ^ 2, r ^ 1 and the columns
+        float v[4 / G::ROW_STEP];
+#pragma unroll
+        for (int k = 0; k < 4 / G::ROW_STEP; ++k) {
+          v[k] = l[u * SLOTS + k];
+          if (ROWS == 8) v[k] += l[u * SLOTS + k + 4 / G::ROW_STEP];
+        }
+        float sum;
+        if (G::ROW_STEP == 1) {
+          sum = (v[0] + v[2 % (4 / G::ROW_STEP)]) + (v[1] + v[3 % (4 / G::ROW_STEP)]);
+        } else {
+          sum = v[0] + v[1];
+          sum += __shfl_xor_sync(0xffffffffu, sum, 16);
+        }
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if (lane % 8 == 0 && lane < TS) loss(u * (TS / 8) + lane / 8, sum);
+      }
+    }
   }
   return cost;
 }
@@ -249,8 +283,8 @@ constexpr float kLargeLoss = 0.25f * kBwdLarge * kBwdLarge;
 // the order are walked in 8x8 blocks (raster_block.cuh), the others in tasks
 // of TaskGeo.  No block count is asked of the compiler: it takes 80 registers
 // by itself (6 blocks of 4 warps per SM), and 10% more instructions when told
-// to (16 views of 1,048,576 Gaussians 2890 -> 3210 us).  slab_loss: `slots` partial L2 losses per tile (when target is
-// given; zero at the start where a tile's blocks do not match its slots).
+// to (16 views of 1,048,576 Gaussians 2890 -> 3210 us).  unit_loss: the items'
+// loss units, row by row in a tile, those inside the view.
 // ---------------------------------------------------------------------------
 template <int TS, int PPL, int NT>
 __global__ void __launch_bounds__(32 * kRasterWarps) k_raster_fwd(
@@ -258,7 +292,7 @@ __global__ void __launch_bounds__(32 * kRasterWarps) k_raster_fwd(
     const uint32_t* __restrict__ off1, uint32_t nchunk, uint64_t capacity, const uint32_t* __restrict__ order,
     uint32_t* __restrict__ sched, uint32_t* __restrict__ work_counter, float* __restrict__ out_rgb,
     float* __restrict__ out_T, float* __restrict__ out_alpha, uint32_t* __restrict__ out_last,
-    const float* __restrict__ target, float* __restrict__ grad_pix, float* __restrict__ slab_loss, uint32_t slots, uint32_t* __restrict__ item_cost,
+    const float* __restrict__ target, float* __restrict__ grad_pix, float* __restrict__ unit_loss, uint32_t* __restrict__ item_cost,
     float nz) {
   using G = TaskGeo<TS, PPL, NT>;
   static_assert(sizeof(EntB) >= sizeof(EntP), "the warps' entries of either form share their place");
@@ -286,37 +320,34 @@ __global__ void __launch_bounds__(32 * kRasterWarps) k_raster_fwd(
       nx = min(uint32_t(NT), 1u << vd.sb_log2);
       if (ig.lx % nx) continue;
     }
+    // unit u of a tile of the run
+    constexpr int ROWS = loss_rows(G::SLAB_ROWS), UNITS = TS * TS / (8 * ROWS);
+    auto loss = [&](uint32_t tile, uint32_t u, float l) {
+      unit_loss[size_t(t.item + tile) * UNITS + u] = l;
+      if (!(l <= kLargeLoss)) sched[kSchedOdd] = 1u;
+    };
     uint32_t cost;
     if (t.block) {
+      auto block_loss = [&](int k, float l) {
+        constexpr uint32_t SIDE = TS / 8;
+        if (TS == 8) loss(t.sub, k, l);
+        else loss(0, ROWS == 8 ? t.sub : (2 * (t.sub / SIDE) + k) * SIDE + t.sub % SIDE, l);
+      };
       BlockPlace p;
-      if (!block_place(b, ig, t.sub, nx, &p)) {
-        // a block of a larger tile outside the view: its slot of the tile is
-        // its own where a tile has as many slots as blocks
-        if (TS > 8 && target && lane == 0 && slots == TS * TS / 64) slab_loss[size_t(t.item) * slots + t.sub] = 0.f;
-        continue;
-      }
+      if (!block_place(b, ig, t.sub, nx, &p)) continue;
       const FwdOut out{out_rgb, out_T, out_alpha, out_last, target, grad_pix};
-      cost = blend_block<false>(SbWords{list1, p.lx, ig.ly, 1u}, PackedBlockSrc{src.rec}, ent, park, park_pos, tab, nz,
-                                ig.s, ig.e, p.px0, p.py0, vd.w, vd.w, vd.h, false, vd.pix_base, out, [&](float l) {
-                                  if (!(l <= kLargeLoss)) sched[kSchedOdd] = 1u;
-                                  float* const p0 = slab_loss + size_t(t.item) * slots;
-                                  constexpr uint32_t blocks = TS * TS / 64;
-                                  if (TS == 8) p0[t.sub * slots] = l;  // the run's tile t.sub
-                                  else if (slots < blocks) atomicAdd(p0 + t.sub * slots / blocks, l);
-                                  else p0[t.sub * (slots / blocks)] = l;
-                                });
+      cost = blend_block<false, ROWS>(SbWords{list1, p.lx, ig.ly, 1u}, PackedBlockSrc{src.rec}, ent, park, park_pos, tab, nz,
+                                      ig.s, ig.e, p.px0, p.py0, vd.w, vd.w, vd.h, false, vd.pix_base, out, block_loss);
     } else {
       SbWalkSpan walk{list1, ig.lx, ig.ly, nx};
       const int xend = min(vd.w, ig.px0 + int(nx) * TS);
       cost = fwd_slab<G::GX, G::PPL, NT == 2 && G::PPL == 4>(
           walk, src, reinterpret_cast<EntP*>(ent), park, park_pos, tab, nz, ig.s, ig.e, ig.px0,
           ig.py0 + int(t.sub) * G::SLAB_ROWS, vd.w, vd.h, xend, out_rgb, vd.pix_base, out_T, out_alpha, out_last, target,
-          grad_pix, [&](float l) {
-            if (!(l <= kLargeLoss)) sched[kSchedOdd] = 1u;
-            float* const p0 = slab_loss + size_t(t.item) * G::SLABS + t.sub;
-            *p0 = l;
-            // the run's other tile has its loss in the leftmost one's slot
-            if (NT > 1 && vd.sb_log2 > 0 && ig.px0 + 8 < vd.w) p0[G::SLABS] = 0.f;
+          grad_pix, [&](int k, float l) {
+            constexpr uint32_t PER_SLAB = UNITS / G::SLABS;
+            if (TS > 8) loss(0, t.sub * PER_SLAB + k, l);
+            else if (ig.px0 + 8 * k < xend) loss(k, t.sub, l);
           });
     }
     // scheduling hint for the backward and the next forward
@@ -345,23 +376,47 @@ __global__ void __launch_bounds__(32 * kRasterWarps, 6) k_raster_fwd_aos(
   const int py0 = int(tile / uint32_t(tile_w)) * ts + int(blk / side) * kBlock;
   if (px0 >= w || py0 >= h) return;
   const FwdOut out{pix2rgb, out_T, nullptr, out_last, nullptr, nullptr};
-  blend_block<CUDA_STOP>(TileWords{idx2pnt}, src, ent[warp], park[warp], park_pos[warp], tab, nz, tile2idx[tile],
-                         tile2idx[tile + 1], px0, py0, w, w, h, true, 0, out, [](float) {});
+  blend_block<CUDA_STOP, 8>(TileWords{idx2pnt}, src, ent[warp], park[warp], park_pos[warp], tab, nz, tile2idx[tile],
+                         tile2idx[tile + 1], px0, py0, w, w, h, true, 0, out, [](int, float) {});
+}
+
+// Units of a tile's slab (8x8 tiles: the slabs' slots are the units').
+uint32_t loss_units_per_slab(int ts, int ppl) {
+  const int slab_rows = ts == 8 ? 4 * ppl : 32 * ppl / ts;
+  return uint32_t(ts / 8 * (slab_rows / loss_rows(slab_rows)));
+}
+
+// A slab's loss: its units' in order, those outside the view (not written by
+// blocks) left out.
+__global__ void __launch_bounds__(256) k_slab_loss(const ViewBatch b, const float* __restrict__ unit_loss, int slab_rows,
+                                                   float* __restrict__ slab_loss) {
+  const uint32_t slabs = uint32_t(b.ts / slab_rows), i = blockIdx.x * 256u + threadIdx.x;
+  if (i >= b.num_items * slabs) return;
+  const uint32_t item = i / slabs;
+  const ViewDev& vd = b.v[view_of_item(b, item)];
+  const uint32_t t = item - vd.item_base;
+  const int px0 = int(t % uint32_t(vd.tile_w)) * b.ts, py0 = int(t / uint32_t(vd.tile_w)) * b.ts + int(i % slabs) * slab_rows;
+  const int rows = loss_rows(slab_rows), cols = b.ts / 8, units = cols * (slab_rows / rows);
+  float sum = 0.f;
+  for (int k = 0; k < units; ++k)
+    if (px0 + 8 * (k % cols) < vd.w && py0 + rows * (k / cols) < vd.h) sum += unit_loss[size_t(i) * units + k];
+  slab_loss[i] = sum;
 }
 
 template <int TS, int PPL>
 static cudaError_t launch_fwd(cudaStream_t st, const ViewBatch& b, const FwdArgs& a) {
   constexpr int NT = TS == 8 ? kFwdGroup8 : 1;
-  const uint32_t slots = raster_slabs_per_tile(TS, PPL);
-  if (a.target && slots != uint32_t(TS * TS / 64)) {
-    const cudaError_t e = cudaMemsetAsync(a.slab_loss, 0, size_t(b.num_items) * slots * sizeof(float), st);
-    if (e != cudaSuccess) return e;
-  }
   k_raster_fwd<TS, PPL, NT>
       <<<persistent_grid(k_raster_fwd<TS, PPL, NT>, max_tasks(b, TaskGeo<TS, PPL, NT>::SLABS)), 32 * kRasterWarps, 0,
          st>>>(b, a.n, a.rec, a.list1, a.off1, a.nchunk, a.capacity, a.order, a.sched, a.counter, a.out_rgb, a.out_T,
-               a.out_alpha, a.out_last, a.target, a.grad_pix, a.slab_loss, slots, a.item_cost, -0.f);
+               a.out_alpha, a.out_last, a.target, a.grad_pix, TS == 8 ? a.slab_loss : a.unit_loss, a.item_cost, -0.f);
   count_launch();
+  if (TS > 8 && a.target) {
+    constexpr int SLAB_ROWS = TaskGeo<TS, PPL, NT>::SLAB_ROWS;
+    const uint32_t slabs = b.num_items * uint32_t(TS / SLAB_ROWS);
+    k_slab_loss<<<(slabs + 255) / 256, 256, 0, st>>>(b, a.unit_loss, SLAB_ROWS, a.slab_loss);
+    count_launch();
+  }
   return cudaGetLastError();
 }
 

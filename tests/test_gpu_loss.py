@@ -34,3 +34,16 @@ def test_every_slot_is_written(dev, size, ts, ppl):
         assert heavy_items(batch) == int((blocks & leaders(batch)).sum())
         want = float(((batch.out_rgb.double() - target.double()) ** 2).sum())
         assert abs(float(batch.slab_loss().double().sum()) - want) <= 1e-5 * want
+
+
+@pytest.mark.parametrize("ts,ppl", CONFIGS)
+def test_loss_does_not_depend_on_the_schedule(dev, ts, ppl):
+    """The same bits in every slot, whichever items are walked in blocks."""
+    batch, p, target = _batch(dev, (133, 94), ts, ppl)
+    seen = []
+    for k in range(6):
+        set_blocks(batch, masks(batch)[k % 2])
+        batch.forward(p, target=target)
+        seen.append(F(batch.slab_loss()).view(np.uint32).copy())
+    for s in seen[1:]:
+        assert np.array_equal(s, seen[0])
