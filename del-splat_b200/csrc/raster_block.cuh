@@ -126,27 +126,30 @@ struct PackedBlockSrc {
 
 // List words of the two forms of tile lists: load() reads a lane's word ahead
 // of time, point() and hit() are its point and whether its entry lies in the
-// task's tiles.
+// block's tile, counts() whether a whole task of the item would stage it.
 struct TileWords {  // a per-tile list (tile2idx / idx2pnt)
   typedef uint32_t word;
   const uint32_t* idx2pnt;
   __device__ __forceinline__ word load(uint32_t pos) const { return idx2pnt[pos]; }
   static __device__ __forceinline__ uint32_t point(word w) { return w; }
   __device__ __forceinline__ bool hit(word) const { return true; }
+  __device__ __forceinline__ bool counts(word) const { return true; }
 };
 
-// A superblock list filtered to the tiles lx .. lx+nx-1 of one superblock
-// row: an entry is kept if its span meets any of them.
+// A superblock list filtered to the block's tile (lx, ly); the item's tasks
+// take the nx tiles from run on.
 struct SbWords {
   typedef uint2 word;
   const uint2* list1;
-  uint32_t lx, ly, nx;
+  uint32_t lx, ly, run, nx;
   __device__ __forceinline__ word load(uint32_t pos) const { return list1[pos]; }
   static __device__ __forceinline__ uint32_t point(word w) { return w.x; }
-  __device__ __forceinline__ bool hit(word w) const {
+  __device__ __forceinline__ bool meets(word w, uint32_t x, uint32_t n) const {
     const uint32_t lr = w.y;
-    return lx < ((lr >> 8) & 15u) && lx + nx > (lr & 15u) && ly >= ((lr >> 4) & 15u) && ly < (lr >> 12);
+    return x < ((lr >> 8) & 15u) && x + n > (lr & 15u) && ly >= ((lr >> 4) & 15u) && ly < (lr >> 12);
   }
+  __device__ __forceinline__ bool hit(word w) const { return meets(w, lx, 1u); }
+  __device__ __forceinline__ bool counts(word w) const { return meets(w, run, nx); }
 };
 
 // ---------------------------------------------------------------------------
@@ -155,7 +158,10 @@ struct SbWords {
 // packed pair.
 // CUDA_STOP: the stop test of the reference's CUDA kernel (alpha_sum >=
 // 0.999f, its double comparison) instead of del-splat-cpu's (> 0.999f).
-// Returns the cost of the walk (in units of a few warp-instructions).
+// Returns the cost of the walk in a whole task's measure (kCostBatch and
+// kCostEntry for what such a task would stage), so that an item's cost, the
+// largest of its tasks' or blocks', is the same in either shape and the schedule
+// of the same inputs does not swing between the two.
 // ---------------------------------------------------------------------------
 struct FwdOut {  // where a block's results go
   float* rgb;
@@ -230,6 +236,7 @@ __device__ __forceinline__ uint32_t blend_block(const Walk& walk, const Src& src
     const uint32_t cnt = min(32u, hi - s);
     // stage the batch's entries that hold a pixel of the block, in order
     bool hit = uint32_t(lane) < cnt && walk.hit(en);
+    const uint32_t counted = __ballot_sync(0xffffffffu, uint32_t(lane) < cnt && walk.counts(en));
     const uint32_t g = walk.point(en);
     uint2 mask = make_uint2(0u, 0u);
     if (hit) {
@@ -242,7 +249,7 @@ __device__ __forceinline__ uint32_t blend_block(const Walk& walk, const Src& src
     if (hit) odd = src.stage(&ent_sm[__popc(bal & (bit - 1u))], g, hi - 1u - uint32_t(lane), mask);
     const bool odd_colour = __any_sync(0xffffffffu, odd);
     hi -= cnt;
-    cost += kCostBatch + uint32_t(staged) * kCostEntry;
+    cost += kCostBatch + uint32_t(__popc(counted)) * kCostEntry;
     // the next batch's list words arrive while this batch is blended
     if (hi > s && uint32_t(lane) < hi - s) en = walk.load(hi - 1u - uint32_t(lane));
     __syncwarp();

@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(32 * kRasterWarps) k_raster_fwd(
       BlockPlace p;
       if (!block_place(b, ig, t.sub, nx, &p)) continue;
       const FwdOut out{out_rgb, out_T, out_alpha, out_last, target, grad_pix};
-      cost = blend_block<false, ROWS>(SbWords{list1, p.lx, ig.ly, 1u}, PackedBlockSrc{src.rec}, ent, park, park_pos, tab, nz,
+      cost = blend_block<false, ROWS>(SbWords{list1, p.lx, ig.ly, ig.lx, nx}, PackedBlockSrc{src.rec}, ent, park, park_pos, tab, nz,
                                       ig.s, ig.e, p.px0, p.py0, vd.w, vd.w, vd.h, false, vd.pix_base, out, block_loss);
     } else {
       SbWalkSpan walk{list1, ig.lx, ig.ly, nx};
