@@ -364,12 +364,11 @@ uint32_t raster_slabs_per_tile(int ts, int ppl) { return uint32_t(ts * ts / (32 
 template <int TS, int PPL>
 static cudaError_t launch_bwd(cudaStream_t st, const ViewBatch& b, const BwdArgs& a) {
   constexpr int NT = TS == 8 ? kBwdGroup8 : 1;
-  const uint32_t units = max_tasks(b, TaskGeo<TS, PPL, NT>::SLABS);
-#define X(CAREFUL)                                                                                                    \
-  k_raster_bwd<TS, PPL, NT, CAREFUL><<<persistent_grid(k_raster_bwd<TS, PPL, NT, CAREFUL>, units), 32 * kRasterWarps, \
-                                       0, st>>>(b, a.n, a.rec, a.list1, a.off1, a.nchunk, a.capacity, a.order,        \
-                                                a.sched, a.counter, a.grad_pix, a.pix_T, a.pix_last, a.grad2d,        \
-                                                a.touched);                                                           \
+  const int grid = persistent_grid(k_raster_bwd<TS, PPL, NT, false>, max_tasks(b, TaskGeo<TS, PPL, NT>::SLABS));
+#define X(CAREFUL)                                                                                                  \
+  k_raster_bwd<TS, PPL, NT, CAREFUL><<<grid, 32 * kRasterWarps, 0, st>>>(                                           \
+      b, a.n, a.rec, a.list1, a.off1, a.nchunk, a.capacity, a.order, a.sched, a.counter, a.grad_pix, a.pix_T,       \
+      a.pix_last, a.grad2d, a.touched);                                                                             \
   count_launch();
   X(false) X(true)
 #undef X
