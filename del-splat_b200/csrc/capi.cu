@@ -57,8 +57,10 @@ bool raster_config_ok(int ts, int ppl);
 int raster_default_ppl(int ts);
 uint32_t raster_slabs_per_tile(int ts, int ppl);
 uint32_t loss_units_per_slab(int ts, int ppl);
-__global__ void k_order_hist(const ViewBatch, const uint32_t*, uint32_t, const uint32_t*, uint32_t*);
-__global__ void k_order_scatter(const ViewBatch, const uint32_t*, uint32_t, uint32_t*, float, uint32_t*, uint32_t*);
+__global__ void k_order_hist(const ViewBatch, const uint32_t*, uint32_t, const uint32_t*, const unsigned long long*,
+                             unsigned long long, uint32_t*);
+__global__ void k_order_scatter(const ViewBatch, const uint32_t*, uint32_t, uint32_t*, unsigned long long*,
+                                unsigned long long, float, uint32_t*, uint32_t*);
 cudaError_t raster_fwd_aos(cudaStream_t, int, int, int, float*, const float*, const float*, const float*, const float*,
                            const float*, const uint32_t*, const uint32_t*, float*, uint32_t*, bool);
 cudaError_t expf_cr_launch(cudaStream_t, size_t, const float*, float*);
@@ -224,12 +226,13 @@ int build_tile_lists(cudaStream_t st, const ViewBatch& b, uint32_t npad, const L
 constexpr float kHeavyShare = 148.f * 64.f;
 
 cudaError_t order_tasks(cudaStream_t st, const ViewBatch& b, const uint32_t* off1, uint32_t nchunk,
-                        uint32_t* cost, uint32_t* sched, uint32_t* order) {
+                        uint32_t* cost, unsigned long long* cost_tag, unsigned long long tag, uint32_t* sched,
+                        uint32_t* order) {
   // costs are those of an item's longest task; its tasks share the total
   const float share = kHeavyShare / float(b.ts == 8 ? 1u : raster_slabs_per_tile(b.ts, b.ppl));
-  k_order_hist<<<296, 256, 0, st>>>(b, off1, nchunk, cost, sched);
+  k_order_hist<<<296, 256, 0, st>>>(b, off1, nchunk, cost, cost_tag, tag, sched);
   count_launch();
-  k_order_scatter<<<296, 256, 0, st>>>(b, off1, nchunk, cost, share, sched, order);
+  k_order_scatter<<<296, 256, 0, st>>>(b, off1, nchunk, cost, cost_tag, tag, share, sched, order);
   count_launch();
   return cudaGetLastError();
 }
@@ -406,8 +409,9 @@ struct BatchWs {
   float* slab_loss;
   float* unit_loss;  // slab_loss's parts (tiles above 8x8)
   float4* grad2d;
-  unsigned long long* grad2d_tag;  // == grad2d_tag_value(): grad2d and touched are all zero
+  unsigned long long* grad2d_tag;  // == layout_tag(): grad2d and touched are all zero
   uint32_t* touched;  // a byte per grad2d record
+  unsigned long long* cost_tag;  // == layout_tag(): item_cost was measured by a forward
   uint32_t *sched, *task_order, *item_cost;
 };
 
@@ -449,10 +453,11 @@ int make_batch(int64_t n64, int32_t nv, const dsplat_view* views, int32_t ts, in
   return DSPLAT_OK;
 }
 
-// Value of the workspace's grad2d tag meaning "grad2d is all zero for this
-// layout": a fixed pattern mixed with the layout, so that a fresh workspace
-// or one carved for another batch is cleared before use.
-unsigned long long grad2d_tag_value(const dsplat_batch_layout& L, uint32_t n, int32_t views) {
+// Value of the workspace's marks, "grad2d is all zero for this layout" and "the
+// item costs are those of a forward of it": a fixed pattern mixed with the
+// layout, so that a fresh workspace or one carved for another batch holds
+// neither.
+unsigned long long layout_tag(const dsplat_batch_layout& L, uint32_t n, int32_t views) {
   unsigned long long h = 0x6a09e667f3bcc909ull;
   const unsigned long long parts[4] = {L.total_bytes, L.off_grad2d, n, uint64_t(uint32_t(views))};
   for (unsigned long long x : parts) {
@@ -503,6 +508,7 @@ BatchWs carve_batch(void* ws, uint32_t n, const ViewBatch& b, uint64_t capacity)
   w.grad2d = c.take<float4>(3 * VN + 3, &L.off_grad2d);
   w.grad2d_tag = c.take<unsigned long long>(1);  // here for callers who clear it (dsplat.h)
   w.touched = c.take<uint32_t>((VN + 3) / 4);
+  w.cost_tag = c.take<unsigned long long>(1);
   w.task_order = c.take<uint32_t>(size_t(b.num_items) + 1);
   w.item_cost = c.take<uint32_t>(size_t(b.num_items) + 1);
   L.total_bytes = align_up(c.off, 256);
@@ -745,7 +751,8 @@ int dsplat_gauss_batch_forward(dsplat_stream stream, const dsplat_gauss_params* 
     stage_mark(st, 3);
   }
   // longest-first raster task order (costs measured by the previous forward)
-  TRY_CUDA(order_tasks(st, b, w.lists.off1, w.L.sb_chunks, w.item_cost, w.sched, w.task_order),
+  TRY_CUDA(order_tasks(st, b, w.lists.off1, w.L.sb_chunks, w.item_cost, w.cost_tag, layout_tag(w.L, n, num_views), w.sched,
+                       w.task_order),
            "task order");
   stage_mark(st, 4);
   const FwdArgs fa{n,           w.rec,   w.lists.list1, w.lists.off1, w.L.sb_chunks, pair_capacity, w.task_order, w.sched,
@@ -780,7 +787,7 @@ int dsplat_gauss_batch_backward(dsplat_stream stream, const dsplat_gauss_params*
   stage_mark(st, 6);
   // grad2d must start at zero; the projection backward zeroes what it
   // consumes, so only a buffer not known to be clean is cleared here
-  const unsigned long long tag = grad2d_tag_value(w.L, n, num_views);
+  const unsigned long long tag = layout_tag(w.L, n, num_views);
   k_prepare_grad2d<<<blocks_for(3 * VN, 256) < 4096 ? blocks_for(3 * VN, 256) : 4096, 256, 0, st>>>(
       w.grad2d_tag, tag, w.grad2d, 3 * VN, w.touched, (VN + 3) / 4, w.flags + 3, grad_rgb, size_t(b.num_pix) * 3,
       w.sched + kSchedOdd);

@@ -95,6 +95,7 @@ struct BwdArgs {
 // cursors [40, 73), and
 constexpr int kSchedCost = 74;   // u64: sum of the items' costs
 constexpr int kSchedHeavy = 76;  // leading items of the order walked in 8x8 blocks
+constexpr int kSchedMeasured = 78;  // not 0: the items' costs are a forward's, not what the memory held before
 constexpr int kSchedOdd = 77;    // not 0: the batch has something odd (see kBwdLarge)
 constexpr int kSchedWords = 80;
 

@@ -863,8 +863,9 @@ cudaError_t sb_scatter_staged(cudaStream_t st, unsigned grid, const uint32_t* or
 // of their cost, heaviest bucket first, so the tail of the persistent launch
 // is made of short tasks.  The cost is that of the item's longest walk in the
 // last forward (measured, kept in the workspace) or, where none is recorded
-// yet, its superblock-list length.  Only the schedule depends on it, never
-// the results.  sched: see kSchedCost in common.cuh.
+// yet, its superblock-list length; the workspace's mark (*cost_tag == tag) says
+// whether a forward of this layout has measured at all.  Only the schedule
+// depends on it, never the results.  sched: see kSchedCost in common.cuh.
 //
 // Heavy items: a task whose cost is a good part of what every resident warp
 // has to do (total / warps) ends after the others, and the GPU waits for it
@@ -873,7 +874,7 @@ cudaError_t sb_scatter_staged(cudaStream_t st, unsigned grid, const uint32_t* or
 // blocks (about 15% more instructions, so short tasks stay whole).
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t item_cost(const ViewBatch& b, uint32_t item, const uint32_t* off1, uint32_t nchunk,
-                                              const uint32_t* cost) {
+                                              const uint32_t* cost, bool measured) {
   int v = 0;
   for (int k = 1; k < b.num_views; ++k)
     if (item >= b.v[k].item_base) v = k;
@@ -882,20 +883,23 @@ __device__ __forceinline__ uint32_t item_cost(const ViewBatch& b, uint32_t item,
   const uint32_t tx = t % uint32_t(vd.tile_w), ty = t / uint32_t(vd.tile_w);
   // 8x8 tiles: the leftmost tile of a run carries the task of both
   if (b.ts == 8 && tx % min(2u, 1u << vd.sb_log2)) return 0u;
-  const uint32_t measured = cost[item];
-  if (measured) return measured;
+  const uint32_t c = measured ? cost[item] : 0u;
+  if (c) return c;
   const uint32_t sb = vd.sb_base + (ty >> vd.sb_log2) * uint32_t(sb_cols(vd)) + (tx >> vd.sb_log2);
   return off1[size_t(sb + 1) * nchunk] - off1[size_t(sb) * nchunk];
 }
 
 __global__ void k_order_hist(const ViewBatch b, const uint32_t* __restrict__ off1, uint32_t nchunk,
-                             const uint32_t* __restrict__ cost, uint32_t* __restrict__ sched) {
+                             const uint32_t* __restrict__ cost, const unsigned long long* __restrict__ cost_tag,
+                             unsigned long long tag, uint32_t* __restrict__ sched) {
   __shared__ uint32_t h[33];
+  const bool measured = *cost_tag == tag;
+  if (blockIdx.x == 0 && threadIdx.x == 0) sched[kSchedMeasured] = measured;
   if (threadIdx.x < 33) h[threadIdx.x] = 0;
   __syncthreads();
   unsigned long long sum = 0;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < b.num_items; i += gridDim.x * blockDim.x) {
-    const uint32_t c = item_cost(b, i, off1, nchunk, cost);
+    const uint32_t c = item_cost(b, i, off1, nchunk, cost, measured);
     atomicAdd(&h[__clz(c)], 1u);
     sum += c;
   }
@@ -911,10 +915,13 @@ __global__ void k_order_hist(const ViewBatch b, const uint32_t* __restrict__ off
 // bucket and block instead of one per item on 33 hot counters); every block
 // forms the buckets' starts from the counts itself.  heavy_share: an item
 // is heavy when its cost times that is above the total cost.
-// The costs are set to zero for the next forward to measure.
+// The costs are set to zero for this forward to measure, and marked as its.
 __global__ void k_order_scatter(const ViewBatch b, const uint32_t* __restrict__ off1, uint32_t nchunk,
-                                uint32_t* __restrict__ cost, float heavy_share, uint32_t* __restrict__ sched,
+                                uint32_t* __restrict__ cost, unsigned long long* __restrict__ cost_tag,
+                                unsigned long long tag, float heavy_share, uint32_t* __restrict__ sched,
                                 uint32_t* __restrict__ order) {
+  const bool measured = sched[kSchedMeasured] != 0u;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *cost_tag = tag;
   __shared__ uint32_t cnt[33], base[33], start[33];
   if (threadIdx.x == 0) {
     const float total = float(*reinterpret_cast<const unsigned long long*>(sched + kSchedCost));
@@ -936,7 +943,7 @@ __global__ void k_order_scatter(const ViewBatch b, const uint32_t* __restrict__ 
     const uint32_t i = i0 + threadIdx.x;
     uint32_t bucket = 0, slot = 0;
     if (i < hi) {
-      bucket = uint32_t(__clz(item_cost(b, i, off1, nchunk, cost)));
+      bucket = uint32_t(__clz(item_cost(b, i, off1, nchunk, cost, measured)));
       cost[i] = 0u;
       slot = atomicAdd(&cnt[bucket], 1u);
     }

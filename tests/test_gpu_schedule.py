@@ -25,3 +25,19 @@ def test_measured_cost_does_not_depend_on_the_shape(dev, ts, ppl):
         costs.append(F(item_cost(batch)).copy())
     assert costs[0].max() > 0
     assert np.array_equal(*costs)
+
+
+def test_first_forward_on_a_workspace_ignores_what_it_held(dev):
+    """The items' costs count once a forward has measured them: on a workspace
+    full of anything else the schedule is that of the list lengths."""
+    sc = scenes.config0(seed=8, n=1500, size=(1297, 1013))  # about 10,000 items that lead a task
+    p = params_of(sc, dev)
+    heavy = []
+    for fill in (0, 0xff, 0x01):
+        batch = GaussBatch(sc.n, sc.cameras, 8, -1, pair_capacity=1 << 18, device=dev)
+        batch.ws.fill_(fill)
+        batch.forward(p)
+        heavy.append(heavy_items(batch))
+        assert batch.status()[0] == 0
+    assert 0 < heavy[0] < int(batch.layout.num_items)
+    assert heavy == [heavy[0]] * 3
