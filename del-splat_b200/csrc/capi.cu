@@ -169,6 +169,11 @@ void carve_lists(Carver& c, const ViewBatch& b, uint32_t npad, size_t cap, Lists
   L->tcnt = c.take<uint32_t>(size_t(b.num_items) + 1);
 }
 
+// Most shared memory of the two superblock scatters' blocks.  A kernel's limit
+// is the process's: every call sets the same value, so that no call lowers it
+// between another thread's setting and its launch.
+constexpr int kSbScatterMost = 200 * 1024;
+
 // Stage 1: superblock lists of (point, local tile span) in rank order.
 // flags[6..7] <- tile pairs P (u64), flags[8..9] <- superblock entries
 // (capacity needed, u64); flags[0] |= overflow when they exceed capacity.
@@ -179,19 +184,17 @@ int build_sb_lists(cudaStream_t st, const ViewBatch& b, uint32_t n, uint32_t npa
   const unsigned grid1 = unsigned(b.num_views) * nchunk;
   const size_t smem1 = size_t(b.max_sb) * sizeof(uint32_t);
   const size_t smem3 = 8 * smem1 + 8 * 2 * size_t(b.max_sb_side) * sizeof(uint32_t);
-  if (smem3 > 48 * 1024) {
-    if (smem3 > 200 * 1024) return fail(DSPLAT_ERR_UNSUPPORTED, "too many superblocks in one view");
-    TRY_CUDA(cudaFuncSetAttribute(k_sb_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem3)), "attr");
-  }
+  if (smem3 > kSbScatterMost) return fail(DSPLAT_ERR_UNSUPPORTED, "too many superblocks in one view");
   unsigned long long* totals = reinterpret_cast<unsigned long long*>(flags + 6);
   k_sb_count<<<grid1, 256, smem1, st>>>(order, srect, npad / nchunk, npad, b, L.cnt1, totals);
   count_launch();
   TRY_CUDA(exclusive_scan(st, L.cnt1, L.off1, m, scan_tmp, 0xffffffffu, nullptr), "scan");
   // staged scatter (coalesced list stores) when its shared memory fits
-  if (sb_scatter_staged_smem(b.max_sb) <= 100 * 1024) {
+  if (sb_scatter_staged_smem(b.max_sb) <= kSbStagedMost) {
     TRY_CUDA(sb_scatter_staged(st, grid1, order, srect, npad / nchunk, npad, b, L.off1, capacity, L.list1, flags),
              "superblock scatter");
   } else {
+    TRY_CUDA(cudaFuncSetAttribute(k_sb_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, kSbScatterMost), "attr");
     k_sb_scatter<<<grid1, 256, smem3, st>>>(order, srect, npad / nchunk, npad, b, L.off1, capacity, L.list1, flags);
     count_launch();
   }

@@ -114,6 +114,10 @@ __device__ __forceinline__ bool odd_record(const float* conic, float hx, float h
            fabsf(rgb[2]) <= kBwdLarge);
 }
 
+// Most shared memory of the staged superblock scatter's blocks (three to an SM
+// up to 75 KB); views that would need more take the unstaged one.
+constexpr int kSbStagedMost = 100 * 1024;
+
 // The five parameter tensors of one fused Adam launch (k_adam_fused).
 struct AdamSeg {
   float* p[5];

@@ -849,8 +849,9 @@ cudaError_t sb_scatter_staged(cudaStream_t st, unsigned grid, const uint32_t* or
                               uint32_t npad, const ViewBatch& b, const uint32_t* off, uint64_t capacity, uint2* list1,
                               uint32_t* flags) {
   const size_t smem = sb_scatter_staged_smem(b.max_sb);
-  if (smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(k_sb_scatter_staged, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  if (smem > 48 * 1024) {  // the same limit in every call (see kSbScatterMost in capi.cu)
+    const cudaError_t e =
+        cudaFuncSetAttribute(k_sb_scatter_staged, cudaFuncAttributeMaxDynamicSharedMemorySize, kSbStagedMost);
     if (e != cudaSuccess) return e;
   }
   k_sb_scatter_staged<<<grid, kMsThreads, smem, st>>>(order, srect, chunk, npad, b, off, capacity, list1, flags);
