@@ -404,7 +404,7 @@ struct BatchWs {
   float4* rec;
   uint2* rect;
   uint2* srect;  // tile spans in depth order per view (written by the sort's last pass)
-  uint32_t *cnt, *dka, *dva, *dkb, *dvb, *hist, *scan_tmp;
+  uint32_t *dka, *dva, *dkb, *dvb, *hist, *scan_tmp;
   ListsWs lists;
   float* pix_T;
   uint32_t* pix_stop;
@@ -488,7 +488,7 @@ BatchWs carve_batch(void* ws, uint32_t n, const ViewBatch& b, uint64_t capacity)
   w.rec = c.take<float4>(3 * VN + 3, &L.off_rec);
   w.rect = c.take<uint2>(VN + 1, &L.off_rect);
   w.srect = c.take<uint2>(Vp);
-  w.cnt = c.take<uint32_t>(VN + 1, &L.off_cnt);
+  c.take<uint32_t>(0, &L.off_cnt);  // kept in the struct, nothing behind it
   w.dka = c.take<uint32_t>(Vp);
   w.dva = c.take<uint32_t>(Vp, &L.off_order);  // the depth sort ends in dva
   w.dkb = c.take<uint32_t>(Vp);

@@ -211,7 +211,7 @@ typedef struct {
   size_t off_flags;      /* u32[16]: [0] flags, [6..7] tile pairs (u64), [8..9] superblock entries (u64) */
   size_t off_rec;        /* float4[V*N*3] per-view 2D records (written where the tile span is not empty) */
   size_t off_rect;       /* uint2[V*N] tile spans */
-  size_t off_cnt;        /* u32[V*N] reserved (tiles per point; not written by the batched forward) */
+  size_t off_cnt;        /* unused: nothing is kept per point (no memory behind it) */
   size_t off_order;      /* u32[V*npad] points in depth order per view */
   size_t off_sb_start;   /* u32[num_sb*sb_chunks+1] superblock list offsets */
   size_t off_sb_list;    /* uint2[capacity] superblock lists */
