@@ -220,12 +220,14 @@ int build_tile_lists(cudaStream_t st, const ViewBatch& b, uint32_t npad, const L
 
 // An item is heavy, walked in 8x8 blocks, when its longest task's cost is
 // above total / kHeavyShare: 0.375 of a resident warp's part (148 SMs, 24
-// warps each).  Forward and backward in us with every task whole, at 0.25, 0.5
-// and 1 of that part, and with every item heavy (8x8 tiles, SH 0):
-//   16 views, 1,048,576 Gaussians      3490 + 4730, 2930 + 3420, 2980 + 3510, 3110 + 3900, 3370 + 4390
-//   4 at 1280x720, 1,048,576           1450 + 1770, 1300 + 1480, 1300 + 1420, 1390 + 1550, 1320 + 1550
-//   one at 1280x720, 262,144            290 +  330,  215 +  244,  204 +  241,  201 +  232,  209 +  238
-//   8 at 640x480, 100,003               460 +  550,  374 +  478,  408 +  458,  444 +  511,  370 +  487
+// warps each).  Forward and backward in us with every task whole, at 0.25,
+// 0.375, 0.5 and 1 of that part, and with every item heavy (8x8 tiles, SH 0):
+//   16 views, 1,048,576 Gaussians  3137 + 3780, 3141 + 3790, 3141 + 3790, 3137 + 3780, 3137 + 3780, 3610 + 4781
+//   4 at 1280x720, 1,048,576       1340 + 1644, 1136 + 1360, 1088 + 1321, 1098 + 1323, 1153 + 1407, 1184 + 1486
+//   one at 1280x720, 262,144        309 +  364,  231 +  299,  233 +  294,  232 +  294,  227 +  288,  232 +  296
+//   8 at 640x480, 100,003           375 +  489,  375 +  456,  376 +  457,  369 +  438,  371 +  489,  383 +  521
+// (How much the 16 views gain depends on the cameras: where a view's rim walks
+// ten times the mean list it is 0.5 + 1.3 ms of 3.5 + 4.7.)
 constexpr float kHeavyShare = 148.f * 64.f;
 
 cudaError_t order_tasks(cudaStream_t st, const ViewBatch& b, const uint32_t* off1, uint32_t nchunk,
@@ -797,7 +799,8 @@ int dsplat_gauss_batch_backward(dsplat_stream stream, const dsplat_gauss_params*
   count_launch();
   // the forward's longest-first task order: it ranks the tasks by the walks
   // of the forward before it, the same measure as this forward's (equal once
-  // the scene stops changing), and every order gives the same results
+  // the scene stops changing); another order only adds the atomics of a
+  // record's gradient in another order
   stage_mark(st, 7);
   const BwdArgs ba{n,           w.rec,    w.lists.list1,  w.lists.off1, w.L.sb_chunks, pair_capacity,
                    w.task_order, w.sched, w.flags + 3, grad_rgb ? grad_rgb : w.grad_pix, w.pix_T, w.pix_stop, w.grad2d,

@@ -16,9 +16,10 @@
 // read or written at all.  Colour + geometry, us: 1,048,576 points in 16 views
 // 529 + 273 -> 313 + 212, 4,194,304 in 8 1411 + 659 -> 733 + 468, 262,144 in
 // one 70 + 27 -> 36 + 26; the marks cost the backward raster 55 of 3400 and 115
-// of 6700.  5 and 6 blocks per SM (registers 96 and 80) are the best caps:
-// colour at 3, 6 and 8 blocks 404, 361 and 435 (16 views), geometry at 4, 5
-// and 8 241, 218 and 222.
+// of 6700.  5 and 6 blocks per SM (registers 96 and 80) are the best caps,
+// although the degree-3 colour kernel and the geometry one keep some 40 values
+// in local memory there: colour at 3, 6 and 8 blocks 404, 361 and 435 (16
+// views), geometry at 4, 5 and 8 241, 218 and 222.
 // Both add into the caller's gradient buffers (so a per-view loop
 // accumulates naturally).
 //

@@ -205,7 +205,7 @@ typedef struct {
   uint32_t num_items; /* sum over views of tiles */
   uint32_t num_pix;   /* sum over views of pixels */
   uint32_t npad;      /* per-view padded point count of the depth sort */
-  uint32_t slabs_per_tile; /* raster warp tasks per tile (4 for 32x32 tiles, else 1) */
+  uint32_t slabs_per_tile; /* loss slots per tile, one for 32 * pixels_per_lane of its pixels */
   uint32_t num_sb;    /* superblocks over all views */
   uint32_t sb_chunks; /* entries of sb_start per superblock */
   size_t off_flags;      /* u32[16]: [0] flags, [6..7] tile pairs (u64), [8..9] superblock entries (u64) */

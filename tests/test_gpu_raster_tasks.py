@@ -1,9 +1,11 @@
-"""The rasterisers' two task shapes: 8x8 blocks (small batches, every drop-in
-call) at the edges of blocks and tiles, 16x8 tasks (views above 1.25 M pixels)
-at every tile size and pixels-per-lane choice.  Images, transmittances and
-stop positions bit for bit against the oracle; gradients against its FP64
-backward at the tolerance of test_gpu_grad.py (rel 1e-3, floor 1e-2 of the
-largest component, 99.9% of the components)."""
+"""The rasterisers' two task shapes, 8x8 blocks (the longest walks of a batch,
+every drop-in call) and whole tasks, at the edges of blocks and tiles and at
+every tile size and pixels-per-lane choice; which items are walked in blocks is
+up to the schedule here (test_gpu_loss.py, test_gpu_schedule.py and
+test_gpu_nonfinite.py choose it).  Images, transmittances and stop positions bit
+for bit against the oracle; gradients against its FP64 backward at the tolerance
+of test_gpu_grad.py (rel 1e-3, floor 1e-2 of the largest component, 99.9% of the
+components)."""
 import numpy as np
 import pytest
 import torch
