@@ -793,7 +793,10 @@ int dsplat_gauss_batch_backward(dsplat_stream stream, const dsplat_gauss_params*
   // grad2d must start at zero; the projection backward zeroes what it
   // consumes, so only a buffer not known to be clean is cleared here
   const unsigned long long tag = layout_tag(w.L, n, num_views);
-  k_prepare_grad2d<<<blocks_for(3 * VN, 256) < 4096 ? blocks_for(3 * VN, 256) : 4096, 256, 0, st>>>(
+  // enough blocks for the records and, four words a thread, for a caller's gradient
+  const unsigned prepare = std::max(std::min(blocks_for(3 * VN, 256), 4096u),
+                                    grad_rgb ? std::min(blocks_for(size_t(b.num_pix) * 3, 1024), 148u * 16u) : 1u);
+  k_prepare_grad2d<<<prepare, 256, 0, st>>>(
       w.grad2d_tag, tag, w.grad2d, 3 * VN, w.touched, (VN + 3) / 4, w.flags + 3, grad_rgb, size_t(b.num_pix) * 3,
       w.sched + kSchedOdd);
   count_launch();
