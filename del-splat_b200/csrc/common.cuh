@@ -101,17 +101,16 @@ constexpr int kSchedWords = 80;
 
 // What the backward raster's packed pairs may meet (bwd_task): nothing that is
 // not finite, and no product that overflows, since a zero alpha has to stay a
-// zero gradient.  Opacities are at most 1, colours and upstream gradients at
-// most kBwdLarge, and the conic's terms at the box's corner at most kBwdTerms
-// (an axis ratio of 670 at 45 degrees): beyond it the exponent's roundings can
-// turn an alpha into e times itself (2.5e-7 kBwdTerms = 1), and a pixel's walk
-// overflows once five of its entries have been held at 1 / (1 - alpha) = 1e7
-// that way.
-constexpr float kBwdLarge = 3e5f, kBwdTerms = 4e6f;
-__device__ __forceinline__ bool odd_record(const float* conic, float hx, float hy, float opacity, const float* rgb) {
-  const float terms = fabsf(conic[0]) * hx * hx + 2.f * fabsf(conic[1]) * hx * hy + fabsf(conic[2]) * hy * hy;
-  return !(terms <= kBwdTerms && fabsf(opacity) <= 1.f && fabsf(rgb[0]) <= kBwdLarge && fabsf(rgb[1]) <= kBwdLarge &&
-           fabsf(rgb[2]) <= kBwdLarge);
+// zero gradient.  With opacities up to 1 and colours and upstream gradients up to
+// kBwdLarge no product does: 3 kBwdLarge^2, times at most 1e7 for
+// 1 / (1 - alpha).  (That takes alphas up to the opacity.  For a conic with an axis
+// ratio in the thousands the exponent's roundings can exceed 0; a pixel that
+// several such entries overflow gives NaN to the Gaussians of its pair's other
+// pixel too.  Such conics are common in captures, so they are not among the odd.)
+constexpr float kBwdLarge = 1e12f;
+__device__ __forceinline__ bool odd_record(const float* conic, float opacity, const float* rgb) {
+  return !(fabsf(opacity) <= 1.f && fabsf(rgb[0]) <= kBwdLarge && fabsf(rgb[1]) <= kBwdLarge &&
+           fabsf(rgb[2]) <= kBwdLarge && fabsf(conic[0]) + fabsf(conic[1]) + fabsf(conic[2]) < INFINITY);
 }
 
 // Most shared memory of the staged superblock scatter's blocks (three to an SM

@@ -419,7 +419,7 @@ __global__ void __launch_bounds__(kProjThreads) k_fused_project(
       rec[3 * o_idx + 0] = make_float4(o.px, o.py, o.conic[0], o.conic[1]);
       rec[3 * o_idx + 1] = make_float4(o.conic[2], op, col[0], col[1]);
       rec[3 * o_idx + 2] = make_float4(col[2], o.hx, o.hy, o.ndcz);
-      if (odd_record(o.conic, o.hx, o.hy, op, col)) *odd = 1u;
+      if (odd_record(o.conic, op, col)) *odd = 1u;
     }
     rect[o_idx] = pack_rect(x0, y0, x1, y1);
     dkey[size_t(v) * npad + g] = c ? depth_bits(o.ndcz) : 0xffffffffu;

@@ -100,8 +100,9 @@ struct BlockGeo {
 // finite; the CAREFUL form takes every pixel by itself.  It has a launch of its
 // own, which does all the work of a batch with something odd in it (kSchedOdd)
 // and else returns at once (2 us): beside the plain form in one kernel its
-// registers cost the walk 3 to 10%, and a look at the values in every task and
-// batch 1 to 8%.
+// registers cost the walk 3 to 10%, a look at the values in every task and batch
+// 1 to 8%, one at every four entries' sums (walking a task again where they are
+// not finite) 2 to 5%.
 template <class GEO, bool CAREFUL>
 __device__ __forceinline__ void bwd_task(const SbWalkSpan& walk, const PackedSrc& src, Ent* sm, RedBuf* red,
                                          const ViewDev& vd, uint32_t s, uint32_t e, int px0, int py0, int xend,

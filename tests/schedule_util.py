@@ -4,7 +4,9 @@ tile) and walks the items whose cost is a good part of the total in 8x8 blocks."
 import torch
 
 CONFIGS = [(8, 1), (8, 2), (16, 2), (16, 4), (16, 8), (32, 4), (32, 8)]  # tile size, pixels per lane
-SCHED_HEAVY = 76  # word of the schedule (256 bytes after the flags): leading items walked in blocks
+# words of the schedule (256 bytes after the flags): leading items walked in
+# blocks; not 0 where the batch holds something odd
+SCHED_HEAVY, SCHED_ODD = 76, 77
 
 
 def item_cost(batch):
@@ -13,8 +15,16 @@ def item_cost(batch):
     return batch._ws(int(L.total_bytes) - (size + 255) // 256 * 256, int(L.num_items), torch.int32)
 
 
+def _sched(batch, word):
+    return int(batch._ws(int(batch.layout.off_flags) + 256, 80, torch.int32)[word])
+
+
 def heavy_items(batch):
-    return int(batch._ws(int(batch.layout.off_flags) + 256, 80, torch.int32)[SCHED_HEAVY])
+    return _sched(batch, SCHED_HEAVY)
+
+
+def odd(batch):
+    return _sched(batch, SCHED_ODD) != 0
 
 
 def leaders(batch):

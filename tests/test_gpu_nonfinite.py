@@ -1,5 +1,7 @@
 """Parameters, upstream gradients and conics that are not finite, or whose
 inverse is not: what they may not reach."""
+import os
+
 import numpy as np
 import pytest
 import torch
@@ -7,7 +9,7 @@ import torch
 from dsplat import scenes
 from dsplat.gauss import GaussBatch
 from gpu_util import F, params_of
-from schedule_util import CONFIGS, masks, set_blocks
+from schedule_util import CONFIGS, masks, odd, set_blocks
 
 pytestmark = pytest.mark.gpu
 GROUPS = ["means", "log_scales", "quats", "opacity", "colors"]
@@ -94,3 +96,25 @@ def test_batched_image_keeps_odd_colours_in_their_boxes(orc, dev, ts, ppl):
         set_blocks(batch, blocks)
         batch.forward(p)
         assert np.array_equal(F(batch.images()[0]), want, equal_nan=True)
+
+
+def test_a_capture_is_not_odd(dev):
+    """The slower form of the backward is for values that are not finite: the
+    thin conics of a capture and an ordinary loss stay with the other."""
+    from dsplat.render_ply import load_scene
+    cams = scenes.sphere_cameras(np.random.default_rng(7), 8, 3.0, [(640, 480)])
+    sc = load_scene(os.path.join(os.path.dirname(__file__), "golden", "bulba_subset.ply"), cams)
+    p = params_of(sc, dev)
+    batch = GaussBatch(sc.n, cams, 8, 3, pair_capacity=1 << 20, device=dev)
+    batch.ensure_capacity(p)
+    target = torch.rand(int(batch.layout.num_pix) * 3, device=dev)
+    batch.forward(p, target=target)
+    assert not odd(batch)
+    target[7] = float("nan")
+    batch.forward(p, target=target)
+    assert odd(batch)
+    batch.forward(p)
+    assert not odd(batch)
+    p["opacity"][5] = float("inf")
+    batch.forward(p)
+    assert odd(batch)
