@@ -329,8 +329,8 @@ __global__ void __launch_bounds__(256) k_count_pairs(uint32_t n, const float* __
 // 1,048,576 points 392 -> 361 us, 8 of 4,194,304 880 -> 765 (61% of what its
 // 3.0 GB take at the copy rate), one of 262,144 30.5 -> 25.9, 8 of 100,003
 // 32 -> 29.  8 words in flight 769 (4,194,304 points), 24 784, 48 912.
-// The look for odd records takes 18 of some 840 instructions (376 us for 365,
-// 789 for 770).
+// The look for odd records takes 11 of some 830 instructions (16 views 374 us for
+// 365).
 // ---------------------------------------------------------------------------
 constexpr int kProjThreads = 128;
 constexpr int kProjLoads = 16;  // words of the colour rows in flight per thread
