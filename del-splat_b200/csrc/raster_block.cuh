@@ -133,7 +133,8 @@ struct TileWords {  // a per-tile list (tile2idx / idx2pnt)
   __device__ __forceinline__ word load(uint32_t pos) const { return idx2pnt[pos]; }
   static __device__ __forceinline__ uint32_t point(word w) { return w; }
   __device__ __forceinline__ bool hit(word) const { return true; }
-  __device__ __forceinline__ bool counts(word) const { return true; }
+  static constexpr bool kMeasured = false;  // nobody asks for the walk's cost
+  __device__ __forceinline__ bool counts(word) const { return false; }
 };
 
 // A superblock list filtered to the block's tile (lx, ly); the item's tasks
@@ -149,6 +150,7 @@ struct SbWords {
     return x < ((lr >> 8) & 15u) && x + n > (lr & 15u) && ly >= ((lr >> 4) & 15u) && ly < (lr >> 12);
   }
   __device__ __forceinline__ bool hit(word w) const { return meets(w, lx, 1u); }
+  static constexpr bool kMeasured = true;
   __device__ __forceinline__ bool counts(word w) const { return meets(w, run, nx); }
 };
 
@@ -236,7 +238,8 @@ __device__ __forceinline__ uint32_t blend_block(const Walk& walk, const Src& src
     const uint32_t cnt = min(32u, hi - s);
     // stage the batch's entries that hold a pixel of the block, in order
     bool hit = uint32_t(lane) < cnt && walk.hit(en);
-    const uint32_t counted = __ballot_sync(0xffffffffu, uint32_t(lane) < cnt && walk.counts(en));
+    const uint32_t counted =
+        Walk::kMeasured ? __ballot_sync(0xffffffffu, uint32_t(lane) < cnt && walk.counts(en)) : 0u;
     const uint32_t g = walk.point(en);
     uint2 mask = make_uint2(0u, 0u);
     if (hit) {
